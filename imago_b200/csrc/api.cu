@@ -24,6 +24,7 @@
 #include <cstdlib>
 #include <string>
 #include <map>
+#include <unordered_map>
 #include <numeric>
 #include <vector>
 
@@ -169,6 +170,11 @@ struct imago_ctx {
   std::vector<HPType> ptypes;
   std::vector<int> type_screen, ptype_screen;
   int nt = 0, ns = 0, npt = 0, nps = 0, nk = 0, ncell = 0;
+  // k-points computed (the others are their negatives), how many of them
+  // have such a partner, and DevSys::kout (then the identity list of the
+  // builds that compute every k-point)
+  int nka = 0, npair = 0;
+  std::vector<int2> kout;
   int vale_dim = 0, core_dim = 0, pot_dim = 0;
   double T = 0.0;
   double rv[9], recip[9], inv[9];
@@ -217,6 +223,7 @@ struct imago_ctx {
   DBuf<double> d_alpha, d_basis, d_site_pos, d_ptype_z, d_ptype_nucalpha,
       d_palpha, d_psite_pos, d_cell, d_csize, d_kxyz;
   DBuf<double2> d_phase;
+  DBuf<int2> d_kout;
   DBuf<DPair> d_pairs;
   DBuf<DUnit> d_units;
   DBuf<DSp> d_sps;
@@ -308,6 +315,7 @@ struct imago_ctx {
     d_site_rank.release(st);
     d_queue.release(st);
     d_flag.release(st);
+    d_kout.release(st);
     if (st) cudaStreamSynchronize(st);
     if (events)
       for (auto &e : ev) cudaEventDestroy(e);
@@ -451,6 +459,63 @@ void nearest_lattice_host(const imago_ctx *c, const double *v, double *out) {
   std::memcpy(out, best, sizeof best);
 }
 
+// The k-points to compute: of each pair with f_b = -f_a up to whole
+// numbers (fractional coordinates; up to 2 ulp of 1, the rounding of a mesh
+// formula, far below the rounding of k.R itself) only the first.  Their
+// order: paired ones, unpaired ones, then the pairs' second members in the
+// order of the first.  kxyz is put in that order.
+void pair_kpoints(imago_ctx *c, const double *f) {
+  const int nk = c->nk;
+  auto wrap = [](double x) { return x - std::rint(x); };  // to [-1/2, 1/2]
+  auto key = [&](const double *v, double sign) {
+    // coordinates mod 1 on a grid of 2^-20; 1/2 and -1/2 share a cell
+    unsigned long long h = 0;
+    for (int x = 0; x < 3; ++x) {
+      long long q = std::llround(wrap(sign * v[x]) * 1048576.0);
+      if (q == -524288) q = 524288;
+      h = h * 2097169ull + (unsigned long long)(q + 1048576);
+    }
+    return h;
+  };
+  auto negatives = [&](int a, int b) {
+    for (int x = 0; x < 3; ++x)
+      if (!(std::fabs(wrap(f[3 * a + x] + f[3 * b + x])) <= 4.5e-16)) return false;
+    return true;
+  };
+  std::unordered_multimap<unsigned long long, int> open;  // unpaired so far, by key
+  std::vector<int> mate(nk, -1), first, second, alone;
+  for (int k = 0; k < nk; ++k) {
+    const auto range = open.equal_range(key(f + 3 * k, -1.0));
+    for (auto it = range.first; it != range.second; ++it)
+      if (negatives(it->second, k)) {
+        mate[k] = it->second;
+        mate[it->second] = k;
+        open.erase(it);
+        break;
+      }
+    if (mate[k] < 0) open.emplace(key(f + 3 * k, 1.0), k);
+  }
+  for (int k = 0; k < nk; ++k) {
+    if (mate[k] < 0) alone.push_back(k);
+    else if (mate[k] > k) {
+      first.push_back(k);
+      second.push_back(mate[k]);
+    }
+  }
+  c->npair = (int)first.size();
+  c->nka = c->npair + (int)alone.size();
+  std::vector<int> order(first);
+  order.insert(order.end(), alone.begin(), alone.end());
+  order.insert(order.end(), second.begin(), second.end());
+  const std::vector<double> xyz(c->kxyz);
+  for (int i = 0; i < nk; ++i)
+    for (int x = 0; x < 3; ++x) c->kxyz[3 * i + x] = xyz[3 * order[i] + x];
+  c->kout.clear();
+  for (int i = 0; i < c->nka; ++i)
+    c->kout.push_back(make_int2(order[i], i < c->npair ? second[i] : -1));
+  for (int i = 0; i < nk; ++i) c->kout.push_back(make_int2(order[i], -1));
+}
+
 // ------------------------------------------------------------ set-up --
 int read_system(imago_ctx *c, const imago_system *s) {
   if (!s || s->num_atom_types <= 0 || s->num_atom_sites <= 0 ||
@@ -586,6 +651,7 @@ int read_system(imago_ctx *c, const imago_system *s) {
       c->kxyz[3 * k + x] = f[0] * c->recip[x] + f[1] * c->recip[3 + x] +
                            f[2] * c->recip[6 + x];
   }
+  pair_kpoints(c, s->kpoints_abc);
   return IMAGO_OK;
 }
 
@@ -871,7 +937,7 @@ int upload(imago_ctx *c) {
   UP(d_psite_ptype, c->psite_ptype) UP(d_cell, c->cells) UP(d_csize, c->csize)
   UP(d_kxyz, c->kxyz) UP(d_pairs, c->pairs) UP(d_units, c->units)
   UP(d_sps, c->sps) UP(d_sp_by_cls, c->sp_by_cls) UP(d_terms, c->ep_terms)
-  UP(d_btile, c->btile) UP(d_btile_w, c->btile_w)
+  UP(d_btile, c->btile) UP(d_btile_w, c->btile_w) UP(d_kout, c->kout)
 #undef UP
   if ((rc = c->d_queue.alloc(4, st))) return rc;
   if ((rc = c->d_flag.alloc(1, st))) return rc;
@@ -887,7 +953,8 @@ int upload(imago_ctx *c) {
   if ((rc = c->d_phase.alloc((size_t)c->ncell * c->nk, st))) return rc;
 
   DevSys &s = c->sys;
-  s.nt = c->nt; s.ns = c->ns; s.npt = c->npt; s.nps = c->nps; s.nk = c->nk;
+  s.nt = c->nt; s.ns = c->ns; s.npt = c->npt; s.nps = c->nps;
+  s.nk = c->nka; s.nkt = c->nk; s.kout = c->d_kout.p;
   s.ncell = c->ncell; s.vale_dim = c->vale_dim; s.core_dim = c->core_dim;
   s.T = c->T;
   std::memcpy(s.rv, c->rv, sizeof s.rv);
@@ -946,19 +1013,22 @@ int upload(imago_ctx *c) {
 
 // Device bytes one term of a build needs between its stages.
 size_t term_bytes(const imago_ctx *c) {
-  const size_t V = c->vale_dim, C = c->core_dim, nk = c->nk;
+  const size_t V = c->vale_dim, C = c->core_dim, nk = c->nk, nka = c->nka;
   return sizeof(double) * (size_t)(c->blk_total + c->m_total) +
-         sizeof(double2) * nk * (V * V + 2 * V * C + C * C) +
+         sizeof(double2) * nka * (V * V + 2 * V * C + C * C) +
          sizeof(double2) * nk * (V * (V + 1) / 2);
 }
 
-int ensure_scratch(imago_ctx *c, int nterm) {
-  const size_t V = c->vale_dim, C = c->core_dim, nk = c->nk;
+// Scratch for nterm sets of blocks and, unless `full` terms over every
+// k-point are asked for, nterm sets of matrices over the computed ones.
+int ensure_scratch(imago_ctx *c, int nterm, int full = 0) {
+  const size_t V = c->vale_dim, C = c->core_dim;
+  const size_t nk = full ? (size_t)c->nk * full : (size_t)c->nka * nterm;
   imago_ctx::Scratch &S = c->scr[c->lane];
   cudaStream_t st = c->cur();
   const size_t nblk = (size_t)c->blk_total * nterm + 1, nm = (size_t)c->m_total * nterm + 1;
-  const size_t nvv = nk * V * V * nterm + 1, ncv = nk * V * C * nterm + 1;
-  const size_t ncc = nk * C * C * nterm + 1;
+  const size_t nvv = nk * V * V + 1, ncv = nk * V * C + 1;
+  const size_t ncc = nk * C * C + 1;
   // A captured build graph holds these buffers' addresses: a build that
   // needs more (more terms per pass, as the three- and six-term builds
   // do) drops the graph before the old buffers are freed, and the next
@@ -1300,7 +1370,7 @@ int run_build(imago_ctx *c, Kind kind, int term0, int nterm,
     return rc;
   if ((rc = launch_contract(s, w, nterm, S.blk.p, S.M.p, st, c->contract_tpc))) return rc;
   mark(c);
-  if (!c->bloch_tuned && !c->capturing && s.nk > kBlochSmallNk) {
+  if (!c->bloch_tuned && !c->capturing && s.nkt > kBlochSmallNk) {
     if ((rc = tune_bloch(c, nterm))) return rc;
     tune_store(c);
   }
@@ -1308,8 +1378,8 @@ int run_build(imago_ctx *c, Kind kind, int term0, int nterm,
     return rc;
   mark(c);
   if (kind == KIND_OL && c->core_dim > 0) {
-    const size_t n = (size_t)c->nk * c->vale_dim * c->core_dim;
-    if ((rc = c->s_cv.alloc(n, st))) return rc;
+    const size_t n = (size_t)c->nka * c->vale_dim * c->core_dim;
+    if ((rc = c->s_cv.alloc((size_t)c->nk * c->vale_dim * c->core_dim, st))) return rc;
     IMAGO_CUDA(cudaMemcpyAsync(c->s_cv.p, S.cv.p, n * sizeof(double2),
                                cudaMemcpyDeviceToDevice, st));
     IMAGO_CUDA(cudaEventRecord(c->ev_scv, st));
@@ -1414,7 +1484,7 @@ int do_ol(imago_ctx *c, double *packed, double *cv_re, double *cv_im) {
       // one of the two requested on the device: split through y
       double *scratch = reinterpret_cast<double *>(c->scr[c->lane].y.p);
       if (!re) re = scratch;
-      if (!im) im = scratch + ncv;
+      if (!im) im = scratch;
     }
     if ((rc = launch_split_cv(c->sys, c->s_cv.p, re, im, c->cur()))) return rc;
     c->launches += 1;
@@ -1466,7 +1536,7 @@ int do_vec(imago_ctx *c, Kind kind, double *packed) {
 int do_kov(imago_ctx *c, const double *dk, double *re, double *im) {
   if (c->core_dim > 0 && !c->have_ol) return IMAGO_ERR_NEED_OVERLAP;
   cudaStream_t st = c->cur();
-  int rc = ensure_scratch(c, 6);
+  int rc = ensure_scratch(c, 6, 3);
   if (rc) return rc;
   imago_ctx::Scratch &S = c->scr[c->lane];
   const size_t n = (size_t)3 * c->nk * c->vale_dim * c->vale_dim;
@@ -1478,9 +1548,12 @@ int do_kov(imago_ctx *c, const double *dk, double *re, double *im) {
   }
   KovWaves q;
   for (int x = 0; x < 9; ++x) q.q[x] = dk[x];
-  const DevSys &s = c->sys;
+  // the plane wave breaks H(-k) = conj H(k): every k-point is computed
+  DevSys s = c->sys;
+  s.nk = c->nk;
+  s.kout = c->d_kout.p + c->nka;
   const DevWork &w = c->work;
-  c->launches += class_launches(c) + 2 + (c->core_dim > 0 ? 2 : 1);
+  c->launches += class_launches(c) + 2 + (c->core_dim > 0 ? 2 : 1) + (c->npair > 0 ? 1 : 0);
   mark(c);
   if ((rc = launch_prim_kov(s, w, c->cls_beg, q, S.blk.p, st))) return rc;
   mark(c);
@@ -1489,6 +1562,7 @@ int do_kov(imago_ctx *c, const double *dk, double *re, double *im) {
   if ((rc = launch_bloch_kov(s, w, S.M.p, S.vv.p, S.cv.p, S.cc.p, st))) return rc;
   mark(c);
   if (c->core_dim > 0 && c->ol_in_call) IMAGO_CUDA(cudaStreamWaitEvent(st, c->ev_scv, 0));
+  if (c->core_dim > 0 && (rc = launch_conj_cv(c->sys, c->npair, c->s_cv.p, st))) return rc;
   if ((rc = launch_ortho_full(s, S.vv.p, S.cv.p, S.cc.p, c->s_cv.p, S.y.p, tre, tim, st)))
     return rc;
   mark(c);
@@ -1611,7 +1685,7 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
   mark(c);
   if ((rc = launch_contract(s, w, spin, c->ham_blk.p, S.M.p, st))) return rc;
   mark(c);
-  if (!c->bloch_tuned && s.nk > kBlochSmallNk) {
+  if (!c->bloch_tuned && s.nkt > kBlochSmallNk) {
     if ((rc = tune_bloch(c, spin))) return rc;
     tune_store(c);
   }

@@ -10,7 +10,15 @@ namespace imago {
 
 // Everything the kernels read about the system, as device pointers.
 struct DevSys {
-  int nt, ns, npt, nps, nk, ncell;
+  int nt, ns, npt, nps, ncell;
+  // k-points the stages compute (nk) and the caller's (nkt): M real gives
+  // H(-k) = conj H(k), so of two k-points that are each other's negative up
+  // to a reciprocal lattice vector only one is summed and orthogonalised.
+  // Device arrays hold the computed ones first, paired ones before the
+  // others; kout[k] is the caller's index of computed k-point k and of its
+  // partner (-1: none)
+  int nk, nkt;
+  const int2 *kout;
   int vale_dim, core_dim;
   double T;            // logBasisFnThresh = -ln(basisFnConvg)
   double rv[9];        // realVectors [abc*3 + xyz]
@@ -43,8 +51,8 @@ struct DevSys {
   // lattice cells sorted by |R|^2, k-points, phase table
   const double *cell;     // [n*3]
   const double *csize;    // [n]
-  const double *kxyz;     // [nk*3]
-  const double2 *phase;   // [cell * nk + k]  exp(i k.R)
+  const double *kxyz;     // [nkt*3], computed k-points first
+  const double2 *phase;   // [cell * nkt + k]  exp(i k.R)
   // device status word: a kernel whose bounded wait ran out records
   // IMAGO_ERR_TIMEOUT here (first failure wins); read after each call
   int *flag;
@@ -236,6 +244,10 @@ int launch_block_axpy(const double *blk, int nterm, long long n, const double *w
                       int wstride, int spin, double *H, cudaStream_t st);
 int launch_split_cv(const DevSys &s, const double2 *cv, double *re, double *im,
                     cudaStream_t st);
+// Entries of the pairs' second k-points behind the computed ones,
+// cv[nk + k] = conj cv[k] for k < npair, for the builds whose k-points are
+// not related by conjugation.
+int launch_conj_cv(const DevSys &s, int npair, double2 *cv, cudaStream_t st);
 int launch_phase(const DevSys &s, double2 *phase, cudaStream_t st);
 int launch_site_images(const DevSys &s, const DevWork &w, SiteImage *simg,
                        float *cl_d1, cudaStream_t st);

@@ -34,6 +34,31 @@ __device__ __forceinline__ void store_packed(double *out, long long idx, double2
   }
 }
 
+// Where the packed results of computed k-point k of a term go: the
+// caller's k-point itself and, where it has one, its partner -k, whose
+// matrix is the conjugate (with the momentum's -i in front, minus the
+// conjugate).  Writing both here costs the partner's stores alone: half
+// the phase sums and orthogonalisations of an inversion-symmetric mesh are
+// never formed (162-atom quartz, 2x2x2 k: orthogonalisation 91.7 -> 46 ms).
+struct OutK {
+  double *a, *b;  // first packed double; b null without a partner
+  double sr, si;
+};
+__device__ __forceinline__ OutK out_k(const DevSys &s, double *packed, int term, int k,
+                                      long long np) {
+  const int2 o = s.kout[k];
+  OutK r;
+  r.a = packed + 2 * ((long long)term * s.nkt + o.x) * np;
+  r.b = o.y < 0 ? nullptr : packed + 2 * ((long long)term * s.nkt + o.y) * np;
+  r.sr = s.minus_i ? -1.0 : 1.0;
+  r.si = -r.sr;
+  return r;
+}
+__device__ __forceinline__ void store_out(const OutK &o, long long idx, double2 v) {
+  store_packed(o.a, idx, v);
+  if (o.b) store_packed(o.b, idx, make_double2(o.sr * v.x, o.si * v.y));
+}
+
 // 16-byte global-to-shared copy that does not pass through registers;
 // with `valid` false nothing is read and the destination is zero-filled.
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem,
@@ -317,7 +342,7 @@ __global__ void __launch_bounds__(4 * BC, (KOV ? 128 : 256) / BC)
       if (i < kBU * kBK) {
         const bool in = u0 + uu < nu && k0 + kk < nk;
         const double2 *src =
-            in ? s.phase + (long long)w.units[p.ubeg + u0 + uu].cell * nk + k0 + kk
+            in ? s.phase + (long long)w.units[p.ubeg + u0 + uu].cell * s.nkt + k0 + kk
                : s.phase;
         cp_async16(&ph_s[buf][uu][kk], src, in);
       }
@@ -459,7 +484,7 @@ __global__ void __launch_bounds__(kBC)
   for (int k = 0; k < kBlochSmallNk; ++k) re[k] = im[k] = 0.0;
   for (int u = p.ubeg; u < p.uend; ++u) {
     const double m = Mt[(long long)(u - p.ubeg) * ne];
-    const double2 *ph = s.phase + (long long)w.units[u].cell * nk;
+    const double2 *ph = s.phase + (long long)w.units[u].cell * s.nkt;
 #pragma unroll
     for (int k = 0; k < kBlochSmallNk; ++k)
       if (k < nk) {
@@ -484,7 +509,7 @@ __global__ void __launch_bounds__(kBC)
 int launch_bloch(const DevSys &s, const DevWork &w, int nterm, const double *M,
                  double2 *vv, double2 *cv, double2 *cc, cudaStream_t st) {
   if (w.nbtile == 0 || nterm == 0) return IMAGO_OK;
-  if (s.nk <= kBlochSmallNk) {
+  if (s.nkt <= kBlochSmallNk) {
     k_bloch_small<<<dim3(w.nbtile, nterm), kBC, 0, st>>>(s, w, M, vv, cv, cc);
     IMAGO_CUDA(cudaGetLastError());
     return IMAGO_OK;
@@ -712,7 +737,7 @@ __global__ void __launch_bounds__(kOThreads, 4)
   }
   const double2 *VVt = vv + tk * V * V;
   const long long np = (long long)V * (V + 1) / 2;
-  double *out = packed + 2 * tk * np;
+  const OutK out = out_k(s, packed, term, k, np);
   const int r0 = (warp >> 1) * 16, cb = (warp & 1) * 16;
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
@@ -728,7 +753,8 @@ __global__ void __launch_bounds__(kOThreads, 4)
         v.x -= p.x;
         v.y -= p.y;
         if (FULL) {  // the whole matrix as real and imaginary planes
-          const long long o = (tk * V + col) * (long long)V + row;
+          const long long o =
+              (((long long)term * s.nkt + s.kout[k].x) * V + col) * (long long)V + row;
           packed[o] = v.x;
           im_plane[o] = v.y;
           continue;
@@ -737,7 +763,7 @@ __global__ void __launch_bounds__(kOThreads, 4)
         if (fabs(v.x) < kPackThresh) v.x = 0.0;
         if (fabs(v.y) < kPackThresh) v.y = 0.0;
         const long long idx = (long long)col * (col + 1) / 2 + row;
-        store_packed(out, idx, v);
+        store_out(out, idx, v);
       }
 }
 
@@ -913,7 +939,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
   // upper subtiles (J <= I) of S^H Y + Y^H S over the stacked k = 2 C4
   const double2 *VVt = vv + tk * V * V;
   const long long np = (long long)V * (V + 1) / 2;
-  double *out = packed + 2 * tk * np;
+  const OutK out = out_k(s, packed, term, k, np);
   const int nt16 = d.V16 / 16, nup = nt16 * (nt16 + 1) / 2;
   for (int tile = warp; tile < nup; tile += kFWarps) {
     int t = tile, I = 0;
@@ -956,7 +982,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
           if (fabs(v.x) < kPackThresh) v.x = 0.0;
           if (fabs(v.y) < kPackThresh) v.y = 0.0;
           const long long idx = (long long)col * (col + 1) / 2 + row;
-          store_packed(out, idx, v);
+          store_out(out, idx, v);
         }
   }
 }
@@ -1078,6 +1104,7 @@ __device__ __forceinline__ void pipe_y_tile(const double2 *XC, int ld, int C, in
 // What every thread of a k_ortho_pipe CTA reads (kept in shared memory,
 // written once by thread 0).
 struct PipeCta {
+  const DevSys *s;
   const double2 *vv;
   double *packed;
   double2 *Ss, *Xb[2], *Xc;
@@ -1096,7 +1123,8 @@ __device__ __forceinline__ void pipe_w_task(const PipeCta &p, long long q, int t
   const long long tk = (long long)(q % p.nterm) * p.nk + q / p.nterm;
   const double2 *Ys = p.Xb[(q - p.i0) & 1];
   const double2 *VVt = p.vv + tk * V * V;
-  double *out = p.packed + 2 * tk * p.np;
+  const OutK out =
+      out_k(*p.s, p.packed, (int)(q % p.nterm), (int)(q / p.nterm), p.np);
   int t = tile, I = 0;
   while (t > I) {
     t -= I + 1;
@@ -1123,7 +1151,7 @@ __device__ __forceinline__ void pipe_w_task(const PipeCta &p, long long q, int t
         if (row == col) v.y = 0.0;
         if (fabs(v.x) < kPackThresh) v.x = 0.0;
         if (fabs(v.y) < kPackThresh) v.y = 0.0;
-        store_packed(out, (long long)col * (col + 1) / 2 + row, v);
+        store_out(out, (long long)col * (col + 1) / 2 + row, v);
       }
 }
 
@@ -1219,7 +1247,7 @@ __device__ __forceinline__ bool pipe_phase(const PipeCta &p, unsigned px[2], int
 
 template <bool REAL>
 __global__ void __launch_bounds__(kFThreads, 1)
-    k_ortho_pipe(DevSys s, const __grid_constant__ CUtensorMap map_x,
+    k_ortho_pipe(const __grid_constant__ DevSys s, const __grid_constant__ CUtensorMap map_x,
                  const __grid_constant__ CUtensorMap map_c,
                  const __grid_constant__ CUtensorMap map_s, const double2 *vv, int nterm,
                  double *packed) {
@@ -1232,6 +1260,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
   __shared__ PipeCta p;
   const int tid = threadIdx.x;
   if (tid == 0) {
+    p.s = &s;
     p.vv = vv;
     p.packed = packed;
     p.Ss = reinterpret_cast<double2 *>(psm);
@@ -1402,7 +1431,7 @@ __global__ void __launch_bounds__(256)
   const long long np = (long long)V * (V + 1) / 2;
   const long long tk = (long long)term * s.nk + k;
   const double2 *VVt = vv + tk * V * V;
-  double *out = packed + 2 * tk * np;
+  const OutK out = out_k(s, packed, term, k, np);
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
        idx < np; idx += (long long)gridDim.x * blockDim.x) {
     int col = (int)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
@@ -1410,7 +1439,7 @@ __global__ void __launch_bounds__(256)
     while ((long long)(col + 1) * (col + 2) / 2 <= idx) ++col;
     const int row = (int)(idx - (long long)col * (col + 1) / 2);
     const double2 v = VVt[(long long)col * V + row];
-    store_packed(out, idx, v);
+    store_out(out, idx, v);
   }
 }
 
@@ -1486,7 +1515,7 @@ __global__ void __launch_bounds__(256)
   for (int u = p.ubeg; u < p.uend; ++u) {
     const long long o = (long long)(u - p.ubeg) * ne;
     const double xr = Mr[o], xi = Mi[o];
-    const double2 f = s.phase[(long long)w.units[u].cell * nk + k];
+    const double2 f = s.phase[(long long)w.units[u].cell * s.nkt + k];
     ar = ar + (f.x * xr - f.y * xi);
     ai = ai + (f.x * xi + f.y * xr);
   }
@@ -1506,7 +1535,7 @@ __global__ void __launch_bounds__(256)
 int launch_bloch_kov(const DevSys &s, const DevWork &w, const double *M, double2 *vv,
                      double2 *cv, double2 *cc, cudaStream_t st) {
   if (w.nbtile == 0) return IMAGO_OK;
-  if (s.nk > kBlochSmallNk) {  // the tensor-core phase sum at the tuned width
+  if (s.nkt > kBlochSmallNk) {  // the tensor-core phase sum at the tuned width
     if (w.nbtile_w == 0) return IMAGO_OK;
     dim3 grid(w.nbtile_w, (s.nk + kBK - 1) / kBK, 3);
     switch (w.bw) {
@@ -1532,11 +1561,15 @@ int launch_bloch_kov(const DevSys &s, const DevWork &w, const double *M, double2
   return IMAGO_OK;
 }
 
-__global__ void k_vv_planes(long long n, const double2 *vv, double *re, double *im) {
+__global__ void k_vv_planes(DevSys s, long long n, const double2 *vv, double *re, double *im) {
+  const long long v2 = (long long)s.vale_dim * s.vale_dim;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    re[i] = vv[i].x;
-    im[i] = vv[i].y;
+    const long long tk = i / v2;
+    const int term = (int)(tk / s.nk), k = (int)(tk % s.nk);
+    const long long o = ((long long)term * s.nkt + s.kout[k].x) * v2 + (i - tk * v2);
+    re[o] = vv[i].x;
+    im[o] = vv[i].y;
   }
 }
 
@@ -1547,7 +1580,7 @@ int launch_ortho_full(const DevSys &s, const double2 *vv, const double2 *cv,
   if (C == 0) {
     const long long n = 3LL * s.nk * V * V;
     k_vv_planes<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
-        n, vv, re, im);
+        s, n, vv, re, im);
     IMAGO_CUDA(cudaGetLastError());
     return IMAGO_OK;
   }
@@ -1587,14 +1620,37 @@ int launch_ortho_general(const DevSys &s, int nterm, const double2 *vv,
 
 // coreValeOL as the reference writes it: separate real and imaginary
 // (coreDim, valeDim) matrices per k.
-__global__ void k_split_cv(long long n, const double2 *cv, double *re,
+__global__ void k_split_cv(DevSys s, long long per, const double2 *cv, double *re,
                            double *im) {
+  const long long n = s.nk * per;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
+    const int k = (int)(i / per);
+    const long long e = i - k * per;
+    const int2 o = s.kout[k];
     const double2 v = cv[i];
-    re[i] = v.x;
-    im[i] = v.y;
+    re[o.x * per + e] = v.x;
+    im[o.x * per + e] = v.y;
+    if (o.y >= 0) {
+      re[o.y * per + e] = v.x;
+      im[o.y * per + e] = -v.y;
+    }
   }
+}
+
+__global__ void k_conj_cv(long long n, const double2 *cv, double2 *out) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x)
+    out[i] = make_double2(cv[i].x, -cv[i].y);
+}
+
+int launch_conj_cv(const DevSys &s, int npair, double2 *cv, cudaStream_t st) {
+  const long long per = (long long)s.vale_dim * s.core_dim, n = npair * per;
+  if (n == 0) return IMAGO_OK;
+  k_conj_cv<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(
+      n, cv, cv + s.nk * per);
+  IMAGO_CUDA(cudaGetLastError());
+  return IMAGO_OK;
 }
 
 int launch_split_cv(const DevSys &s, const double2 *cv, double *re, double *im,
@@ -1602,7 +1658,7 @@ int launch_split_cv(const DevSys &s, const double2 *cv, double *re, double *im,
   const long long n = (long long)s.nk * s.vale_dim * s.core_dim;
   if (n == 0) return IMAGO_OK;
   k_split_cv<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(
-      n, cv, re, im);
+      s, (long long)s.vale_dim * s.core_dim, cv, re, im);
   IMAGO_CUDA(cudaGetLastError());
   return IMAGO_OK;
 }
@@ -1640,10 +1696,10 @@ int launch_block_axpy(const double *blk, int nterm, long long n, const double *w
 // phaseFactor(k, cell) = exp(i k.R) (kpoints.f90:578-609), stored cell-major
 // so one image's phases for consecutive k are contiguous.
 __global__ void k_phase(DevSys s, double2 *phase) {
-  const long long n = (long long)s.ncell * s.nk;
+  const long long n = (long long)s.ncell * s.nkt;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i / s.nk), k = (int)(i % s.nk);
+    const int c = (int)(i / s.nkt), k = (int)(i % s.nkt);
     const double *kv = s.kxyz + 3 * k, *R = s.cell + 3 * c;
     const double dot = kv[0] * R[0] + kv[1] * R[1] + kv[2] * R[2];
     double sn, cs;
@@ -1653,7 +1709,7 @@ __global__ void k_phase(DevSys s, double2 *phase) {
 }
 
 int launch_phase(const DevSys &s, double2 *phase, cudaStream_t st) {
-  const long long n = (long long)s.ncell * s.nk;
+  const long long n = (long long)s.ncell * s.nkt;
   k_phase<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(s, phase);
   IMAGO_CUDA(cudaGetLastError());
   return IMAGO_OK;
