@@ -17,7 +17,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(ROOT, "_build", "imago_b200")
 LIB = os.path.join(HERE, "libimago_b200.so")
-SOURCES = ["api.cu", "k_dense.cu", "k_prim.cu", "k_eval.cu", "noalloc.cu",
+SOURCES = ["api.cu", "k_dense.cu", "k_prim.cu", "k_terms.cu", "k_nuc.cu", "k_ham.cu", "k_eval.cu", "noalloc.cu",
            "k_secular.cu", "k_reduce.cu", "populate.cu", "scf.cu", "learned.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr",
@@ -31,10 +31,18 @@ def nvcc():
     return "nvcc"
 
 
-def _headers():
-    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
-    hs += [os.path.join(ROOT, "include", f) for f in os.listdir(os.path.join(ROOT, "include"))]
-    return hs
+def _deps(path, seen=None):
+    """`path` and the files it includes by quoted name, directly or not."""
+    seen = set() if seen is None else seen
+    if path in seen or not os.path.exists(path):
+        return seen
+    seen.add(path)
+    with open(path) as fh:
+        for line in fh:
+            if line.startswith('#include "'):
+                name = line.split('"')[1]
+                _deps(os.path.normpath(os.path.join(os.path.dirname(path), name)), seen)
+    return seen
 
 
 def _stale(target, deps):
@@ -46,8 +54,7 @@ def _stale(target, deps):
 
 def _compile(src):
     obj = os.path.join(OBJ, src.replace(".cu", ".o"))
-    deps = [os.path.join(CSRC, src)] + _headers()
-    if not _stale(obj, deps):
+    if not _stale(obj, _deps(os.path.join(CSRC, src))):
         return obj
     cmd = [nvcc()] + ARCH + FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)

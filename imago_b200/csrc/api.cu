@@ -219,9 +219,9 @@ struct imago_ctx {
       d_type_state_off, d_type_basis_off, d_type_screen, d_alpha_cls,
       d_state_lm, d_site_type, d_site_cum_vale, d_site_cum_core,
       d_ptype_alpha_off, d_ptype_nalpha, d_ptype_first_site, d_ptype_mult,
-      d_ptype_screen, d_psite_ptype, d_sp_by_cls;
+      d_ptype_screen, d_sp_by_cls;
   DBuf<double> d_alpha, d_basis, d_site_pos, d_ptype_z, d_ptype_nucalpha,
-      d_palpha, d_psite_pos, d_cell, d_csize, d_kxyz;
+      d_palpha, d_cell, d_csize, d_kxyz;
   DBuf<double2> d_phase;
   DBuf<int2> d_kout;
   DBuf<DPair> d_pairs;
@@ -231,9 +231,13 @@ struct imago_ctx {
   DBuf<unsigned long long> d_queue;  // one work-queue counter per lane
   DBuf<int> d_flag;                  // DevSys::flag
   DBuf<int2> d_btile, d_btile_w;
-  DBuf<SiteImage> d_simg;
-  DBuf<float> d_cl_d1;
-  DBuf<int> d_site_rank;
+  // the three-centre screens' image table and lists (DevWork)
+  DBuf<double4> d_ipos;
+  DBuf<float4> d_ftab;
+  DBuf<int> d_img_off, d_ptype_ascends;
+  DBuf<int2> d_uoff;
+  DBuf<ImageRef> d_ulist;
+  DBuf<float> d_rad;
 
   // scratch
   // Each build kind (OL, KE, NP, EP) has its own scratch and stream (a
@@ -296,10 +300,10 @@ struct imago_ctx {
                     &d_type_screen, &d_alpha_cls, &d_state_lm, &d_site_type,
                     &d_site_cum_vale, &d_site_cum_core, &d_ptype_alpha_off,
                     &d_ptype_nalpha, &d_ptype_first_site, &d_ptype_mult,
-                    &d_ptype_screen, &d_psite_ptype, &d_sp_by_cls})
+                    &d_ptype_screen, &d_sp_by_cls})
       b->release(st);
     for (auto *b : {&d_alpha, &d_basis, &d_site_pos, &d_ptype_z,
-                    &d_ptype_nucalpha, &d_palpha, &d_psite_pos, &d_cell,
+                    &d_ptype_nucalpha, &d_palpha, &d_cell,
                     &d_csize, &d_kxyz, &out_stage, &ham_blk, &ham_w, &ham_out, &vec_out})
       b->release(st);
     for (auto &sc : scr) {
@@ -309,10 +313,10 @@ struct imago_ctx {
     }
     for (auto *b : {&d_phase, &s_cv}) b->release(st);
     d_pairs.release(st); d_units.release(st); d_sps.release(st);
-    d_terms.release(st); d_btile.release(st); d_simg.release(st);
-    d_btile_w.release(st);
-    d_cl_d1.release(st);
-    d_site_rank.release(st);
+    d_terms.release(st); d_btile.release(st); d_btile_w.release(st);
+    d_ipos.release(st); d_ftab.release(st); d_img_off.release(st);
+    d_ptype_ascends.release(st); d_uoff.release(st); d_ulist.release(st);
+    d_rad.release(st);
     d_queue.release(st);
     d_flag.release(st);
     d_kout.release(st);
@@ -378,40 +382,6 @@ void recip_vectors(imago_ctx *c) {
     for (int j = 0; j < 3; ++j) c->recip[3 * i + j] = 2.0 * kPi * r[j] / vol;
   }
   for (int i = 0; i < 9; ++i) c->inv[i] = c->recip[i] / (2.0 * kPi);
-}
-
-// Smallest singular value of realVectors: the square root of the smallest
-// eigenvalue of the Gram matrix G = R R^T, by cyclic Jacobi rotations.
-double smallest_singular(const double *rv) {
-  double g[3][3];
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      g[i][j] = 0.0;
-      for (int x = 0; x < 3; ++x) g[i][j] += rv[3 * i + x] * rv[3 * j + x];
-    }
-  for (int sweep = 0; sweep < 50; ++sweep) {
-    const double off = g[0][1] * g[0][1] + g[0][2] * g[0][2] + g[1][2] * g[1][2];
-    const double dia = g[0][0] * g[0][0] + g[1][1] * g[1][1] + g[2][2] * g[2][2];
-    if (off <= 1e-30 * dia) break;
-    for (int p = 0; p < 2; ++p)
-      for (int q = p + 1; q < 3; ++q) {
-        if (g[p][q] == 0.0) continue;
-        const double th = 0.5 * std::atan2(2.0 * g[p][q], g[q][q] - g[p][p]);
-        const double c = std::cos(th), sn = std::sin(th);
-        for (int k = 0; k < 3; ++k) {  // G <- G J
-          const double a = g[k][p], b = g[k][q];
-          g[k][p] = c * a - sn * b;
-          g[k][q] = sn * a + c * b;
-        }
-        for (int k = 0; k < 3; ++k) {  // G <- J^T G
-          const double a = g[p][k], b = g[q][k];
-          g[p][k] = c * a - sn * b;
-          g[q][k] = sn * a + c * b;
-        }
-      }
-  }
-  const double lmin = std::min(g[0][0], std::min(g[1][1], g[2][2]));
-  return std::sqrt(std::max(lmin, 0.0));
 }
 
 int make_cells(imago_ctx *c, double min_atom_alpha, double min_pot_alpha) {
@@ -742,7 +712,7 @@ void build_pairs(const imago_ctx *c, const std::vector<int2> &ij, size_t lo,
             sp.la = (short)t1.cls[a];
             sp.lb = (short)t2.cls[b];
             sp.boff = w.boff;
-            w.boff += nsh(sp.la) * nsh(sp.lb);
+            w.boff += blk_len(sp.la, sp.lb);
             w.sps.push_back(sp);
             // the pair's own part of the three-centre screening radius^2,
             // frac T / (a1 + a2) (gaussRelations alphaNucDist/alphaPotDist
@@ -887,12 +857,108 @@ int build_work(imago_ctx *c) {
   return IMAGO_OK;
 }
 
-constexpr size_t kMaxSiteImageBytes = size_t(4) << 30;
+constexpr size_t kMaxImageListBytes = size_t(4) << 30;
+
+// The images of the potential sites that a shell pair may reach, by type:
+// with a the smallest orbital and a3 the smallest third exponent, a centre
+// lies within sqrt(T / xi) of atom 1 and an image within sqrt(T / mu) of it,
+// the two sharing T, so that |C - A|^2 <= T (1 / xi + 1 / zeta + 1 / a3) <=
+// T (5 / (2 a) + 1 / a3) (screening exponents); atom 1 is in the home cell.
+struct ImageTable {
+  std::vector<double4> pos;
+  std::vector<float4> fpos;
+  std::vector<int> off;
+  double a3_min = 0.0;
+  float margin = 0.f;
+};
+
+void make_images(const imago_ctx *c, ImageTable &tab) {
+  double amin = 1e300, a3 = 1e300;
+  for (int t = 0; t < c->nt; ++t)
+    for (double a : c->types[c->type_screen[t]].alphas) amin = std::min(amin, a);
+  for (int t = 0; t < c->npt; ++t) {
+    const HPType &p = c->ptypes[c->ptype_screen[t]];
+    for (double a : p.alphas) a3 = std::min(a3, a);
+    a3 = std::min(a3, p.nucalpha);
+  }
+  tab.a3_min = a3;
+  double mid[3] = {0, 0, 0}, rho = 0.0, rho_p = 0.0;
+  for (int i = 0; i < c->ns; ++i)
+    for (int x = 0; x < 3; ++x) mid[x] += c->site_pos[3 * i + x] / c->ns;
+  auto from_mid = [&](const double *p) {
+    double d = 0.0;
+    for (int x = 0; x < 3; ++x) d += (p[x] - mid[x]) * (p[x] - mid[x]);
+    return std::sqrt(d);
+  };
+  for (int i = 0; i < c->ns; ++i) rho = std::max(rho, from_mid(&c->site_pos[3 * i]));
+  for (int i = 0; i < c->nps; ++i) rho_p = std::max(rho_p, from_mid(&c->psite_pos[3 * i]));
+  const double rad = (rho + std::sqrt(c->T * (2.5 / amin + 1.0 / a3))) * (1.0 + 1e-9) + 1e-6;
+  // lattice vectors that bring some site into the sphere
+  int lim[3];
+  for (int i = 0; i < 3; ++i) {
+    double n = 0.0;
+    for (int x = 0; x < 3; ++x) n += c->inv[3 * i + x] * c->inv[3 * i + x];
+    lim[i] = (int)std::floor((rad + rho_p) * std::sqrt(n) + 1e-9);
+  }
+  std::vector<std::array<double, 3>> lat;
+  for (int i = -lim[0]; i <= lim[0]; ++i)
+    for (int j = -lim[1]; j <= lim[1]; ++j)
+      for (int k = -lim[2]; k <= lim[2]; ++k) {
+        std::array<double, 3> L;
+        double d = 0.0;
+        for (int x = 0; x < 3; ++x) {
+          L[x] = i * c->rv[x] + j * c->rv[3 + x] + k * c->rv[6 + x];
+          d += L[x] * L[x];
+        }
+        if (d <= (rad + rho_p) * (rad + rho_p)) lat.push_back(L);
+      }
+  double far = 0.0;
+  tab.off.assign(1, 0);
+  for (int t = 0; t < c->npt; ++t) {
+    const HPType &p = c->ptypes[t];
+    for (int q = 0; q < p.mult; ++q) {
+      const double *C = &c->psite_pos[3 * (p.first_site + q)];
+      for (const auto &L : lat) {
+        const double v[3] = {C[0] + L[0], C[1] + L[1], C[2] + L[2]};
+        if (from_mid(v) > rad) continue;
+        tab.pos.push_back(make_double4(v[0], v[1], v[2], 0.0));
+        tab.fpos.push_back(make_float4((float)v[0], (float)v[1], (float)v[2], 0.f));
+        for (int x = 0; x < 3; ++x) far = std::max(far, std::fabs(v[x]));
+      }
+    }
+    tab.off.push_back((int)tab.pos.size());
+  }
+  // float positions and differences: each within 2^-23 of the largest
+  // coordinate, a handful of roundings
+  tab.margin = (float)(1e-4 + 4e-6 * (far + rad));
+}
 
 void set_bloch_width(imago_ctx *c, int wi) {
   c->work.bw = bloch_width(wi);
   c->work.btile_w = c->d_btile_w.p + c->btile_off[wi];
   c->work.nbtile_w = c->btile_off[wi + 1] - c->btile_off[wi];
+}
+
+// The units' image lists; without memory for them (or beyond
+// kMaxImageListBytes) the kernels test every image of a type.
+int build_lists(imago_ctx *c, float margin) {
+  cudaStream_t st = c->stream;
+  DevWork &w = c->work;
+  const size_t nu = (size_t)w.nunits;
+  const char *env = std::getenv("IMAGO_TUNING");
+  if (env && std::strstr(env, "lists=off")) return IMAGO_OK;
+  if (nu == 0 || c->d_uoff.alloc(nu * c->npt, st) || c->d_rad.alloc(nu, st)) return IMAGO_OK;
+  int rc = launch_list_count(c->sys, w, margin, c->d_uoff.p, c->d_rad.p, c->d_queue.p, st);
+  if (rc) return rc;
+  unsigned long long total = 0;
+  IMAGO_CUDA(cudaMemcpyAsync(&total, c->d_queue.p, sizeof total, cudaMemcpyDeviceToHost, st));
+  IMAGO_CUDA(cudaStreamSynchronize(st));
+  if (total * sizeof(ImageRef) > kMaxImageListBytes ||
+      c->d_ulist.alloc(std::max<size_t>(total, 1), st))
+    return IMAGO_OK;
+  w.uoff = c->d_uoff.p;
+  w.ulist = c->d_ulist.p;
+  return launch_list_fill(c->sys, w, margin, c->d_rad.p, c->d_ulist.p, st);
 }
 
 int upload(imago_ctx *c) {
@@ -922,6 +988,15 @@ int upload(imago_ctx *c) {
     pnuc.push_back(p.nucalpha);
     palpha.insert(palpha.end(), p.alphas.begin(), p.alphas.end());
   }
+  std::vector<int> pasc;
+  for (int t = 0; t < c->npt; ++t) {
+    const std::vector<double> &a = c->ptypes[t].alphas;
+    const std::vector<double> &b = c->ptypes[c->ptype_screen[t]].alphas;
+    pasc.push_back(std::is_sorted(a.begin(), a.end()) &&
+                   std::is_sorted(b.begin(), b.begin() + a.size()));
+  }
+  ImageTable tab;
+  make_images(c, tab);
   int rc = 0;
 #define UP(buf, vec) \
   if ((rc = c->buf.upload(vec, st))) return rc;
@@ -933,11 +1008,11 @@ int upload(imago_ctx *c) {
   UP(d_site_cum_core, c->cum_core) UP(d_ptype_z, pz) UP(d_ptype_nucalpha, pnuc)
   UP(d_palpha, palpha) UP(d_ptype_alpha_off, paoff) UP(d_ptype_nalpha, pn)
   UP(d_ptype_first_site, pfirst) UP(d_ptype_mult, pmult)
-  UP(d_ptype_screen, c->ptype_screen) UP(d_psite_pos, c->psite_pos)
-  UP(d_psite_ptype, c->psite_ptype) UP(d_cell, c->cells) UP(d_csize, c->csize)
+  UP(d_ptype_screen, c->ptype_screen) UP(d_cell, c->cells) UP(d_csize, c->csize)
   UP(d_kxyz, c->kxyz) UP(d_pairs, c->pairs) UP(d_units, c->units)
   UP(d_sps, c->sps) UP(d_sp_by_cls, c->sp_by_cls) UP(d_terms, c->ep_terms)
   UP(d_btile, c->btile) UP(d_btile_w, c->btile_w) UP(d_kout, c->kout)
+  UP(d_ptype_ascends, pasc) UP(d_ipos, tab.pos) UP(d_ftab, tab.fpos) UP(d_img_off, tab.off)
 #undef UP
   if ((rc = c->d_queue.alloc(4, st))) return rc;
   if ((rc = c->d_flag.alloc(1, st))) return rc;
@@ -959,7 +1034,8 @@ int upload(imago_ctx *c) {
   s.T = c->T;
   std::memcpy(s.rv, c->rv, sizeof s.rv);
   std::memcpy(s.inv, c->inv, sizeof s.inv);
-  s.far_lattice = 1.5 * smallest_singular(c->rv) * (1.0 - 1e-6);
+  s.a3_min = tab.a3_min;
+  s.ptype_ascends = c->d_ptype_ascends.p;
   s.real_k = 1;
   for (double x : c->kxyz) s.real_k &= x == 0.0;
   s.minus_i = 0;
@@ -974,7 +1050,6 @@ int upload(imago_ctx *c) {
   s.palpha = c->d_palpha.p; s.ptype_alpha_off = c->d_ptype_alpha_off.p;
   s.ptype_nalpha = c->d_ptype_nalpha.p; s.ptype_first_site = c->d_ptype_first_site.p;
   s.ptype_mult = c->d_ptype_mult.p; s.ptype_screen = c->d_ptype_screen.p;
-  s.psite_pos = c->d_psite_pos.p; s.psite_ptype = c->d_psite_ptype.p;
   s.cell = c->d_cell.p; s.csize = c->d_csize.p; s.kxyz = c->d_kxyz.p;
   s.phase = c->d_phase.p;
   s.flag = c->d_flag.p;
@@ -989,26 +1064,13 @@ int upload(imago_ctx *c) {
   w.nbtile = (int)c->btile.size();
   w.btile = c->d_btile.p;
   set_bloch_width(c, kNumBlochWidths - 1);
-  w.simg = nullptr;
-  w.cl_d1 = nullptr;
-  w.site_rank = nullptr;
-  w.ncl = (c->nps + kSiteCluster - 1) / kSiteCluster;
+  w.ipos = c->d_ipos.p;
+  w.ftab = c->d_ftab.p;
+  w.img_off = c->d_img_off.p;
+  w.uoff = nullptr;
+  w.ulist = nullptr;
   if ((rc = launch_phase(s, c->d_phase.p, st))) return rc;
-  // midpoint images of the potential sites, their cluster bounds and each
-  // unit's sites by distance, for the three-centre screens, when the
-  // tables fit in kMaxSiteImageBytes; without them every site is searched
-  // in full
-  const size_t nb = (size_t)w.nunits * c->nps;
-  if (nb > 0 && nb * (sizeof(SiteImage) + sizeof(int)) <= kMaxSiteImageBytes &&
-      c->d_simg.alloc(nb, st) == IMAGO_OK &&
-      c->d_cl_d1.alloc((size_t)w.nunits * w.ncl, st) == IMAGO_OK &&
-      c->d_site_rank.alloc(nb, st) == IMAGO_OK) {
-    w.simg = c->d_simg.p;
-    w.cl_d1 = c->d_cl_d1.p;
-    w.site_rank = c->d_site_rank.p;
-    rc = launch_site_images(s, w, c->d_simg.p, c->d_cl_d1.p, st);
-  }
-  return rc;
+  return build_lists(c, tab.margin);
 }
 
 // Device bytes one term of a build needs between its stages.
@@ -1186,7 +1248,8 @@ void tune_apply(imago_ctx *c) {
 // IMAGO_TUNING fixes measured choices in every context, for profiling
 // runs (a profiler's serialised replays distort the trial timings): a
 // comma-separated list of bloch=32|48|64, sched=per_class|queue|pairs,
-// ortho=per_item|piped, contract=4|8.  Unknown entries are ignored.
+// ortho=per_item|piped, contract=4|8; lists=off does without the image
+// lists (build_lists).  Unknown entries are ignored.
 void tune_from_env(imago_ctx *c) {
   const char *env = std::getenv("IMAGO_TUNING");
   if (!env) return;
@@ -1256,16 +1319,14 @@ int tune_contract(imago_ctx *c, const DevSys &s, const DevWork &w, int nterm,
 }
 
 int launch_prim3c_sched(imago_ctx *c, const DevSys &s, const DevWork &w,
-                        const Term3c *terms, int nterm, bool nuclear, double *blk,
-                        cudaStream_t st) {
+                        const Term3c *terms, int nterm, double *blk, cudaStream_t st) {
   if (c->sched == 1)
-    return launch_prim3c_queue(s, w, c->cls_beg, terms, nterm, nuclear, blk,
-                               c->d_queue.p + c->lane, c->queue_ctas, st);
-  // the same terms on the host, for the pairing of EP terms
-  const Term3c *th = c->sched != 2 || nuclear || c->ep_terms.empty()
-                         ? nullptr
-                         : c->ep_terms.data() + (terms - c->d_terms.p);
-  return launch_prim3c(s, w, c->cls_beg, terms, nterm, nuclear, blk, st, th);
+    return launch_prim3c_queue(s, w, c->cls_beg, terms, nterm, blk, c->d_queue.p + c->lane,
+                               c->queue_ctas, st);
+  if (c->sched == 0) return launch_prim3c(s, w, c->cls_beg, terms, nterm, blk, st);
+  // the same terms on the host, for their grouping
+  return launch_prim3c_terms(s, w, c->cls_beg, terms,
+                             c->ep_terms.data() + (terms - c->d_terms.p), nterm, blk, st);
 }
 
 // The three-centre schedule is picked by measurement, as the phase-sum
@@ -1284,7 +1345,7 @@ int tune_sched(imago_ctx *c, const DevSys &s, const DevWork &w, const Term3c *te
   cudaEventRecord(e[0], st);
   for (int k = 0; k < kNumSchedules && !rc; ++k) {
     c->sched = k;
-    rc = launch_prim3c_sched(c, s, w, terms, nterm, false, blk, st);
+    rc = launch_prim3c_sched(c, s, w, terms, nterm, blk, st);
     cudaEventRecord(e[k + 1], st);
   }
   if (!rc && cudaEventSynchronize(e[kNumSchedules]) != cudaSuccess) rc = IMAGO_ERR_CUDA;
@@ -1356,12 +1417,12 @@ int run_build(imago_ctx *c, Kind kind, int term0, int nterm,
   } else if (kind == KIND_MM || kind == KIND_DM) {
     rc = launch_prim2c_vec(s, w, c->cls_beg, kind == KIND_DM, c->dip_center, S.blk.p, st);
   } else if (kind == KIND_NP) {
-    rc = launch_prim3c_sched(c, s, w, c->d_terms.p, 1, true, S.blk.p, st);
+    rc = launch_prim3c_nuc(s, w, c->cls_beg, S.blk.p, st);
   } else {
     if (c->sched_mode < 0 && !c->sched_tuned && !c->capturing)
       rc = tune_sched(c, s, w, c->d_terms.p + term0, nterm, S.blk.p, st);
     if (!rc)
-      rc = launch_prim3c_sched(c, s, w, c->d_terms.p + term0, nterm, false, S.blk.p, st);
+      rc = launch_prim3c_sched(c, s, w, c->d_terms.p + term0, nterm, S.blk.p, st);
   }
   if (rc) return rc;
   mark(c);
@@ -1617,16 +1678,14 @@ int do_ep(imago_ctx *c, double *packed, int first = 0, int count = -1) {
 // orthoHamPSCF 3913-4043): the potential terms weighted by potCoeffs(potDim,
 // spin), then the kinetic, mass-velocity (rel) and nuclear blocks added.
 // The contraction, phase sum and orthogonalisation are linear, so they then
-// run once per spin instead of once per term.  For one spin the potential
-// terms are summed in registers per shell pair (k_prim3c_ham; four lanes
-// per pair below kHamFusedMinPairs shell pairs, so that a small system
-// fills the GPU); for two spins, which would run that term loop twice, as
-// the EP build's per-term blocks added with their weights (k_block_axpy).
-// imago_intg_set_ham_mode forces either.  Measured on one B200, spin 1:
-// Si8 (62k shell pairs) 2.6 ms fused with four lanes, 4.2 ms with one,
-// 2.9 ms by blocks; 162-atom quartz (1.36M) 37 ms fused, 51 ms by blocks.
-// Two spins: Si8 4.2 ms fused, 3.2 ms by blocks; quartz 70 and 53 ms.
-constexpr long long kHamFusedMinPairs = 300000;
+// run once per spin instead of once per term.  The potential terms are
+// summed in registers per shell pair (k_prim3c_ham, once per spin);
+// imago_intg_set_ham_mode selects the EP build's per-term blocks added with
+// their weights (k_block_axpy) instead.  Lanes per shell pair: Si8 (62k
+// shell pairs) 1.72 / 0.84 / 0.78 ms of primitives with 1 / 4 / 8 lanes
+// (2.07 with a Hermite product per term and triple), Si32 with two spins
+// (230k) 4.68 / 4.16 / 4.37 ms.
+constexpr long long kHamWidePairs = 150000;
 
 int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packed) {
   if (c->core_dim > 0 && !c->have_ol) return IMAGO_ERR_NEED_OVERLAP;
@@ -1639,11 +1698,8 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
   const long long n = c->blk_total;
   if ((rc = c->ham_blk.alloc((size_t)n * spin + 1, st))) return rc;
   if ((rc = c->ham_w.alloc((size_t)c->pot_dim * spin + 1, st))) return rc;
-  const bool fused = c->pot_dim > 0 &&
-                     (c->ham_mode >= 2 || (c->ham_mode == 0 && spin == 1));
-  // a small system's shell pairs get four lanes each
-  const int lanes =
-      c->ham_mode == 3 || (long long)c->sps.size() >= kHamFusedMinPairs ? 1 : 4;
+  const bool fused = c->pot_dim > 0 && c->ham_mode != 1;
+  const int lanes = c->ham_mode == 3 ? 1 : (long long)c->sps.size() >= kHamWidePairs ? 4 : 8;
   const int chunk = fused ? 0 : ep_chunk_size(c);
   if (!fused && (rc = ensure_scratch(c, std::max(chunk, spin)))) return rc;
   if (!fused)
@@ -1664,8 +1720,8 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
   } else {
     for (int t0 = 0; t0 < c->pot_dim; t0 += chunk) {
       const int nt = std::min(chunk, c->pot_dim - t0);
-      if ((rc = launch_prim3c(s, w, c->cls_beg, c->d_terms.p + t0, nt, false, S.blk.p, st,
-                              c->ep_terms.data() + t0)))
+      if ((rc = launch_prim3c_terms(s, w, c->cls_beg, c->d_terms.p + t0,
+                                    c->ep_terms.data() + t0, nt, S.blk.p, st)))
         return rc;
       if ((rc = launch_block_axpy(S.blk.p, nt, n, c->ham_w.p + t0, c->pot_dim, spin,
                                   c->ham_blk.p, st)))
@@ -1680,7 +1736,7 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
     if ((rc = launch_block_axpy(S.blk.p, 1, n, nullptr, 0, spin, c->ham_blk.p, st)))
       return rc;
   }
-  if ((rc = launch_prim3c(s, w, c->cls_beg, c->d_terms.p, 1, true, S.blk.p, st))) return rc;
+  if ((rc = launch_prim3c_nuc(s, w, c->cls_beg, S.blk.p, st))) return rc;
   if ((rc = launch_block_axpy(S.blk.p, 1, n, nullptr, 0, spin, c->ham_blk.p, st))) return rc;
   mark(c);
   if ((rc = launch_contract(s, w, spin, c->ham_blk.p, S.M.p, st))) return rc;

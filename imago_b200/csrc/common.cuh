@@ -18,6 +18,11 @@ constexpr double kPackThresh = 1.0e-10;     // intgOrtho.F90:138-139
 // to l, as lmAlphaIndex classes them: basis.f90:138-146) and the number of
 // Cartesian components behind them.
 __host__ __device__ constexpr int nsh(int l) { return (l + 1) * (l + 1); }
+// Doubles a class's sh block takes in a block buffer: padded so that every
+// block starts on a 32-byte sector.
+__host__ __device__ constexpr int blk_len(int la, int lb) {
+  return (nsh(la) * nsh(lb) + 3) / 4 * 4;
+}
 __host__ __device__ constexpr int ncart(int l) {
   return (l + 1) * (l + 2) * (l + 3) / 6;
 }

@@ -5,108 +5,6 @@
 
 namespace imago {
 
-// Nearest lattice vector to v: round the fractional coordinates, then take
-// the closest of that lattice point and its 26 neighbours.  This is the
-// role of findLatticeVector (lattice.f90:784-888).
-__device__ __forceinline__ void nearest_lattice(const DevSys &s,
-                                                const double v[3],
-                                                double out[3]) {
-  double base[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const double f = v[0] * s.inv[3 * i] + v[1] * s.inv[3 * i + 1] +
-                     v[2] * s.inv[3 * i + 2];
-    double r = (double)(long long)(fabs(f) + 0.5);
-    if (f < 0.0) r = -r;
-#pragma unroll
-    for (int x = 0; x < 3; ++x) base[x] += s.rv[3 * i + x] * r;
-  }
-  double best[3] = {base[0], base[1], base[2]};
-  double bd = 0.0;
-#pragma unroll
-  for (int x = 0; x < 3; ++x) bd += (v[x] - base[x]) * (v[x] - base[x]);
-  for (int i = -1; i <= 1; ++i)
-    for (int j = -1; j <= 1; ++j)
-      for (int k = -1; k <= 1; ++k) {
-        if (!i && !j && !k) continue;
-        double cand[3], d = 0.0;
-#pragma unroll
-        for (int x = 0; x < 3; ++x) {
-          cand[x] = base[x] + i * s.rv[x] + j * s.rv[3 + x] + k * s.rv[6 + x];
-          d += (v[x] - cand[x]) * (v[x] - cand[x]);
-        }
-        if (d < bd * (1.0 - 1e-12)) {
-          bd = d;
-          best[0] = cand[0];
-          best[1] = cand[1];
-          best[2] = cand[2];
-        }
-      }
-  out[0] = best[0];
-  out[1] = best[1];
-  out[2] = best[2];
-}
-
-// Nearest image of potential site `site` to the midpoint of the unit's
-// segment, over the 27 lattice points around the rounded fractional
-// coordinates; every lattice point outside that block is at least
-// far_lattice away, which caps both bounds.  Bounds are shrunk by 1e-9
-// relative and 1e-9 bohr and rounded down to float, so that they stay
-// below the exact distances.
-__device__ __forceinline__ SiteImage site_image(const DevSys &s,
-                                                const DevWork &w, int unit,
-                                                int site) {
-  const DUnit u = w.units[unit];
-  const DPair p = w.pairs[u.pair];
-  double d[3], f[3];
-#pragma unroll
-  for (int x = 0; x < 3; ++x) {
-    const double a = s.site_pos[3 * p.i + x];
-    const double b = s.site_pos[3 * p.j + x] + p.L0[x] + s.cell[3 * u.cell + x];
-    d[x] = 0.5 * (a + b) - s.psite_pos[3 * site + x];
-  }
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-    f[i] = rint(d[0] * s.inv[3 * i] + d[1] * s.inv[3 * i + 1] +
-                d[2] * s.inv[3 * i + 2]);
-  double b1 = 1e300, b2 = 1e300;
-  int n1[3] = {0, 0, 0};
-  for (int i = -1; i <= 1; ++i)
-    for (int j = -1; j <= 1; ++j)
-      for (int k = -1; k <= 1; ++k) {
-        const double c0 = f[0] + i, c1 = f[1] + j, c2 = f[2] + k;
-        double dd = 0.0;
-#pragma unroll
-        for (int x = 0; x < 3; ++x) {
-          const double e = d[x] - (c0 * s.rv[x] + c1 * s.rv[3 + x] + c2 * s.rv[6 + x]);
-          dd += e * e;
-        }
-        if (dd < b1) {
-          b2 = b1;
-          b1 = dd;
-          n1[0] = (int)c0;
-          n1[1] = (int)c1;
-          n1[2] = (int)c2;
-        } else if (dd < b2) {
-          b2 = dd;
-        }
-      }
-  SiteImage r;
-  const bool fits = abs(n1[0]) < 32000 && abs(n1[1]) < 32000 && abs(n1[2]) < 32000;
-  auto lower = [](double dist) {
-    return __double2float_rd(fmax(0.0, dist * (1.0 - 1e-9) - 1e-9));
-  };
-  r.n[0] = fits ? (short)n1[0] : 0;
-  r.n[1] = fits ? (short)n1[1] : 0;
-  r.n[2] = fits ? (short)n1[2] : 0;
-  r.pad = 0;
-  // without a representable image both bounds are 0: the kernels then fall
-  // back to the full search whenever the stored image is out of range
-  r.d1 = fits ? lower(fmin(sqrt(b1), s.far_lattice)) : 0.f;
-  r.d2 = fits ? lower(fmin(sqrt(b2), s.far_lattice)) : 0.f;
-  return r;
-}
-
 // True when a point at least d - pm from every lattice point of interest
 // is certainly outside the screening radius^2 t: the float lower bound of
 // d - pm (pmf >= pm, rounded down) squared, rounded down, exceeds tf >= t.
@@ -115,47 +13,30 @@ __device__ __forceinline__ bool beyond(float d, float pmf, float tf) {
   return a > 0.f && __fmul_rd(a, a) > tf;
 }
 
-// Closest-image search of a three-centre screen (the findLatticeVector step
-// of nuclearPE/electronicPE, integrals.F90:2632,2791) for the point Ps with
-// |Ps - M| = pm, radius^2 t.  Returns false when no image of site C lies
-// within the radius; otherwise sets L2, the lattice vector from which the
-// images in range are enumerated, and v = Ps - C - L2 with |v|^2 <= t.  With
-// the stored midpoint image: no lattice point is nearer to Ps - C than
-// d1 - pm, none but the stored one nearer than d2 - pm.  pmf and tf are
-// float upper bounds of pm and t for those tests.
-__device__ __forceinline__ bool site_search(const DevSys &s, const DevWork &w,
-                                            int unit, int site,
-                                            const double Ps[3], float pmf,
-                                            double t, float tf, double L2[3],
-                                            double v[3], double &c0) {
-  const double *C = s.psite_pos + 3 * site;
-  if (w.simg) {
-    const SiteImage im = w.simg[(long long)unit * s.nps + site];
-    if (beyond(im.d1, pmf, tf)) return false;
-    double c = 0.0;
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-      L2[x] = im.n[0] * s.rv[x] + im.n[1] * s.rv[3 + x] + im.n[2] * s.rv[6 + x];
-      v[x] = Ps[x] - C[x] - L2[x];
-      c += v[x] * v[x];
-    }
-    if (c <= t) {
-      c0 = c;
-      return true;
-    }
-    if (beyond(im.d2, pmf, tf)) return false;
+// The images of one potential type that a unit's shell pairs are tested
+// against: entry r in [beg, end) is image idx(r), at least d1(r) from the
+// unit's midpoint, d1 ascending.
+struct UnitWalk {
+  int beg, end;
+  const ImageRef *list;
+  __device__ __forceinline__ ImageRef at(int r) const {
+    return list ? list[r] : ImageRef{r, 0.f};
   }
-  double d[3];
-#pragma unroll
-  for (int x = 0; x < 3; ++x) d[x] = Ps[x] - C[x];
-  nearest_lattice(s, d, L2);
-  c0 = 0.0;
-#pragma unroll
-  for (int x = 0; x < 3; ++x) {
-    v[x] = Ps[x] - C[x] - L2[x];
-    c0 += v[x] * v[x];
+};
+
+__device__ __forceinline__ UnitWalk unit_walk(const DevSys &s, const DevWork &w, int unit,
+                                              int pt) {
+  if (w.ulist) {
+    const int2 o = w.uoff[(long long)unit * s.npt + pt];
+    return {o.x, o.y, w.ulist};
   }
-  return c0 <= t;
+  return {w.img_off[pt], w.img_off[pt + 1], nullptr};
+}
+
+// v = Ps - C for image position C; returns |v|^2.
+__device__ __forceinline__ double image_d2(const double Ps[3], const double4 &C) {
+  const double x = Ps[0] - C.x, y = Ps[1] - C.y, z = Ps[2] - C.z;
+  return x * x + y * y + z * z;
 }
 
 struct SpGeom {
@@ -185,5 +66,53 @@ __device__ __forceinline__ SpGeom sp_geom(const DevSys &s, const DevWork &w,
   g.r2 = u.r2;
   return g;
 }
+
+// What the three-centre screens need of a shell pair (alphaDist and
+// alphaCenter, gaussRelations.f90:112-131, from the element's first-type
+// exponents, as the reference tables are built), and its product Gaussian.
+struct SpScreen {
+  double Ps[3], Pt[3];   // screening centre, centre of the product
+  double zs, frac;       // a1s + a2s, 1 - r2 / alphaDist
+  double zeta, xi;
+  float pmf;             // at least |Ps - midpoint|
+  // alphaPotDist / alphaNucDist (gaussRelations.f90:187-196, 262-270) for a
+  // third screening exponent a3s: the radius^2 about Ps
+  __device__ __forceinline__ double reach2(double T, double a3s) const {
+    return frac * (T * (zs + a3s) / zs / a3s);
+  }
+};
+
+__device__ __forceinline__ SpScreen sp_screen(const SpGeom &q, double T) {
+  SpScreen r;
+  const double cen = q.a1s / (q.a1s + q.a2s);
+  const double adist = T / q.a2s / cen;
+  r.frac = 1 - q.r2 / adist;
+  r.zs = q.a1s + q.a2s;
+  r.zeta = q.a1 + q.a2;
+  r.xi = q.a1 * q.a2 / r.zeta;
+  double pm = 0.0;
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    r.Ps[x] = cen * (q.A[x] - q.B[x]) + q.B[x];
+    r.Pt[x] = (q.a1 * q.A[x] + q.a2 * q.B[x]) / r.zeta;
+    const double e = r.Ps[x] - 0.5 * (q.A[x] + q.B[x]);
+    pm += e * e;
+  }
+  r.pmf = __double2float_ru(sqrt(pm));
+  return r;
+}
+
+// The Hermite accumulators of the T adjacent lanes that share a shell pair,
+// added by warp shuffles (every lane of the warp calls it).
+template <int L, int T>
+__device__ __forceinline__ void team_sum(double Q[nherm(L)]) {
+#pragma unroll
+  for (int off = T / 2; off > 0; off /= 2)
+#pragma unroll
+    for (int i = 0; i < nherm(L); ++i) Q[i] += __shfl_xor_sync(0xffffffffu, Q[i], off);
+}
+
+#define IMAGO_FOR_SPD_CLASSES(M) \
+  M(0, 0) M(0, 1) M(0, 2) M(1, 0) M(1, 1) M(1, 2) M(2, 0) M(2, 1) M(2, 2)
 
 }  // namespace imago

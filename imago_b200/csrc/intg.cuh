@@ -23,9 +23,6 @@ struct DevSys {
   double T;            // logBasisFnThresh = -ln(basisFnConvg)
   double rv[9];        // realVectors [abc*3 + xyz]
   double inv[9];       // invRealVectors [abc*3 + xyz]
-  // 1.5 x the smallest singular value of realVectors: every lattice point
-  // outside the 3x3x3 block around a rounded point is at least this far
-  double far_lattice;
   // every k-point is Gamma: all phases are exactly 1, every matrix is real,
   // and the orthogonalisation runs on the real parts only
   int real_k;
@@ -46,8 +43,10 @@ struct DevSys {
   const double *ptype_z, *ptype_nucalpha, *palpha;
   const int *ptype_alpha_off, *ptype_nalpha, *ptype_first_site, *ptype_mult,
       *ptype_screen;
-  const double *psite_pos;
-  const int *psite_ptype;
+  // 1 where the type's exponents and its screening exponents ascend, so
+  // that the screening radius falls from term to term
+  const int *ptype_ascends;
+  double a3_min;          // smallest screening exponent of any third centre
   // lattice cells sorted by |R|^2, k-points, phase table
   const double *cell;     // [n*3]
   const double *csize;    // [n]
@@ -82,6 +81,14 @@ struct DSp {
   long long boff;         // offset of its sh block in a term's block buffer
 };
 
+// An image (index into DevWork::ipos) and a lower bound, rounded down to the
+// list's distance step, of its distance from the unit's midpoint; the bound
+// never falls along a list.
+struct __align__(8) ImageRef {
+  int idx;
+  float d1;
+};
+
 struct DevWork {
   int npairs, nunits, nsp;
   const DPair *pairs;
@@ -95,31 +102,18 @@ struct DevWork {
   int bw;                 // column width of the tensor-core phase sum
   int nbtile_w;           // its tiles: (pair, tile of bw columns)
   const int2 *btile_w;
-  // [unit * nps + site]: the potential site's nearest image to the midpoint
-  // of the unit's A-B segment (null: every site is searched in full)
-  const struct SiteImage *simg;
-  // [unit * ncl + c]: the smallest d1 of sites kSiteCluster*c .. +7 (null
-  // with simg)
-  const float *cl_d1;
-  int ncl;
-  // [unit * nps + first site of type + r]: the r-th site of the type in
-  // ascending d1 for that unit, as an offset within the type (null with
-  // simg)
-  const int *site_rank;
-};
-
-// Consecutive potential sites screened together before their own tests.
-constexpr int kSiteCluster = 8;
-
-// Nearest image of a potential site C to the midpoint M of a unit's A-B
-// segment: M - C - (n0 a + n1 b + n2 c) is shortest for lattice coordinates
-// n; d1 and d2 are lower bounds of the distance from M - C to that lattice
-// point and to every other one.  16 bytes, so that the table of a large
-// cell stays compact.
-struct __align__(16) SiteImage {
-  short n[3];
-  short pad;
-  float d1, d2;
+  // Every lattice image of a potential site that some shell pair may reach,
+  // ordered by type, then site: ipos[i] its position, ftab[i] the same in
+  // float, img_off[t] the first image of type t (npt + 1 entries)
+  const double4 *ipos;
+  const float4 *ftab;
+  const int *img_off;
+  // For each (unit, type), at unit * npt + type, its range of `ulist`: the
+  // images within reach of the unit's shell pairs in ascending order of
+  // distance from the midpoint of its A-B segment, in 64 steps of the
+  // reach (null: every image of the type is tested)
+  const int2 *uoff;
+  const ImageRef *ulist;
 };
 
 // Columns (block elements) per CTA of the register phase sum, and the
@@ -149,7 +143,7 @@ int launch_prim2c(const DevSys &s, const DevWork &w, const int *cls_beg,
                   int op, double *blk, cudaStream_t st);
 // The PSCF Hamiltonian's potential terms for one spin, summed in registers
 // per shell pair: H = sum_t coef[t] EP_t (sh blocks, written, not added).
-// lanes (1 or 4) threads share a shell pair's terms (s, p, d classes).
+// lanes (1, 4 or 8) threads share a shell pair's images (s, p, d classes).
 int launch_prim3c_ham(const DevSys &s, const DevWork &w, const int *cls_beg,
                       const Term3c *terms_dev, int nterm, const double *coef,
                       int lanes, double *H, cudaStream_t st);
@@ -180,18 +174,15 @@ int launch_prim2c_vec(const DevSys &s, const DevWork &w, const int *cls_beg,
 // The classes of one three-centre build in work-queue order: class code
 // la * 4 + lb, first entry of its shell-pair list, count, and the first
 // queue item of each class (off[ncls] is the total).
-// Consecutive EP terms of one potential type evaluated by one thread, so
-// that they share the site and image walk: group g is terms first[g] ..
-// first[g] + count[g] - 1 of a launch's term list.
+// EP terms that one thread evaluates in turn: group g is the count[g]
+// terms first[g], first[g] + stride, ... of a launch's term list, all of
+// one potential type.
 constexpr int kMaxTermGroups = 64;
 struct TermGroups {
-  int n;
+  int n, stride;
   unsigned short first[kMaxTermGroups];
-  unsigned char count[kMaxTermGroups];
+  unsigned short count[kMaxTermGroups];
 };
-// Pairs of consecutive terms of one type (a single term where a type's
-// count is odd); n = 0 when there would be more than kMaxTermGroups.
-TermGroups term_pairs(const Term3c *terms_host, int nterm);
 
 struct Prim3cQueue {
   int ncls;
@@ -199,11 +190,11 @@ struct Prim3cQueue {
   long long off[17];
 };
 
-// All classes of a three-centre build in one persistent launch of `ctas`
-// CTAs fed by a device counter (8 bytes at `counter`, zeroed here on the
-// stream before the launch).
+// All classes of an EP build in one persistent launch of `ctas` CTAs fed by
+// a device counter (8 bytes at `counter`, zeroed here on the stream before
+// the launch).
 int launch_prim3c_queue(const DevSys &s, const DevWork &w, const int *cls_beg,
-                        const Term3c *terms_dev, int nterm, bool nuclear, double *blk,
+                        const Term3c *terms_dev, int nterm, double *blk,
                         unsigned long long *counter, int ctas, cudaStream_t st);
 // CTAs of k_prim3c_queue resident per SM.
 int prim3c_queue_ctas_per_sm();
@@ -213,11 +204,25 @@ int launch_prim3c_count(const DevSys &s, const DevWork &w, const int *cls_beg,
                         const Term3c *terms_dev, int nterm, bool nuclear,
                         unsigned long long *count16, cudaStream_t st);
 
-// terms_host (the same list on the host): EP classes up to d-p run two
-// terms of a type per thread (k_prim3c_pair); null: one term per thread.
+// EP terms, one launch per class, one (shell pair, term) per thread.
 int launch_prim3c(const DevSys &s, const DevWork &w, const int *cls_beg,
-                  const Term3c *terms_dev, int nterm, bool nuclear,
-                  double *blk, cudaStream_t st, const Term3c *terms_host = nullptr);
+                  const Term3c *terms_dev, int nterm, double *blk, cudaStream_t st);
+// EP terms, one launch per class, a thread taking several terms of a type
+// of its shell pair (terms_host: the same list on the host).
+int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
+                        const Term3c *terms_dev, const Term3c *terms_host, int nterm,
+                        double *blk, cudaStream_t st);
+// The f classes of the EP terms (terms_dev) or of the nuclear term.
+int launch_prim3c_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
+                     const Term3c *terms_dev, int nterm, bool nuclear, double *blk,
+                     cudaStream_t st);
+// The f classes of launch_prim3c_ham.
+int launch_prim3c_ham_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
+                         const Term3c *terms_dev, int nterm, const double *coef, double *H,
+                         cudaStream_t st);
+// The nuclear term (all potential types), several lanes per shell pair.
+int launch_prim3c_nuc(const DevSys &s, const DevWork &w, const int *cls_beg, double *blk,
+                      cudaStream_t st);
 // terms_per_cta: 4 or 8 EP terms per CTA (builds of up to 4 terms use 4)
 int launch_contract(const DevSys &s, const DevWork &w, int nterm,
                     const double *blk, double *M, cudaStream_t st, int terms_per_cta = 4);
@@ -249,8 +254,13 @@ int launch_split_cv(const DevSys &s, const double2 *cv, double *re, double *im,
 // not related by conjugation.
 int launch_conj_cv(const DevSys &s, int npair, double2 *cv, cudaStream_t st);
 int launch_phase(const DevSys &s, double2 *phase, cudaStream_t st);
-int launch_site_images(const DevSys &s, const DevWork &w, SiteImage *simg,
-                       float *cl_d1, cudaStream_t st);
+// The image lists: count gives every (unit, type) its range in `uoff`, taken
+// from *cursor (zeroed here), and each unit's reach in `rad`; fill writes
+// the entries.  `margin` bounds the error of a float distance.
+int launch_list_count(const DevSys &s, const DevWork &w, float margin, int2 *uoff,
+                      float *rad, unsigned long long *cursor, cudaStream_t st);
+int launch_list_fill(const DevSys &s, const DevWork &w, float margin, const float *rad,
+                     ImageRef *list, cudaStream_t st);
 int launch_prim_eval(int kind, int n, const double *params, const int *cls,
                      double *sh, cudaStream_t st);
 

@@ -8,7 +8,7 @@ namespace imago {
 // ---------------------------------------------------------- prim_eval --
 // Single primitives for checking against the reference's kernels.
 template <int LA, int LB>
-__device__ void eval_one(int kind, const double *p, double *out) {
+__device__ __noinline__ void eval_one(int kind, const double *p, double *out) {
   constexpr int L = LA + LB;
   const double a1 = p[0], a2 = p[1], a3 = p[2];
   const double *A = p + 3, *B = p + 6, *C = p + 9;
@@ -45,7 +45,7 @@ __device__ void eval_one(int kind, const double *p, double *out) {
 }
 
 template <int LA, int LB>
-__device__ void eval_mv(const double *p, double *out) {
+__device__ __noinline__ void eval_mv(const double *p, double *out) {
   double blk[nsh(LA) * nsh(LB)];
   prim_mv<LA, LB>(p[0], p[1], p + 3, p + 6, kMassVelPref, blk);
   for (int i = 0; i < 256; ++i) out[i] = 0.0;
@@ -58,7 +58,7 @@ __device__ void eval_mv(const double *p, double *out) {
 // routine: the build kernels' unrolled s/p/d variants share its arithmetic
 // (vec_factor, the same tables) and are checked by the build tests.
 template <bool DIP>
-__device__ void eval_vec_rt(int la, int lb, int comp, const double *p, double *out) {
+__device__ __noinline__ void eval_vec_rt(int la, int lb, int comp, const double *p, double *out) {
   const int nb = nsh(la) * nsh(lb);
   double blk[3 * 256];
   prim_vec_rt<DIP>(la, lb, p[0], p[1], p + 3, p + 6, p + 9, blk, nb);

@@ -1,0 +1,298 @@
+// k_terms.cu -- the three-centre primitive stage: the image lists of its
+// screens and the electronic-potential terms of a shell pair walked
+// together.
+#include <algorithm>
+
+#include "geom.cuh"
+#include "prim.cuh"
+
+namespace imago {
+
+// ------------------------------------------------------- image lists --
+// One warp per unit.  The unit's reach is the largest |Ps - M| + sqrt(t)
+// over its shell pairs (t for the smallest third exponent), M the midpoint
+// of its A-B segment; an image belongs to the unit's list when its float
+// distance from M, less the margin that bounds the float error, is within
+// that reach.  Entries are placed in kListBins steps of the reach, in table
+// order inside a step, and carry the lower edge of their step: a walk may
+// stop at the first entry whose edge is beyond its own reach.  The list
+// replaces a nearest-image search per (shell pair, term, site) and the loop
+// over lattice cells behind it (the walk alone was 15 of the 35 ms of the
+// 162-atom quartz EP primitives).
+constexpr int kListBins = 64;
+constexpr int kListWarps = 8;
+
+__device__ __forceinline__ float3 unit_mid(const DevSys &s, const DevWork &w, const DUnit &u) {
+  const DPair p = w.pairs[u.pair];
+  float m[3];
+#pragma unroll
+  for (int x = 0; x < 3; ++x)
+    m[x] = (float)(0.5 * (s.site_pos[3 * p.i + x] + s.site_pos[3 * p.j + x] + p.L0[x] +
+                          s.cell[3 * u.cell + x]));
+  return make_float3(m[0], m[1], m[2]);
+}
+
+__device__ __forceinline__ float list_dist(const float4 &c, const float3 &m, float margin) {
+  const float x = c.x - m.x, y = c.y - m.y, z = c.z - m.z;
+  return fmaxf(0.f, sqrtf(x * x + y * y + z * z) - margin);
+}
+
+__global__ void __launch_bounds__(32 * kListWarps)
+    k_list_count(DevSys s, DevWork w, float margin, int2 *uoff, float *rad,
+                 unsigned long long *cursor) {
+  const int lane = threadIdx.x & 31;
+  const int nw = gridDim.x * kListWarps;
+  for (int ui = blockIdx.x * kListWarps + (threadIdx.x >> 5); ui < w.nunits; ui += nw) {
+    const DUnit u = w.units[ui];
+    const DPair p = w.pairs[u.pair];
+    const double *as1 = s.alpha + s.type_alpha_off[s.type_screen[p.ti]];
+    const double *as2 = s.alpha + s.type_alpha_off[s.type_screen[p.tj]];
+    const double r = sqrt(u.r2);
+    double reach = 0.0;
+    for (int q = u.spbeg + lane; q < u.spend; q += 32) {
+      const DSp sp = w.sps[q];
+      const double a = as1[sp.a], b = as2[sp.b], z = a + b;
+      const double frac = fmax(0.0, 1.0 - u.r2 * (a * b / z) / s.T);
+      const double t = frac * s.T * (z + s.a3_min) / (z * s.a3_min);
+      reach = fmax(reach, fabs(a / z - 0.5) * r + sqrt(t));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) reach = fmax(reach, __shfl_xor_sync(0xffffffffu, reach, o));
+    // rounding of the formulas above against the screens' own
+    const float R = __double2float_ru(reach * (1.0 + 1e-9) + 1e-6);
+    const float3 m = unit_mid(s, w, u);
+    int2 *out = uoff + (long long)ui * s.npt;
+    int run = 0;
+    for (int pt = 0; pt < s.npt; ++pt) {
+      int n = 0;
+      for (int i = w.img_off[pt] + lane; i < w.img_off[pt + 1]; i += 32)
+        n += list_dist(w.ftab[i], m, margin) <= R;
+      n = __reduce_add_sync(0xffffffffu, n);
+      if (lane == 0) out[pt] = make_int2(run, run + n);
+      run += n;
+    }
+    // the units' ranges in the order they come by; their contents do not
+    // depend on it
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(cursor, (unsigned long long)run);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    __syncwarp();
+    for (int pt = lane; pt < s.npt; pt += 32) {
+      const int2 o = out[pt];
+      out[pt] = make_int2((int)(base + o.x), (int)(base + o.y));
+    }
+    if (lane == 0) rad[ui] = R;
+  }
+}
+
+__global__ void __launch_bounds__(32 * kListWarps)
+    k_list_fill(DevSys s, DevWork w, float margin, const float *rad, ImageRef *list) {
+  __shared__ int bins[kListWarps][kListBins];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = gridDim.x * kListWarps;
+  int *bin = bins[warp];
+  for (int ui = blockIdx.x * kListWarps + warp; ui < w.nunits; ui += nw) {
+    const DUnit u = w.units[ui];
+    const float3 m = unit_mid(s, w, u);
+    const float R = rad[ui], step = R / kListBins, inv = kListBins / R;
+    for (int pt = 0; pt < s.npt; ++pt) {
+      const int i0 = w.img_off[pt], i1 = w.img_off[pt + 1];
+      bin[lane] = bin[lane + 32] = 0;
+      __syncwarp();
+      for (int i = i0 + lane; i < i1; i += 32) {
+        const float d = list_dist(w.ftab[i], m, margin);
+        if (d <= R) atomicAdd(&bin[min(kListBins - 1, (int)(d * inv))], 1);
+      }
+      __syncwarp();
+      // exclusive prefix over the steps, two per lane
+      const int c0 = bin[2 * lane], c1 = bin[2 * lane + 1];
+      int sum = c0 + c1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += x;
+      }
+      __syncwarp();
+      bin[2 * lane] = sum - c0 - c1;
+      bin[2 * lane + 1] = sum - c1;
+      __syncwarp();
+      ImageRef *out = list + w.uoff[(long long)ui * s.npt + pt].x;
+      for (int ib = i0; ib < i1; ib += 32) {
+        const int i = ib + lane;
+        const float d = i < i1 ? list_dist(w.ftab[i], m, margin) : 0.f;
+        const bool in = i < i1 && d <= R;
+        const int b = in ? min(kListBins - 1, (int)(d * inv)) : -1 - lane;
+        const unsigned peers = __match_any_sync(0xffffffffu, b);
+        if (in) {
+          const int pos = bin[b] + __popc(peers & ((1u << lane) - 1));
+          // the step's lower edge, rounded to stay below d
+          out[pos] = ImageRef{i, b * step * (1.f - 1e-5f)};
+        }
+        __syncwarp();
+        if (in && (peers >> lane) == 1u) bin[b] += __popc(peers);
+        __syncwarp();
+      }
+      __syncwarp();
+    }
+  }
+}
+
+int launch_list_count(const DevSys &s, const DevWork &w, float margin, int2 *uoff, float *rad,
+                      unsigned long long *cursor, cudaStream_t st) {
+  IMAGO_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), st));
+  if (w.nunits == 0) return IMAGO_OK;
+  const int grid = std::min((w.nunits + kListWarps - 1) / kListWarps, 148 * 8);
+  k_list_count<<<grid, 32 * kListWarps, 0, st>>>(s, w, margin, uoff, rad, cursor);
+  IMAGO_CUDA(cudaGetLastError());
+  return IMAGO_OK;
+}
+
+int launch_list_fill(const DevSys &s, const DevWork &w, float margin, const float *rad,
+                     ImageRef *list, cudaStream_t st) {
+  if (w.nunits == 0) return IMAGO_OK;
+  const int grid = std::min((w.nunits + kListWarps - 1) / kListWarps, 148 * 8);
+  k_list_fill<<<grid, 32 * kListWarps, 0, st>>>(s, w, margin, rad, list);
+  IMAGO_CUDA(cudaGetLastError());
+  return IMAGO_OK;
+}
+
+// ---------------------------------------------------------- EP terms --
+// One thread per (shell pair, group of terms of one potential type).  The
+// geometry, the screening quantities and the product Gaussian are formed
+// once for the group.  The first terms, the most diffuse, walk the unit's
+// image list; while doing so a thread notes the images that the next term
+// still reaches, and as soon as every lane of the warp could note all of
+// its own (kTermCap), the following terms run over the notes, each term
+// striking out what it no longer reaches.  Every lane then works on an
+// image of its own at each step, where a walk has the warp wait at images
+// that only some lanes reach.  The triples of a term are exactly those of
+// its own walk.
+constexpr int kTermThreads = 128;
+constexpr int kTermCap = 64;
+
+template <int LA, int LB>
+__global__ void __launch_bounds__(kTermThreads, LA + LB >= 4 ? 3 : (LA + LB >= 3 ? 4 : 5))
+    k_prim3c_terms(DevSys s, DevWork w, int beg, int n, const Term3c *terms, TermGroups tg,
+                   double *blk) {
+  constexpr int L = LA + LB;
+  __shared__ int note[kTermCap][kTermThreads];
+  const int tid = threadIdx.x;
+  const long long g = (long long)blockIdx.x * kTermThreads + tid;
+  const bool live = g < (long long)n * tg.n;
+  const int gi = live ? (int)(g / n) : 0;
+  const int t0 = tg.first[gi], cnt = live ? tg.count[gi] : 0;
+  const DSp sp = w.sps[w.sp_by_cls[beg + (live ? (int)(g % n) : 0)]];
+  const SpGeom q = sp_geom(s, w, sp);
+  const SpScreen c = sp_screen(q, s.T);
+  const int pt = terms[t0].ptype;
+  const double *al = s.palpha + s.ptype_alpha_off[pt];
+  const double *als = s.palpha + s.ptype_alpha_off[s.ptype_screen[pt]];
+  const bool ascends = s.ptype_ascends[pt];
+  const UnitWalk uw = unit_walk(s, w, sp.unit, pt);
+  const double ex = exp(-c.xi * q.r2);
+  bool have = false;  // the notes hold every image of this and later terms
+  int nn = 0;
+  double t = cnt > 0 ? c.reach2(s.T, als[terms[t0].j]) : -1.0;
+  for (int it = 0; __any_sync(0xffffffffu, it < cnt); ++it) {
+    const bool on = it < cnt;
+    const double a3 = on ? al[terms[t0 + it * tg.stride].j] : 1.0;
+    const double tn = it + 1 < cnt ? c.reach2(s.T, als[terms[t0 + (it + 1) * tg.stride].j]) : -1.0;
+    const double z3 = c.zeta + a3, mu = c.zeta * a3 / z3;
+    double Q[nherm(L)];
+#pragma unroll
+    for (int i = 0; i < nherm(L); ++i) Q[i] = 0.0;
+    if (__all_sync(0xffffffffu, have || !on)) {
+      int keep = 0;
+      for (int i = 0; i < nn; ++i) {
+        const int id = note[i][tid];
+        const double4 C = w.ipos[id];
+        if (image_d2(c.Ps, C) > t) continue;
+        note[keep++][tid] = id;
+        const double X[3] = {c.Pt[0] - C.x, c.Pt[1] - C.y, c.Pt[2] - C.z};
+        accumulate_overlap_q<L>(X, mu, 1.0, Q);
+      }
+      nn = keep;
+    } else if (on) {
+      const float tf = __double2float_ru(t);
+      nn = 0;
+      for (int r = uw.beg; r < uw.end; ++r) {
+        const ImageRef e = uw.at(r);
+        if (beyond(e.d1, c.pmf, tf)) break;
+        const double4 C = w.ipos[e.idx];
+        const double d2 = image_d2(c.Ps, C);
+        if (d2 > t) continue;
+        if (d2 <= tn) {
+          if (nn < kTermCap) note[nn][tid] = e.idx;
+          ++nn;
+        }
+        const double X[3] = {c.Pt[0] - C.x, c.Pt[1] - C.y, c.Pt[2] - C.z};
+        accumulate_overlap_q<L>(X, mu, 1.0, Q);
+      }
+      have = ascends && nn <= kTermCap;
+    }
+    if (on) {
+      const double pz = kPi / z3;
+      hermite_to_sh<LA, LB, true>(
+          q.A, q.B, q.a1, q.a2, pz * sqrt(pz) * ex, Q,
+          blk + (long long)(t0 + it * tg.stride) * w.blk_total + sp.boff);
+    }
+    t = tn;
+  }
+}
+
+// Term groups of one launch: the terms from `from` on, split into runs of
+// one potential type and each run into `split` interleaved groups, at most
+// kMaxTermGroups of them.  Returns the first term not covered.
+static int group_terms(const Term3c *terms, int nterm, int from, int split, TermGroups &tg) {
+  tg.n = 0;
+  tg.stride = split;
+  int i = from;
+  while (i < nterm) {
+    int e = i + 1;
+    while (e < nterm && terms[e].ptype == terms[i].ptype && e - i < 65535) ++e;
+    const int k = std::min(split, e - i);
+    if (tg.n + k > kMaxTermGroups) break;
+    for (int h = 0; h < k; ++h) {
+      tg.first[tg.n] = (unsigned short)(i - from + h);
+      tg.count[tg.n] = (unsigned short)((e - i - h + split - 1) / split);
+      ++tg.n;
+    }
+    i = e;
+  }
+  return i;
+}
+
+// Threads that the widest class launch should at least have: a GPU of 148
+// SMs holds 75,000 to 95,000 of this kernel's, and the images of a thread's
+// terms differ enough that a few rounds even them out.
+constexpr long long kTermThreadsWanted = 400000;
+
+int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
+                        const Term3c *terms_dev, const Term3c *terms_host, int nterm,
+                        double *blk, cudaStream_t st) {
+  int runs = 0;
+  for (int i = 0; i < nterm; ++i) runs += i == 0 || terms_host[i].ptype != terms_host[i - 1].ptype;
+  const long long base = std::max(1LL, (long long)w.nsp * std::max(1, runs));
+  const int split = (int)std::min<long long>(8, (kTermThreadsWanted + base - 1) / base);
+  for (int from = 0; from < nterm;) {
+    TermGroups tg;
+    const int next = group_terms(terms_host + from, nterm - from, 0, split, tg) + from;
+    double *b = blk + (long long)from * w.blk_total;
+#define IMAGO_PT(a, c)                                                                     \
+  {                                                                                       \
+    const int beg = cls_beg[a * 4 + c], n = cls_beg[a * 4 + c + 1] - beg;                 \
+    if (n > 0) {                                                                          \
+      const unsigned grid = (unsigned)(((long long)n * tg.n + kTermThreads - 1) / kTermThreads); \
+      k_prim3c_terms<a, c><<<grid, kTermThreads, 0, st>>>(s, w, beg, n, terms_dev + from, tg, b); \
+      IMAGO_CUDA(cudaGetLastError());                                                     \
+    }                                                                                     \
+  }
+    IMAGO_PT(2, 2) IMAGO_PT(1, 2) IMAGO_PT(2, 1) IMAGO_PT(1, 1) IMAGO_PT(0, 2) IMAGO_PT(2, 0)
+    IMAGO_PT(0, 1) IMAGO_PT(1, 0) IMAGO_PT(0, 0)
+#undef IMAGO_PT
+    from = next;
+  }
+  return launch_prim3c_rt(s, w, cls_beg, terms_dev, nterm, false, blk, st);
+}
+
+}  // namespace imago

@@ -60,8 +60,11 @@ __device__ __forceinline__ void boys_ref(double T, double F[NMAX + 1]) {
     }
     return;
   }
-  const double erf_T = erf(sqrt(T));
-  F[0] = 0.5 * ((sqrt_pi / pow(T, 0.5)) * erf_T);
+  // T^(m + 1/2) as sqrt(T) times the product form of T^m: a pow costs as
+  // much as the rest of an order
+  const double root_T = sqrt(T);
+  const double erf_T = erf(root_T);
+  F[0] = 0.5 * ((sqrt_pi / root_T) * erf_T);
   const double T2 = T * T, T3 = T2 * T;
   const double Tp[7] = {1.0, T, T2, T3, T2 * T2, T3 * T2, T3 * T3};
   const double fact[13] = {1, 1, 2, 6, 24, 120, 720, 5040, 40320, 362880,
@@ -71,7 +74,7 @@ __device__ __forceinline__ void boys_ref(double T, double F[NMAX + 1]) {
   for (int m = 1; m <= NMAX; ++m) {
     if (m > 1) c *= (double)(4 * m - 2);
     p4m *= 4.0;
-    double erfterm = (sqrt_pi / (p4m * pow(T, (double)m + 0.5))) * erf_T;
+    double erfterm = (sqrt_pi / (p4m * (root_T * Tp[m]))) * erf_T;
     double s = 0.0, p4k = 1.0;
 #pragma unroll
     for (int k = 1; k <= m; ++k) {
@@ -108,10 +111,21 @@ __device__ __forceinline__ void os1d(double PA, double PB, double inv2p,
     }
 }
 
+// Four doubles in one 32-byte store (one whole sector; 32-byte aligned).
+__device__ __forceinline__ void store4(double *p, const double v[4]) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]),
+               "d"(v[2]), "d"(v[3])
+               : "memory");
+}
+
 // Write the real-solid-harmonic block from a Cartesian block
-// pc[p * ncart(LB) + q].
-template <int LA, int LB>
+// pc[p * ncart(LB) + q].  PAD: to a build's block buffer, where every block
+// starts on 32 bytes and has blk_len doubles: each thread writes its own
+// block, so single 8-byte stores would send one partial sector each (162-atom
+// quartz EP: 2.0 G of them; the whole-sector stores are a quarter).
+template <int LA, int LB, bool PAD = false>
 __device__ __forceinline__ void cart_to_sh(const double *pc, double *out) {
+  double quad[4];
 #pragma unroll
   for (int s1 = 0; s1 < nsh(LA); ++s1)
 #pragma unroll
@@ -127,7 +141,19 @@ __device__ __forceinline__ void cart_to_sh(const double *pc, double *out) {
                pc[sh_cart(s1, k1) * ncart(LB) + sh_cart(s2, k2)];
         }
       }
-      out[s1 * nsh(LB) + s2] = v;
+      const int o = s1 * nsh(LB) + s2;
+      if (!PAD) {
+        out[o] = v;
+        continue;
+      }
+      quad[o & 3] = v;
+      if (o == nsh(LA) * nsh(LB) - 1) {
+#pragma unroll
+        for (int i = (o & 3) + 1; i < 4; ++i) quad[i] = 0.0;
+        store4(out + (o & ~3), quad);
+      } else if ((o & 3) == 3) {
+        store4(out + (o & ~3), quad);
+      }
     }
 }
 
@@ -423,12 +449,52 @@ __device__ __forceinline__ void accumulate_overlap_q(const double X[3],
     }
 }
 
+// Add d^{tuv}/dX^{tuv} of a radial function f(|X|^2) to Q, t + u + v <= L <=
+// 4, from G_n = (2 d/d|X|^2)^n f: with the one-axis coefficients
+//   c(t, i) = t! / (2^i i! (t - 2i)!),
+//   d^{tuv} f = sum_ijk c(t, i) c(u, j) c(v, k) X^{t-2i} Y^{u-2j} Z^{v-2k}
+//               G_{t+u+v-i-j-k},
+// which needs no intermediate orders in registers.
+__host__ __device__ constexpr double radial_coef(int t, int i) {
+  constexpr double c[5][3] = {{1, 0, 0}, {1, 0, 0}, {1, 1, 0}, {1, 3, 0}, {1, 6, 3}};
+  return c[t][i];
+}
+
+template <int L>
+__device__ __forceinline__ void accumulate_radial_q(const double X[3], const double G[L + 1],
+                                                    double Q[nherm(L)]) {
+  double p[3][L + 1];
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    p[x][0] = 1.0;
+#pragma unroll
+    for (int t = 0; t < L; ++t) p[x][t + 1] = p[x][t] * X[x];
+  }
+#pragma unroll
+  for (int t = 0; t <= L; ++t)
+#pragma unroll
+    for (int u = 0; u <= L - t; ++u)
+#pragma unroll
+      for (int v = 0; v <= L - t - u; ++v) {
+        double sum = 0.0;
+#pragma unroll
+        for (int i = 0; 2 * i <= t; ++i)
+#pragma unroll
+          for (int j = 0; 2 * j <= u; ++j)
+#pragma unroll
+            for (int k = 0; 2 * k <= v; ++k)
+              sum += radial_coef(t, i) * radial_coef(u, j) * radial_coef(v, k) *
+                     (p[0][t - 2 * i] * p[1][u - 2 * j] * p[2][v - 2 * k]) *
+                     G[t + u + v - i - j - k];
+        Q[herm_index(t, u, v)] += sum;
+      }
+}
+
 // Accumulate one nuclear term: w * d^{tuv}/dX^{tuv} of
 // f(X) = exp(-mu |X|^2) F_0(nu |X|^2), the Gaussian-damped Coulomb
 // potential integrated against the Hermite Gaussian of exponent p about P.
-// With f = int_0^1 exp(-(mu + nu s^2)|X|^2) ds the Hermite recursion
-//   R^n_{t+1,u,v} = t R^{n+1}_{t-1,u,v} + X R^{n+1}_{t,u,v}
-// starts from R^n_000 = (-2)^n exp(-mu|X|^2) sum_k C(n,k) mu^{n-k} nu^k F_k.
+// With f = int_0^1 exp(-(mu + nu s^2)|X|^2) ds,
+//   G_n = (-2)^n exp(-mu|X|^2) sum_k C(n,k) mu^{n-k} nu^k F_k.
 template <int L>
 __device__ __forceinline__ void accumulate_nuclear_q(const double X[3],
                                                      double mu, double nu,
@@ -438,61 +504,33 @@ __device__ __forceinline__ void accumulate_nuclear_q(const double X[3],
   double F[L + 1];
   boys_ref<L>(nu * r2, F);
   const double g = w * exp(-mu * r2);
-  double R[L + 1][nherm(L)];
-  // R^n_000
-  {
-    double mpow[L + 1], npow[L + 1];
-    mpow[0] = 1.0;
-    npow[0] = 1.0;
+  double G[L + 1];
+  double mpow[L + 1], npow[L + 1];
+  mpow[0] = 1.0;
+  npow[0] = 1.0;
 #pragma unroll
-    for (int n = 1; n <= L; ++n) {
-      mpow[n] = mpow[n - 1] * mu;
-      npow[n] = npow[n - 1] * nu;
-    }
-    double sgn = 1.0;
-#pragma unroll
-    for (int n = 0; n <= L; ++n) {
-      double s = 0.0, binom = 1.0;
-#pragma unroll
-      for (int k = 0; k <= n; ++k) {
-        s += binom * mpow[n - k] * npow[k] * F[k];
-        binom = binom * (n - k) / (k + 1);
-      }
-      R[n][0] = sgn * g * s;
-      sgn *= -2.0;
-    }
+  for (int n = 1; n <= L; ++n) {
+    mpow[n] = mpow[n - 1] * mu;
+    npow[n] = npow[n - 1] * nu;
   }
+  double sgn = 1.0;
 #pragma unroll
-  for (int tot = 1; tot <= L; ++tot)
+  for (int n = 0; n <= L; ++n) {
+    double v = 0.0, binom = 1.0;
 #pragma unroll
-    for (int t = tot; t >= 0; --t)
-#pragma unroll
-      for (int u = tot - t; u >= 0; --u) {
-        const int v = tot - t - u;
-        const int id = herm_index(t, u, v);
-#pragma unroll
-        for (int n = 0; n <= L - tot; ++n) {
-          double val;
-          if (t > 0) {
-            val = X[0] * R[n + 1][herm_index(t - 1, u, v)];
-            if (t > 1) val += (t - 1) * R[n + 1][herm_index(t - 2, u, v)];
-          } else if (u > 0) {
-            val = X[1] * R[n + 1][herm_index(t, u - 1, v)];
-            if (u > 1) val += (u - 1) * R[n + 1][herm_index(t, u - 2, v)];
-          } else {
-            val = X[2] * R[n + 1][herm_index(t, u, v - 1)];
-            if (v > 1) val += (v - 1) * R[n + 1][herm_index(t, u, v - 2)];
-          }
-          R[n][id] = val;
-        }
-      }
-#pragma unroll
-  for (int i = 0; i < nherm(L); ++i) Q[i] += R[0][i];
+    for (int k = 0; k <= n; ++k) {
+      v += binom * mpow[n - k] * npow[k] * F[k];
+      binom = binom * (n - k) / (k + 1);
+    }
+    G[n] = sgn * g * v;
+    sgn *= -2.0;
+  }
+  accumulate_radial_q<L>(X, G, Q);
 }
 
 // Turn accumulated Hermite integrals Q into the sh block:
 // pc(a, b) = pref * sum_tuv Ex[ax][bx][t] Ey[ay][by][u] Ez[az][bz][v] Q_tuv.
-template <int LA, int LB>
+template <int LA, int LB, bool PAD = false>
 __device__ void hermite_to_sh(const double *A, const double *B, double a1,
                               double a2, double pref,
                               const double Q[nherm(LA + LB)], double *out) {
@@ -528,7 +566,7 @@ __device__ void hermite_to_sh(const double *A, const double *B, double a1,
       }
       pc[p * ncart(LB) + q] = pref * s;
     }
-  cart_to_sh<LA, LB>(pc, out);
+  cart_to_sh<LA, LB, PAD>(pc, out);
 }
 
 // ------------------------------------------------ f classes, runtime loops --
