@@ -1030,7 +1030,9 @@ inline size_t pipe_smem(int C, int V) {
 
 bool ortho_pipe_fits(int C, int V) {
   const PipeDims d = pipe_dims(C, V);
-  return C > 0 && V > 0 && V <= 256 && d.C4 <= 256 && 2 * d.ld <= 256 &&
+  // each box of V rows x 64 bytes starts where the one before it ends, and a
+  // TMA destination in shared memory is a multiple of 128 bytes: V even
+  return C > 0 && V > 0 && V % 2 == 0 && V <= 256 && d.C4 <= 256 && 2 * d.ld <= 256 &&
          pipe_smem(C, V) <= kPipeMaxSmem;
 }
 

@@ -9,6 +9,8 @@ launch takes, images in plenty and hardly any, f classes.
 import numpy as np
 import pytest
 
+import oracle
+from conftest import packed_mismatch
 from imago_b200 import configs, intg
 
 pytestmark = pytest.mark.gpu
@@ -93,3 +95,19 @@ def test_without_image_lists(imago_lib, monkeypatch, name):
         b = _build(s, schedule)
         for k in ("ep", "np", "ham"):
             _close(a[k], b[k], np.abs(a[k]).max())
+
+
+@pytest.mark.parametrize("schedule", ["per_item", "piped", "auto"])
+def test_odd_valence_dimension_runs_under_every_orthogonalisation_schedule(imago_lib, schedule):
+    # V = 87: the TMA-fed kernel's boxes would start off their 128 bytes, so
+    # it does not take the system; the other one serves every schedule
+    s = SYSTEMS["quartz9"]()
+    assert s.vale_dim % 2 == 1
+    ob = oracle.OracleBuild(s)
+    ob.overlap()
+    ref = ob.elec_pot()
+    with intg.IntegralSetup(s) as g:
+        g.set_ortho_schedule(schedule)
+        g.gauss_overlap_ol()
+        ep = g.elec_pot_gauss_overlap()
+    assert packed_mismatch(ep, ref)[1] == 0
