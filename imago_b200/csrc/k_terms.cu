@@ -189,7 +189,13 @@ __global__ void __launch_bounds__(kTermThreads, LA + LB >= 4 ? 3 : (LA + LB >= 3
   const double *als = s.palpha + s.ptype_alpha_off[s.ptype_screen[pt]];
   const bool ascends = s.ptype_ascends[pt];
   const UnitWalk uw = unit_walk(s, w, sp.unit, pt);
-  const double ex = exp(-c.xi * q.r2);
+  const double ex = exp(-c.xi * q.r2), inv2p = 1.0 / (2.0 * c.zeta);
+  double PA[3], PB[3];
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    PA[x] = c.Pt[x] - q.A[x];
+    PB[x] = c.Pt[x] - q.B[x];
+  }
   bool have = false;  // the notes hold every image of this and later terms
   int nn = 0;
   double t = cnt > 0 ? c.reach2(s.T, als[terms[t0].j]) : -1.0;
@@ -233,7 +239,7 @@ __global__ void __launch_bounds__(kTermThreads, LA + LB >= 4 ? 3 : (LA + LB >= 3
     if (on) {
       const double pz = kPi / z3;
       hermite_to_sh<LA, LB, true>(
-          q.A, q.B, q.a1, q.a2, pz * sqrt(pz) * ex, Q,
+          PA, PB, inv2p, pz * sqrt(pz) * ex, Q,
           blk + (long long)(t0 + it * tg.stride) * w.blk_total + sp.boff);
     }
     t = tn;

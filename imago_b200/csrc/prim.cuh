@@ -119,13 +119,9 @@ __device__ __forceinline__ void store4(double *p, const double v[4]) {
 }
 
 // Write the real-solid-harmonic block from a Cartesian block
-// pc[p * ncart(LB) + q].  PAD: to a build's block buffer, where every block
-// starts on 32 bytes and has blk_len doubles: each thread writes its own
-// block, so single 8-byte stores would send one partial sector each (162-atom
-// quartz EP: 2.0 G of them; the whole-sector stores are a quarter).
-template <int LA, int LB, bool PAD = false>
+// pc[p * ncart(LB) + q].
+template <int LA, int LB>
 __device__ __forceinline__ void cart_to_sh(const double *pc, double *out) {
-  double quad[4];
 #pragma unroll
   for (int s1 = 0; s1 < nsh(LA); ++s1)
 #pragma unroll
@@ -141,19 +137,7 @@ __device__ __forceinline__ void cart_to_sh(const double *pc, double *out) {
                pc[sh_cart(s1, k1) * ncart(LB) + sh_cart(s2, k2)];
         }
       }
-      const int o = s1 * nsh(LB) + s2;
-      if (!PAD) {
-        out[o] = v;
-        continue;
-      }
-      quad[o & 3] = v;
-      if (o == nsh(LA) * nsh(LB) - 1) {
-#pragma unroll
-        for (int i = (o & 3) + 1; i < 4; ++i) quad[i] = 0.0;
-        store4(out + (o & ~3), quad);
-      } else if ((o & 3) == 3) {
-        store4(out + (o & ~3), quad);
-      }
+      out[s1 * nsh(LB) + s2] = v;
     }
 }
 
@@ -392,35 +376,9 @@ __device__ void prim_vec(double a1, double a2, const double *A, const double *B,
 }
 
 // ---------------------------------------------- McMurchie-Davidson 3C --
-// Hermite expansion coefficients of one axis:
+// Hermite expansion coefficients of one axis (hermite_e_row):
 // E^{00}_0 = 1, E^{i+1,j}_t = E^{ij}_{t-1}/(2p) + PA E^{ij}_t + (t+1) E^{ij}_{t+1}
 // and likewise for j with PB.
-template <int LA, int LB>
-__device__ __forceinline__ void hermite_e(double PA, double PB, double inv2p,
-                                          double E[LA + 1][LB + 1][LA + LB + 1]) {
-#pragma unroll
-  for (int i = 0; i <= LA; ++i)
-#pragma unroll
-    for (int j = 0; j <= LB; ++j)
-#pragma unroll
-      for (int t = 0; t <= LA + LB; ++t) {
-        double v;
-        if (t > i + j) {
-          v = 0.0;
-        } else if (i == 0 && j == 0) {
-          v = 1.0;
-        } else if (i > 0) {
-          v = PA * E[i - 1][j][t];
-          if (t > 0) v += inv2p * E[i - 1][j][t - 1];
-          if (t + 1 <= i - 1 + j) v += (t + 1) * E[i - 1][j][t + 1];
-        } else {
-          v = PB * E[i][j - 1][t];
-          if (t > 0) v += inv2p * E[i][j - 1][t - 1];
-          if (t + 1 <= i + j - 1) v += (t + 1) * E[i][j - 1][t + 1];
-        }
-        E[i][j][t] = v;
-      }
-}
 
 // Accumulate one three-centre overlap term into Q: w * exp(-mu |X|^2)
 // h_t(X) h_u(Y) h_v(Z), h_t = (d/dX)^t exp(-mu X^2) / exp(-mu X^2),
@@ -528,45 +486,215 @@ __device__ __forceinline__ void accumulate_nuclear_q(const double X[3],
   accumulate_radial_q<L>(X, G, Q);
 }
 
-// Turn accumulated Hermite integrals Q into the sh block:
-// pc(a, b) = pref * sum_tuv Ex[ax][bx][t] Ey[ay][by][u] Ez[az][bz][v] Q_tuv.
+// Cartesian component of an exponent triple, x + y + z <= 2 (cart_exp's
+// inverse).
+__host__ __device__ constexpr int cart_index(int x, int y, int z) {
+  constexpr int t[27] = {0, 3, 6, 2, 9, -1, 5, -1, -1, 1, 8, -1, 7, -1,
+                         -1, -1, -1, -1, 4, -1, -1, -1, -1, -1, -1, -1, -1};
+  return t[9 * x + 3 * y + z];
+}
+
+// f(0), f(1), ... f(N - 1) with the index as a type, so that everything
+// derived from it is a constant and small arrays stay in registers.
+template <int I>
+struct Idx {
+  static constexpr int value = I;
+};
+template <int N, int I = 0, class F>
+__device__ __forceinline__ void static_for(F &&f) {
+  if constexpr (I < N) {
+    f(Idx<I>{});
+    static_for<N, I + 1>(f);
+  }
+}
+
+// One axis's Hermite coefficients E^{ij}_t for one i and every j <= LB:
+// E[j][t], t <= i + j.
+template <int I, int LB>
+__device__ __forceinline__ void hermite_e_row(double PA, double PB, double inv2p,
+                                              double (&E)[LB + 1][I + LB + 1]) {
+  double e[I + LB + 1];
+  e[0] = 1.0;
+  static_for<I + LB>([&](auto iq) {
+    // raise from order q to q + 1: with PA up to I, then with PB
+    constexpr int q = decltype(iq)::value;
+    if constexpr (q >= I) static_for<q + 1>([&](auto it) {
+        E[q - I][decltype(it)::value] = e[decltype(it)::value];
+      });
+    const double X = q < I ? PA : PB;
+    double f[I + LB + 1];
+    static_for<q + 2>([&](auto it) {
+      constexpr int t = decltype(it)::value;
+      double v = 0.0;
+      if constexpr (t <= q) v = X * e[t];
+      if constexpr (t > 0) v += inv2p * e[t - 1];
+      if constexpr (t + 1 <= q) v += (t + 1) * e[t + 1];
+      f[t] = v;
+    });
+    static_for<q + 2>([&](auto it) { e[decltype(it)::value] = f[decltype(it)::value]; });
+  });
+  static_for<I + LB + 1>([&](auto it) { E[LB][decltype(it)::value] = e[decltype(it)::value]; });
+}
+
+// Row P (a Cartesian component of atom 1) of the block, as atom 2's real
+// solid harmonics: pc(P, b) = sum_tuv Ex[ax][bx][t] Ey[ay][by][u]
+// Ez[az][bz][v] Q_tuv, one axis after another.
+// The coefficients are formed anew for every row: the empty asm keeps the
+// compiler from holding all rows' (81 for d-d) in registers it has to spill.
+template <int LA, int LB, int P>
+__device__ __forceinline__ void hermite_row(const double (&PA0)[3], const double (&PB0)[3],
+                                            double inv2p, const double (&Q)[nherm(LA + LB)],
+                                            double (&row)[nsh(LB)]) {
+  constexpr int AX = cart_exp(P, 0), AY = cart_exp(P, 1), AZ = cart_exp(P, 2);
+  double PA[3] = {PA0[0], PA0[1], PA0[2]}, PB[3] = {PB0[0], PB0[1], PB0[2]};
+  if constexpr (LA + LB >= 3)
+    asm volatile("" : "+d"(PA[0]), "+d"(PA[1]), "+d"(PA[2]), "+d"(PB[0]), "+d"(PB[1]),
+                 "+d"(PB[2]));
+  double ex[LB + 1][AX + LB + 1], ey[LB + 1][AY + LB + 1], ez[LB + 1][AZ + LB + 1];
+  hermite_e_row<AX, LB>(PA[0], PB[0], inv2p, ex);
+  hermite_e_row<AY, LB>(PA[1], PB[1], inv2p, ey);
+  hermite_e_row<AZ, LB>(PA[2], PB[2], inv2p, ez);
+  double pc[ncart(LB)];
+  static_for<LB + 1>([&](auto ibx) {
+    constexpr int bx = decltype(ibx)::value;
+    double T[AY + LB - bx + 1][AZ + LB - bx + 1];
+    static_for<AY + LB - bx + 1>([&](auto iu) {
+      static_for<AZ + LB - bx + 1>([&](auto iv) {
+        constexpr int u = decltype(iu)::value, v = decltype(iv)::value;
+        if constexpr (u + v <= AY + AZ + LB - bx) {
+          double q = 0.0;
+          static_for<AX + bx + 1>([&](auto it) {
+            constexpr int t = decltype(it)::value, h = herm_index(t, u, v);
+            q += ex[bx][t] * Q[h];
+          });
+          T[u][v] = q;
+        }
+      });
+    });
+    static_for<LB - bx + 1>([&](auto iby) {
+      constexpr int by = decltype(iby)::value;
+      double U[AZ + LB - bx - by + 1];
+      static_for<AZ + LB - bx - by + 1>([&](auto iv) {
+        constexpr int v = decltype(iv)::value;
+        double q = 0.0;
+        static_for<AY + by + 1>([&](auto iu) {
+          constexpr int u = decltype(iu)::value;
+          q += ey[by][u] * T[u][v];
+        });
+        U[v] = q;
+      });
+      static_for<LB - bx - by + 1>([&](auto ibz) {
+        constexpr int bz = decltype(ibz)::value, c = cart_index(bx, by, bz);
+        double q = 0.0;
+        static_for<AZ + bz + 1>([&](auto iv) {
+          constexpr int v = decltype(iv)::value;
+          q += ez[bz][v] * U[v];
+        });
+        pc[c] = q;
+      });
+    });
+  });
+  static_for<nsh(LB)>([&](auto im) {
+    constexpr int m = decltype(im)::value;
+    double v = 0.0;
+    static_for<sh_nterm(m)>([&](auto ik) {
+      constexpr int k = decltype(ik)::value, c = sh_cart(m, k);
+      constexpr double f = sh_coef(m, k);
+      v += f * pc[c];
+    });
+    row[m] = v;
+  });
+}
+
+// A block's rows as they are finished: to `out`, or (PAD) to a build's
+// block buffer, where every block starts on 32 bytes and has blk_len
+// doubles: each thread writes its own block, so single 8-byte stores would
+// send one partial sector each (162-atom quartz EP: 2.0 G of them; whole
+// sectors are a quarter).
+template <int N, bool PAD>
+struct BlockWriter {
+  double *out;
+  double quad[4];
+  template <int R, int M>
+  __device__ __forceinline__ void row(const double (&v)[M]) {
+    static_for<M>([&](auto im) {
+      constexpr int m = decltype(im)::value, o = R * M + m;
+      if constexpr (!PAD) {
+        out[o] = v[m];
+      } else {
+        quad[o & 3] = v[m];
+        if constexpr (o == N - 1)
+          for (int i = (o & 3) + 1; i < 4; ++i) quad[i] = 0.0;
+        if constexpr (o == N - 1 || (o & 3) == 3) store4(out + (o & ~3), quad);
+      }
+    });
+  }
+};
+
+// Turn accumulated Hermite integrals Q into the sh block, one Cartesian row
+// of atom 1 at a time: a d-d block as a whole (100 Cartesian values beside
+// 81 E coefficients) does not fit the registers, and its spills (1.6 KB a
+// thread, now 0.3) were half of that class's memory traffic (1.2 GB written
+// for 0.6 GB of Si8 blocks).  162-atom quartz EP primitives 10.5 -> 8.9 ms,
+// Si8 0.78 -> 0.65 ms.
 template <int LA, int LB, bool PAD = false>
-__device__ void hermite_to_sh(const double *A, const double *B, double a1,
-                              double a2, double pref,
-                              const double Q[nherm(LA + LB)], double *out) {
-  constexpr int L = LA + LB;
-  const double zeta = a1 + a2, inv2p = 1.0 / (2.0 * zeta);
-  double E[3][LA + 1][LB + 1][L + 1];
+__device__ __forceinline__ void hermite_to_sh(const double (&PA)[3], const double (&PB)[3],
+                                              double inv2p, double pref,
+                                              const double Q[nherm(LA + LB)], double *out) {
+  double H[nherm(LA + LB)];
+#pragma unroll
+  for (int i = 0; i < nherm(LA + LB); ++i) H[i] = pref * Q[i];
+  BlockWriter<nsh(LA) * nsh(LB), PAD> w{out, {}};
+  double row[nsh(LB)];
+  hermite_row<LA, LB, 0>(PA, PB, inv2p, H, row);
+  w.template row<0>(row);
+  if constexpr (LA >= 1) {
+    hermite_row<LA, LB, 1>(PA, PB, inv2p, H, row);
+    w.template row<1>(row);
+    hermite_row<LA, LB, 2>(PA, PB, inv2p, H, row);
+    w.template row<2>(row);
+    hermite_row<LA, LB, 3>(PA, PB, inv2p, H, row);
+    w.template row<3>(row);
+  }
+  if constexpr (LA >= 2) {
+    // xy, xz, yz, xx - yy, 2 zz - xx - yy
+    hermite_row<LA, LB, 7>(PA, PB, inv2p, H, row);
+    w.template row<4>(row);
+    hermite_row<LA, LB, 8>(PA, PB, inv2p, H, row);
+    w.template row<5>(row);
+    hermite_row<LA, LB, 9>(PA, PB, inv2p, H, row);
+    w.template row<6>(row);
+    double yy[nsh(LB)], sum[nsh(LB)];
+    hermite_row<LA, LB, 4>(PA, PB, inv2p, H, row);
+    hermite_row<LA, LB, 5>(PA, PB, inv2p, H, yy);
+#pragma unroll
+    for (int m = 0; m < nsh(LB); ++m) {
+      sum[m] = row[m] + yy[m];
+      row[m] -= yy[m];
+    }
+    w.template row<7>(row);
+    hermite_row<LA, LB, 6>(PA, PB, inv2p, H, row);
+#pragma unroll
+    for (int m = 0; m < nsh(LB); ++m) row[m] = 2.0 * row[m] - sum[m];
+    w.template row<8>(row);
+  }
+  static_assert(LA <= 2 && LB <= 2, "f classes: hermite_to_sh_rt");
+}
+
+// The same from the centres and exponents.
+template <int LA, int LB, bool PAD = false>
+__device__ __forceinline__ void hermite_to_sh(const double *A, const double *B, double a1,
+                                              double a2, double pref,
+                                              const double Q[nherm(LA + LB)], double *out) {
+  const double zeta = a1 + a2;
+  double PA[3], PB[3];
 #pragma unroll
   for (int x = 0; x < 3; ++x) {
     const double P = (a1 * A[x] + a2 * B[x]) / zeta;
-    hermite_e<LA, LB>(P - A[x], P - B[x], inv2p, E[x]);
+    PA[x] = P - A[x];
+    PB[x] = P - B[x];
   }
-  double pc[ncart(LA) * ncart(LB)];
-#pragma unroll
-  for (int p = 0; p < ncart(LA); ++p)
-#pragma unroll
-    for (int q = 0; q < ncart(LB); ++q) {
-      const int ax = cart_exp(p, 0), ay = cart_exp(p, 1), az = cart_exp(p, 2);
-      const int bx = cart_exp(q, 0), by = cart_exp(q, 1), bz = cart_exp(q, 2);
-      double s = 0.0;
-#pragma unroll
-      for (int t = 0; t <= L; ++t) {
-        if (t > ax + bx) break;
-#pragma unroll
-        for (int u = 0; u <= L; ++u) {
-          if (u > ay + by) break;
-          const double etu = E[0][ax][bx][t] * E[1][ay][by][u];
-#pragma unroll
-          for (int v = 0; v <= L; ++v) {
-            if (v > az + bz) break;
-            s += etu * E[2][az][bz][v] * Q[herm_index(t, u, v)];
-          }
-        }
-      }
-      pc[p * ncart(LB) + q] = pref * s;
-    }
-  cart_to_sh<LA, LB, PAD>(pc, out);
+  hermite_to_sh<LA, LB, PAD>(PA, PB, 1.0 / (2.0 * zeta), pref, Q, out);
 }
 
 // ------------------------------------------------ f classes, runtime loops --

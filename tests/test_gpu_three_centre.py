@@ -84,17 +84,18 @@ def test_term_groups_equal_one_term_per_thread(imago_lib, name):
     assert np.abs(a["ham"][0] - ham).max() <= 2e-14 * scale + 1e-10 * (len(w) + 3)
 
 
-@pytest.mark.parametrize("name", ["small", "f", "si8", "type_per_site"])
-def test_without_image_lists(imago_lib, monkeypatch, name):
-    # beyond the lists' memory limit every image of a type is tested; the
-    # images come in another order
+@pytest.mark.parametrize("schedule", ["pairs", "per_class", "queue"])
+@pytest.mark.parametrize("name", ["small", "f", "si8"])
+def test_without_image_lists(imago_lib, monkeypatch, name, schedule):
+    # beyond the lists' memory limit every image of a type is tested, in
+    # another order: against the oracle, within the builds' 1e-10 bar
     s = SYSTEMS[name]()
-    a = _build(s, "pairs")
     monkeypatch.setenv("IMAGO_TUNING", "lists=off")
-    for schedule in ("pairs", "per_class", "queue"):
-        b = _build(s, schedule)
-        for k in ("ep", "np", "ham"):
-            _close(a[k], b[k], np.abs(a[k]).max())
+    got = _build(s, schedule)
+    ob = oracle.OracleBuild(s)
+    ob.overlap()
+    assert packed_mismatch(got["np"], ob.nuclear())[1] == 0
+    assert packed_mismatch(got["ep"], ob.elec_pot())[1] == 0
 
 
 @pytest.mark.parametrize("schedule", ["per_item", "piped", "auto"])
