@@ -233,8 +233,8 @@ struct imago_ctx {
   DBuf<int2> d_btile, d_btile_w;
   // the three-centre screens' image table and lists (DevWork)
   DBuf<double4> d_ipos;
-  DBuf<float4> d_ftab;
-  DBuf<int> d_img_off, d_ptype_ascends;
+  DBuf<float4> d_ftab, d_chunk;
+  DBuf<int> d_img_off, d_chunk_off, d_ptype_ascends;
   DBuf<int2> d_uoff;
   DBuf<ImageRef> d_ulist;
   DBuf<float> d_rad;
@@ -315,6 +315,7 @@ struct imago_ctx {
     d_pairs.release(st); d_units.release(st); d_sps.release(st);
     d_terms.release(st); d_btile.release(st); d_btile_w.release(st);
     d_ipos.release(st); d_ftab.release(st); d_img_off.release(st);
+    d_chunk.release(st); d_chunk_off.release(st);
     d_ptype_ascends.release(st); d_uoff.release(st); d_ulist.release(st);
     d_rad.release(st);
     d_queue.release(st);
@@ -867,7 +868,8 @@ constexpr size_t kMaxImageListBytes = size_t(4) << 30;
 struct ImageTable {
   std::vector<double4> pos;
   std::vector<float4> fpos;
-  std::vector<int> off;
+  std::vector<float4> chunk;  // bounding spheres of 32 images each
+  std::vector<int> off, chunk_off;
   double a3_min = 0.0;
   float margin = 0.f;
 };
@@ -912,25 +914,69 @@ void make_images(const imago_ctx *c, ImageTable &tab) {
         }
         if (d <= (rad + rho_p) * (rad + rho_p)) lat.push_back(L);
       }
+  // a grid whose cells hold about 32 images of a type each; the images of
+  // a type are kept in the order of its cells
+  double vol = std::fabs(c->rv[0] * (c->rv[4] * c->rv[8] - c->rv[5] * c->rv[7]) -
+                         c->rv[1] * (c->rv[3] * c->rv[8] - c->rv[5] * c->rv[6]) +
+                         c->rv[2] * (c->rv[3] * c->rv[7] - c->rv[4] * c->rv[6]));
   double far = 0.0;
   tab.off.assign(1, 0);
+  tab.chunk_off.assign(1, 0);
+  std::vector<double4> img;
+  std::vector<int> cell, start;
   for (int t = 0; t < c->npt; ++t) {
     const HPType &p = c->ptypes[t];
+    const double edge = std::max(std::cbrt(32.0 * vol / std::max(1, p.mult)), rad / 16.0);
+    const int n = (int)(2.0 * rad / edge) + 1;
+    img.clear();
+    cell.clear();
+    start.assign((size_t)n * n * n + 1, 0);
     for (int q = 0; q < p.mult; ++q) {
       const double *C = &c->psite_pos[3 * (p.first_site + q)];
       for (const auto &L : lat) {
         const double v[3] = {C[0] + L[0], C[1] + L[1], C[2] + L[2]};
         if (from_mid(v) > rad) continue;
-        tab.pos.push_back(make_double4(v[0], v[1], v[2], 0.0));
-        tab.fpos.push_back(make_float4((float)v[0], (float)v[1], (float)v[2], 0.f));
-        for (int x = 0; x < 3; ++x) far = std::max(far, std::fabs(v[x]));
+        int id = 0;
+        for (int x = 0; x < 3; ++x) {
+          id = id * n + std::min(n - 1, std::max(0, (int)((v[x] - mid[x] + rad) / edge)));
+          far = std::max(far, std::fabs(v[x]));
+        }
+        img.push_back(make_double4(v[0], v[1], v[2], 0.0));
+        cell.push_back(id);
+        ++start[id + 1];
       }
     }
-    tab.off.push_back((int)tab.pos.size());
+    for (size_t i = 1; i < start.size(); ++i) start[i] += start[i - 1];
+    const size_t beg = tab.pos.size(), end = beg + img.size();
+    tab.pos.resize(end);
+    tab.fpos.resize(end);
+    for (size_t i = 0; i < img.size(); ++i) {
+      const size_t o = beg + start[cell[i]]++;
+      tab.pos[o] = img[i];
+      tab.fpos[o] = make_float4((float)img[i].x, (float)img[i].y, (float)img[i].z, 0.f);
+    }
+    for (size_t b = beg; b < end; b += 32) {
+      const size_t e = std::min(end, b + 32);
+      double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+      for (size_t i = b; i < e; ++i) {
+        const double v[3] = {tab.pos[i].x, tab.pos[i].y, tab.pos[i].z};
+        for (int x = 0; x < 3; ++x) {
+          lo[x] = std::min(lo[x], v[x]);
+          hi[x] = std::max(hi[x], v[x]);
+        }
+      }
+      double r2 = 0.0;
+      for (int x = 0; x < 3; ++x) r2 += 0.25 * (hi[x] - lo[x]) * (hi[x] - lo[x]);
+      tab.chunk.push_back(make_float4((float)(0.5 * (lo[0] + hi[0])), (float)(0.5 * (lo[1] + hi[1])),
+                                      (float)(0.5 * (lo[2] + hi[2])), (float)std::sqrt(r2)));
+    }
+    tab.off.push_back((int)end);
+    tab.chunk_off.push_back((int)tab.chunk.size());
   }
   // float positions and differences: each within 2^-23 of the largest
   // coordinate, a handful of roundings
   tab.margin = (float)(1e-4 + 4e-6 * (far + rad));
+  for (float4 &q : tab.chunk) q.w += 2.f * tab.margin;
 }
 
 void set_bloch_width(imago_ctx *c, int wi) {
@@ -1013,6 +1059,7 @@ int upload(imago_ctx *c) {
   UP(d_sps, c->sps) UP(d_sp_by_cls, c->sp_by_cls) UP(d_terms, c->ep_terms)
   UP(d_btile, c->btile) UP(d_btile_w, c->btile_w) UP(d_kout, c->kout)
   UP(d_ptype_ascends, pasc) UP(d_ipos, tab.pos) UP(d_ftab, tab.fpos) UP(d_img_off, tab.off)
+  UP(d_chunk, tab.chunk) UP(d_chunk_off, tab.chunk_off)
 #undef UP
   if ((rc = c->d_queue.alloc(4, st))) return rc;
   if ((rc = c->d_flag.alloc(1, st))) return rc;
@@ -1067,6 +1114,8 @@ int upload(imago_ctx *c) {
   w.ipos = c->d_ipos.p;
   w.ftab = c->d_ftab.p;
   w.img_off = c->d_img_off.p;
+  w.chunk = c->d_chunk.p;
+  w.chunk_off = c->d_chunk_off.p;
   w.uoff = nullptr;
   w.ulist = nullptr;
   if ((rc = launch_phase(s, c->d_phase.p, st))) return rc;

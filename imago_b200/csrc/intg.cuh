@@ -103,11 +103,15 @@ struct DevWork {
   int nbtile_w;           // its tiles: (pair, tile of bw columns)
   const int2 *btile_w;
   // Every lattice image of a potential site that some shell pair may reach,
-  // ordered by type, then site: ipos[i] its position, ftab[i] the same in
+  // ordered by type: ipos[i] its position, ftab[i] the same in
   // float, img_off[t] the first image of type t (npt + 1 entries)
   const double4 *ipos;
   const float4 *ftab;
   const int *img_off;
+  // within a type the images come by place; chunk_off[t] is the type's first
+  // group of 32 consecutive ones, chunk[] their bounding spheres
+  const float4 *chunk;
+  const int *chunk_off;
   // For each (unit, type), at unit * npt + type, its range of `ulist`: the
   // images within reach of the unit's shell pairs in ascending order of
   // distance from the midpoint of its A-B segment, in 64 steps of the
