@@ -203,13 +203,11 @@ constexpr int kTermThreads = 128;
 constexpr int kTermCap = 64;
 
 template <int LA, int LB>
-__global__ void __launch_bounds__(kTermThreads, LA + LB >= 4 ? 3 : (LA + LB >= 3 ? 4 : 5))
-    k_prim3c_terms(DevSys s, DevWork w, int beg, int n, const Term3c *terms, TermGroups tg,
-                   double *blk) {
+__device__ __forceinline__ void terms_item(const DevSys &s, const DevWork &w, int beg, int n,
+                                           const Term3c *terms, const TermGroups &tg, double *blk,
+                                           long long g, int (*note)[kTermThreads]) {
   constexpr int L = LA + LB;
-  __shared__ int note[kTermCap][kTermThreads];
   const int tid = threadIdx.x;
-  const long long g = (long long)blockIdx.x * kTermThreads + tid;
   const bool live = g < (long long)n * tg.n;
   const int gi = live ? (int)(g / n) : 0;
   const int t0 = tg.first[gi], cnt = live ? tg.count[gi] : 0;
@@ -278,6 +276,41 @@ __global__ void __launch_bounds__(kTermThreads, LA + LB >= 4 ? 3 : (LA + LB >= 3
   }
 }
 
+template <int LA, int LB>
+__global__ void __launch_bounds__(kTermThreads, LA + LB >= 4 ? 3 : (LA + LB >= 3 ? 4 : 5))
+    k_prim3c_terms(DevSys s, DevWork w, int beg, int n, const Term3c *terms, TermGroups tg,
+                   double *blk) {
+  __shared__ int note[kTermCap][kTermThreads];
+  terms_item<LA, LB>(s, w, beg, n, terms, tg, blk,
+                     (long long)blockIdx.x * kTermThreads + threadIdx.x, note);
+}
+
+// Every class in one launch, costliest first: cta[c] is the first CTA of the
+// c-th class.  A small system's classes are a few CTAs each (Si8: 16 for
+// p-p) and last as long as their longest thread; in turn they leave the GPU
+// nearly empty, together they fill in behind the largest.
+struct ClassCtas {
+  int ncls;
+  int cls[9], beg[9], n[9], cta[10];
+};
+
+__global__ void __launch_bounds__(kTermThreads, 3)
+    k_prim3c_terms_all(DevSys s, DevWork w, ClassCtas cc, const Term3c *terms, TermGroups tg,
+                       double *blk) {
+  __shared__ int note[kTermCap][kTermThreads];
+  int c = 0;
+  while ((int)blockIdx.x >= cc.cta[c + 1]) ++c;
+  const long long g = (long long)((int)blockIdx.x - cc.cta[c]) * kTermThreads + threadIdx.x;
+  switch (cc.cls[c]) {
+#define IMAGO_TA(a, b)                                                              \
+  case a * 4 + b:                                                                   \
+    terms_item<a, b>(s, w, cc.beg[c], cc.n[c], terms, tg, blk, g, note);            \
+    break;
+    IMAGO_FOR_SPD_CLASSES(IMAGO_TA)
+#undef IMAGO_TA
+  }
+}
+
 // Term groups of one launch: the terms from `from` on, split into runs of
 // one potential type and each run into `split` interleaved groups, at most
 // kMaxTermGroups of them.  Returns the first term not covered.
@@ -300,10 +333,19 @@ static int group_terms(const Term3c *terms, int nterm, int from, int split, Term
   return i;
 }
 
-// Threads that the widest class launch should at least have: a GPU of 148
-// SMs holds 75,000 to 95,000 of this kernel's, and the images of a thread's
-// terms differ enough that a few rounds even them out.
-constexpr long long kTermThreadsWanted = 400000;
+// Several classes and at most kTermsMergedPairs (shell pair, run of terms of
+// one type): all classes in one launch.  Else a launch per class, with the
+// class's own occupancy: one class gains nothing, and a large system's
+// classes fill the GPU each.  Terms are split into interleaved groups until
+// a launch has about the threads wanted.  One B200, EP primitives in ms, per
+// class / merged, each at its best split: Si8 (62k pairs) 0.89 / 0.55, Si16
+// (118k) 1.26 / 0.95, Si32 (230k) 2.03 / 1.67, 18-atom quartz (158k x 2)
+// 1.58 / 1.26, 36-atom quartz (307k x 2) 2.64 / 2.32, 162-atom quartz (1.36M
+// x 2) 8.79 / 8.92; one class: 16-atom diamond (226k) 2.02 / 2.29, 64-atom
+// graphite (534k) 2.69 / 3.34.  Split, Si8 merged: 1.28, 0.77, 0.55, 0.57,
+// 0.59, 0.69 with 1, 2, 4, 7, 10, 20 groups.
+constexpr long long kTermsMergedPairs = 1000000;
+constexpr long long kTermThreadsMerged = 400000, kTermThreadsWanted = 800000;
 
 int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
                         const Term3c *terms_dev, const Term3c *terms_host, int nterm,
@@ -311,11 +353,36 @@ int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
   int runs = 0;
   for (int i = 0; i < nterm; ++i) runs += i == 0 || terms_host[i].ptype != terms_host[i - 1].ptype;
   const long long base = std::max(1LL, (long long)w.nsp * std::max(1, runs));
-  const int split = (int)std::min<long long>(8, (kTermThreadsWanted + base - 1) / base);
+  int classes = 0;
+  for (int c : {0, 1, 2, 4, 5, 6, 8, 9, 10}) classes += cls_beg[c + 1] > cls_beg[c];
+  const bool merged = classes > 1 && base <= kTermsMergedPairs;
+  const long long wanted = merged ? kTermThreadsMerged : kTermThreadsWanted;
+  const int split = (int)std::min<long long>(32, (wanted + base - 1) / base);
   for (int from = 0; from < nterm;) {
     TermGroups tg;
     const int next = group_terms(terms_host + from, nterm - from, 0, split, tg) + from;
     double *b = blk + (long long)from * w.blk_total;
+    if (merged) {
+      static const int order[9] = {10, 6, 9, 5, 2, 8, 1, 4, 0};  // la * 4 + lb
+      ClassCtas cc{};
+      for (int c : order) {
+        const int n = cls_beg[c + 1] - cls_beg[c];
+        if (n <= 0) continue;
+        cc.cls[cc.ncls] = c;
+        cc.beg[cc.ncls] = cls_beg[c];
+        cc.n[cc.ncls] = n;
+        cc.cta[cc.ncls + 1] =
+            cc.cta[cc.ncls] + (int)(((long long)n * tg.n + kTermThreads - 1) / kTermThreads);
+        ++cc.ncls;
+      }
+      if (cc.ncls) {
+        k_prim3c_terms_all<<<cc.cta[cc.ncls], kTermThreads, 0, st>>>(s, w, cc, terms_dev + from,
+                                                                    tg, b);
+        IMAGO_CUDA(cudaGetLastError());
+      }
+      from = next;
+      continue;
+    }
 #define IMAGO_PT(a, c)                                                                     \
   {                                                                                       \
     const int beg = cls_beg[a * 4 + c], n = cls_beg[a * 4 + c + 1] - beg;                 \
