@@ -539,54 +539,86 @@ int launch_bloch(const DevSys &s, const DevWork &w, int nterm, const double *M,
 // and makeValeVale):
 //   VV' = VV - S^H X_cv - X_cv^H S + S^H X_cc S.
 // Here it is formed as VV' = VV - (S^H Y + Y^H S) with Y = X_cv - X_cc S/2
-// (X_cc is Hermitian), two complex GEMMs on 32x32 output tiles:
+// (X_cc is Hermitian), two complex GEMMs:
 //   k_ortho_y: Y (C x V),  k_ortho_w: the upper tiles of S^H Y + Y^H S,
 // then the packing of the upper triangle with the 1e-10 zeroing.
 // For the overlap itself X = S: VV - 2 S^H S + S^H S_cc S.
-constexpr int kOT = 32;   // output tile
-constexpr int kOK = 16;   // complex K per shared-memory stage
-constexpr int kOP = kOT + 2;  // 34 double2 = 136 bank words: conflict-free fragment reads
-constexpr int kOThreads = 128;
-constexpr int kOLoads = kOK * kOT / kOThreads;  // double2 per thread per operand
+//
+// Output tiles of 64 x 64 (eight warps of 16 x 32 each) or 32 x 32 (four of
+// 16 x 16), 16 complex core indices per stage, two stages filled by cp.async.
+// With 32 x 32 tiles a 162-atom quartz term reads 1.9 GB of operands from L2
+// (76 GB per Gamma EP build), which bounds the real arithmetic at Gamma and
+// is half of that with 64 x 64: 7.37 -> 4.61 ms (2x2x2 k: 42.4 -> 40.8).
+// Smaller matrices have too few of the large tiles, and too much of them
+// outside the matrix: Si16 (V = 208) 0.59 ms with 64, 0.42 with 32 (0.50 with
+// stages through registers), Si32 (V = 416) 0.15 and 0.10.  Warps whose subtile
+// lies outside or below the diagonal leave the tensor cores to the SM's
+// other CTAs.
+constexpr int kOK = 16;        // complex K per shared-memory stage
+constexpr int kOLd = kOK + 4;  // row pitch, 4 mod 8: conflict-free fragment reads
+constexpr int kOWideDim = 512; // valence dimension from which the tile is 64
 
-// Shared operands of one stage: A(k, r) and B(k, c), complex, interleaved.
-struct OStage {
-  double2 a[kOK][kOP];
-  double2 b[kOK][kOP];
+template <int TILE>
+struct OTile {
+  static constexpr int WN = TILE / 16;         // 8-column fragments per warp
+  static constexpr int threads = 4 * TILE;
+  static constexpr int ldk = TILE + 2;         // pitch of the Y product's k-major A
+  static constexpr int operand = TILE * kOLd;  // complex values of one operand of a stage
+  static constexpr size_t smem = sizeof(double2) * 2 * 2 * operand;
+  static constexpr int ctas = TILE == 64 ? 2 : 4;  // resident per SM
+  static_assert(kOK * ldk <= operand, "the k-major form fits the same buffer");
 };
 
-// Accumulate the stage into the warp's 16x16 complex tile, op(A)^T B with
-// op = conj when CONJ, by three real products per complex one (the 3M
-// form): t1 += ar br, t2 += ai bi, t3 += (ar -/+ ai)(br + bi).  Then
+// The warp's 16 x 8 WN subtile: origin, and whether any of it is wanted.
+struct OWarp {
+  int r0, c0;
+  bool on;
+};
+template <int WN>
+__device__ __forceinline__ OWarp owarp(int warp, int row0, int nrow, int col0, int ncol,
+                                       bool upper) {
+  OWarp w;
+  w.r0 = (warp >> 1) * 16;
+  w.c0 = (warp & 1) * 8 * WN;
+  w.on = row0 + w.r0 < nrow && col0 + w.c0 < ncol &&
+         !(upper && row0 + w.r0 > col0 + w.c0 + 8 * WN - 1);
+  return w;
+}
+
+// Accumulate one stage, op(A)^T B with op = conj when CONJ, by three real
+// products per complex one (the 3M form): t1 += ar br, t2 += ai bi,
+// t3 += (ar -/+ ai)(br + bi).  Then
 //   CONJ:  re = t1 + t2, im = t3 - t1 + t2
 //   plain: re = t1 - t2, im = t3 - t1 - t2.
-// Warp w owns rows 16*(w/2).. and columns 16*(w%2)..
-template <bool CONJ, bool REAL>
-__device__ __forceinline__ void ostage_mma(const OStage &st, double t1[2][2][2],
-                                           double t2[2][2][2], double t3[2][2][2],
-                                           int lane, int warp) {
-  const int r0 = (warp >> 1) * 16, cb = (warp & 1) * 16;
+// A(k, r) is at a[r kOLd + k], or (LDK > 0) a[k LDK + r]; B(k, c) at
+// b[c kOLd + k].
+template <bool CONJ, bool REAL, int LDK, int WN>
+__device__ __forceinline__ void ostage_mma(const double2 *a, const double2 *b, const OWarp &w,
+                                           double (&t1)[2][WN][2], double (&t2)[2][WN][2],
+                                           double (&t3)[2][WN][2], int lane) {
 #pragma unroll
   for (int ks = 0; ks < kOK; ks += 4) {
     const int kk = ks + (lane & 3);
-    double2 a[2], b[2];
-    double as[2], bs[2];
+    double2 x[2];
+    double xs[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-      a[t] = st.a[kk][r0 + 8 * t + (lane >> 2)];
-      b[t] = st.b[kk][cb + 8 * t + (lane >> 2)];
-      as[t] = CONJ ? a[t].x - a[t].y : a[t].x + a[t].y;
-      bs[t] = b[t].x + b[t].y;
+      const int r = w.r0 + 8 * t + (lane >> 2);
+      x[t] = LDK > 0 ? a[kk * LDK + r] : a[r * kOLd + kk];
+      xs[t] = CONJ ? x[t].x - x[t].y : x[t].x + x[t].y;
     }
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int nt = 0; nt < WN; ++nt) {
+      const double2 y = b[(w.c0 + 8 * nt + (lane >> 2)) * kOLd + kk];
+      const double ys = y.x + y.y;
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        dmma(t1[mt][nt][0], t1[mt][nt][1], a[mt].x, b[nt].x);
+      for (int mt = 0; mt < 2; ++mt) {
+        dmma(t1[mt][nt][0], t1[mt][nt][1], x[mt].x, y.x);
         if (REAL) continue;  // imaginary parts are zero: t2 = 0, t3 = t1
-        dmma(t2[mt][nt][0], t2[mt][nt][1], a[mt].y, b[nt].y);
-        dmma(t3[mt][nt][0], t3[mt][nt][1], as[mt], bs[nt]);
+        dmma(t2[mt][nt][0], t2[mt][nt][1], x[mt].y, y.y);
+        dmma(t3[mt][nt][0], t3[mt][nt][1], xs[mt], ys);
       }
+    }
   }
 }
 
@@ -600,63 +632,59 @@ __device__ __forceinline__ double2 ocombine(double t1, double t2, double t3) {
 
 // Y(c, v) = X_cv(c, v) - ycc sum_l X_cc(c, l) S(l, v), ycc = 1/2 for a
 // Hermitian X_cc (the her2k form) and 1 for the general form below.
-// Operands are staged through registers one K stage ahead of the MMAs.
-template <bool REAL>
-__global__ void __launch_bounds__(kOThreads, 4)
+template <bool REAL, int TILE>
+__global__ void __launch_bounds__(OTile<TILE>::threads, OTile<TILE>::ctas)
     k_ortho_y(DevSys s, const double2 *cv, const double2 *cc,
               const double2 *s_cv, double2 *y, double ycc) {
-  __shared__ OStage st;
+  using O = OTile<TILE>;
+  extern __shared__ double2 osm[];
   const int V = s.vale_dim, C = s.core_dim;
-  const int ntc = (C + kOT - 1) / kOT;
-  const int tr = blockIdx.x % ntc, tc = blockIdx.x / ntc;  // c tile, v tile
+  const int ntc = (C + TILE - 1) / TILE;
+  const int row0 = (blockIdx.x % ntc) * TILE, col0 = (blockIdx.x / ntc) * TILE;  // c, v
   const int k = blockIdx.y, term = blockIdx.z;
   const long long tk = (long long)term * s.nk + k;
   const double2 *XC = cc + tk * C * C;
   const double2 *S = s_cv + (long long)k * V * C;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double t1[2][2][2] = {}, t2[2][2][2] = {}, t3[2][2][2] = {};
-  double2 ra[kOLoads], rb[kOLoads];
-  auto fetch = [&](int l0) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const OWarp w = owarp<O::WN>(tid >> 5, row0, C, col0, V, false);
+  double t1[2][O::WN][2] = {}, t2[2][O::WN][2] = {}, t3[2][O::WN][2] = {};
+  auto issue = [&](int l0, int st) {
+    double2 *a = osm + st * 2 * O::operand, *b = a + O::operand;
 #pragma unroll
-    for (int q = 0; q < kOLoads; ++q) {
-      const int i = tid + q * kOThreads;
-      // A: X_cc(c, l), c fastest in memory
-      const int ar = i % kOT, ak = i / kOT;
-      const int l = l0 + ak, c = tr * kOT + ar;
-      ra[q] = (l < C && c < C) ? XC[(long long)l * C + c] : make_double2(0.0, 0.0);
-      // B: S(l, v), l fastest in memory
-      const int bk = i % kOK, br = i / kOK;
-      const int lb = l0 + bk, v = tc * kOT + br;
-      rb[q] = (lb < C && v < V) ? S[(long long)v * C + lb] : make_double2(0.0, 0.0);
+    for (int q = 0; q < kOK * TILE / O::threads; ++q) {
+      const int i = tid + q * O::threads;
+      // A: X_cc(c, l), c fastest in memory; B: S(l, v), l fastest
+      const int ar = i % TILE, ak = i / TILE, bk = i % kOK, br = i / kOK;
+      const bool ia = l0 + ak < C && row0 + ar < C, ib = l0 + bk < C && col0 + br < V;
+      cp_async16(&a[ak * O::ldk + ar], XC + (ia ? (long long)(l0 + ak) * C + row0 + ar : 0), ia);
+      cp_async16(&b[br * kOLd + bk], S + (ib ? (long long)(col0 + br) * C + l0 + bk : 0), ib);
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  auto store = [&]() {
-#pragma unroll
-    for (int q = 0; q < kOLoads; ++q) {
-      const int i = tid + q * kOThreads;
-      st.a[i / kOT][i % kOT] = ra[q];
-      st.b[i % kOK][i / kOK] = rb[q];
+  issue(0, 0);
+  for (int l0 = 0, st = 0; l0 < C; l0 += kOK, st ^= 1) {
+    if (l0 + kOK < C) {
+      issue(l0 + kOK, st ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
-  };
-  fetch(0);
-  for (int l0 = 0; l0 < C; l0 += kOK) {
     __syncthreads();
-    store();
+    const double2 *a = osm + st * 2 * O::operand;
+    if (w.on) ostage_mma<false, REAL, O::ldk, O::WN>(a, a + O::operand, w, t1, t2, t3, lane);
     __syncthreads();
-    if (l0 + kOK < C) fetch(l0 + kOK);
-    ostage_mma<false, REAL>(st, t1, t2, t3, lane, warp);
   }
+  if (!w.on) return;
   const double2 *X = cv + tk * V * C;
   double2 *Y = y + tk * V * C;
-  const int r0 = (warp >> 1) * 16, cb = (warp & 1) * 16;
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int nt = 0; nt < O::WN; ++nt)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int c = tr * kOT + r0 + 8 * mt + (lane >> 2);
-        const int v = tc * kOT + cb + 8 * nt + 2 * (lane & 3) + i;
+        const int c = row0 + w.r0 + 8 * mt + (lane >> 2);
+        const int v = col0 + w.c0 + 8 * nt + 2 * (lane & 3) + i;
         if (c >= C || v >= V) continue;
         const double2 x = X[(long long)v * C + c];
         const double2 p = ocombine<false, REAL>(t1[mt][nt][i], t2[mt][nt][i], t3[mt][nt][i]);
@@ -669,16 +697,17 @@ __global__ void __launch_bounds__(kOThreads, 4)
 // i(i+1)/2 + j.  The her2k form passes X2 = Y and makes the diagonal real;
 // the general form (`general`, X2 = X_cv, Y = X_cv - X_cc S) keeps on the
 // diagonal the imaginary part of S^H X_cc S = -Im W there.
-template <bool REAL, bool FULL = false>
-__global__ void __launch_bounds__(kOThreads, 4)
+template <bool REAL, bool FULL, int TILE>
+__global__ void __launch_bounds__(OTile<TILE>::threads, OTile<TILE>::ctas)
     k_ortho_w(DevSys s, const double2 *vv, const double2 *y, const double2 *x2,
-              const double2 *s_cv, double *packed, bool general, double *im_plane = nullptr) {
-  __shared__ OStage st;
+              const double2 *s_cv, double *packed, bool general, double *im_plane) {
+  using O = OTile<TILE>;
+  extern __shared__ double2 osm[];
   const int V = s.vale_dim, C = s.core_dim;
   // upper-triangular tile index -> (J, I), J <= I; FULL: every tile
   int I = 0, J = 0;
   if (FULL) {
-    const int tvv = (V + kOT - 1) / kOT;
+    const int tvv = (V + TILE - 1) / TILE;
     J = blockIdx.x % tvv;
     I = blockIdx.x / tvv;
   } else {
@@ -689,64 +718,55 @@ __global__ void __launch_bounds__(kOThreads, 4)
     }
     J = t;
   }
+  const int row0 = J * TILE, col0 = I * TILE;
   const int k = blockIdx.y, term = blockIdx.z;
   const long long tk = (long long)term * s.nk + k;
   const double2 *S = s_cv + (long long)k * V * C;
   const double2 *Y = y + tk * V * C, *X2 = x2 + tk * V * C;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int K2 = 2 * C;
-  double t1[2][2][2] = {}, t2[2][2][2] = {}, t3[2][2][2] = {};
-  // on a diagonal tile the warp owning rows 16..31 x columns 0..15 lies
-  // wholly below the diagonal, which is never stored
-  const bool lower = !FULL && J == I && (warp >> 1) > (warp & 1);
-  double2 ra[kOLoads], rb[kOLoads];
-  auto fetch = [&](int l0) {
+  const OWarp w = owarp<O::WN>(tid >> 5, row0, V, col0, V, !FULL);
+  double t1[2][O::WN][2] = {}, t2[2][O::WN][2] = {}, t3[2][O::WN][2] = {};
+  auto issue = [&](int l0, int st) {
+    double2 *a = osm + st * 2 * O::operand, *b = a + O::operand;
 #pragma unroll
-    for (int q = 0; q < kOLoads; ++q) {
-      const int i = tid + q * kOThreads;
-      const int kk = i % kOK, r = i / kOK;
-      const int l = l0 + kk;
-      const int j = J * kOT + r, ii = I * kOT + r;
-      double2 a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
-      if (l < K2) {
-        const double2 *Aop = l < C ? S : X2;  // (S; X2), conjugated in the MMA
-        const double2 *Bop = l < C ? Y : S;   // (Y; S)
-        const int lc = l < C ? l : l - C;
-        if (j < V) a = Aop[(long long)j * C + lc];
-        if (ii < V) b = Bop[(long long)ii * C + lc];
-      }
-      ra[q] = a;
-      rb[q] = b;
+    for (int q = 0; q < kOK * TILE / O::threads; ++q) {
+      const int i = tid + q * O::threads;
+      const int kk = i % kOK, r = i / kOK, l = l0 + kk;
+      const bool ia = l < K2 && row0 + r < V, ib = l < K2 && col0 + r < V;
+      const double2 *Aop = l < C ? S : X2;  // (S; X2), conjugated in the MMA
+      const double2 *Bop = l < C ? Y : S;   // (Y; S)
+      const int lc = l < C ? l : l - C;
+      cp_async16(&a[r * kOLd + kk], ia ? Aop + (long long)(row0 + r) * C + lc : S, ia);
+      cp_async16(&b[r * kOLd + kk], ib ? Bop + (long long)(col0 + r) * C + lc : S, ib);
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  auto store = [&]() {
-#pragma unroll
-    for (int q = 0; q < kOLoads; ++q) {
-      const int i = tid + q * kOThreads;
-      st.a[i % kOK][i / kOK] = ra[q];
-      st.b[i % kOK][i / kOK] = rb[q];
+  issue(0, 0);
+  for (int l0 = 0, st = 0; l0 < K2; l0 += kOK, st ^= 1) {
+    if (l0 + kOK < K2) {
+      issue(l0 + kOK, st ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
-  };
-  fetch(0);
-  for (int l0 = 0; l0 < K2; l0 += kOK) {
     __syncthreads();
-    store();
+    const double2 *a = osm + st * 2 * O::operand;
+    if (w.on) ostage_mma<true, REAL, 0, O::WN>(a, a + O::operand, w, t1, t2, t3, lane);
     __syncthreads();
-    if (l0 + kOK < K2) fetch(l0 + kOK);
-    if (!lower) ostage_mma<true, REAL>(st, t1, t2, t3, lane, warp);
   }
+  if (!w.on) return;
   const double2 *VVt = vv + tk * V * V;
   const long long np = (long long)V * (V + 1) / 2;
   const OutK out = out_k(s, packed, term, k, np);
-  const int r0 = (warp >> 1) * 16, cb = (warp & 1) * 16;
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int nt = 0; nt < O::WN; ++nt)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int row = J * kOT + r0 + 8 * mt + (lane >> 2);
-        const int col = I * kOT + cb + 8 * nt + 2 * (lane & 3) + i;
+        const int row = row0 + w.r0 + 8 * mt + (lane >> 2);
+        const int col = col0 + w.c0 + 8 * nt + 2 * (lane & 3) + i;
         if (row >= V || col >= V || (!FULL && row > col)) continue;
         double2 v = VVt[(long long)col * V + row];
         const double2 p = ocombine<true, REAL>(t1[mt][nt][i], t2[mt][nt][i], t3[mt][nt][i]);
@@ -765,6 +785,62 @@ __global__ void __launch_bounds__(kOThreads, 4)
         const long long idx = (long long)col * (col + 1) / 2 + row;
         store_out(out, idx, v);
       }
+}
+
+// Lets `kernel` take `bytes` of dynamic shared memory, once per device.
+template <class K>
+static int ortho_smem(K kernel, size_t bytes, bool (&done)[64]) {
+  int dev = 0;
+  IMAGO_CUDA(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && done[dev]) return IMAGO_OK;
+  IMAGO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (dev >= 0 && dev < 64) done[dev] = true;
+  return IMAGO_OK;
+}
+
+template <bool REAL, int TILE>
+static int ortho_y(const DevSys &s, int nterm, const double2 *cv, const double2 *cc,
+                   const double2 *s_cv, double2 *y, double ycc, cudaStream_t st) {
+  using O = OTile<TILE>;
+  static bool done[64] = {};
+  const int rc = ortho_smem(k_ortho_y<REAL, TILE>, O::smem, done);
+  if (rc) return rc;
+  const int tc = (s.core_dim + TILE - 1) / TILE, tv = (s.vale_dim + TILE - 1) / TILE;
+  k_ortho_y<REAL, TILE><<<dim3(tc * tv, s.nk, nterm), O::threads, O::smem, st>>>(s, cv, cc, s_cv, y,
+                                                                               ycc);
+  IMAGO_CUDA(cudaGetLastError());
+  return IMAGO_OK;
+}
+
+template <bool REAL, bool FULL, int TILE>
+static int ortho_w(const DevSys &s, int nterm, const double2 *vv, const double2 *y,
+                   const double2 *x2, const double2 *s_cv, double *packed, bool general,
+                   double *im, cudaStream_t st) {
+  using O = OTile<TILE>;
+  static bool done[64] = {};
+  const int rc = ortho_smem(k_ortho_w<REAL, FULL, TILE>, O::smem, done);
+  if (rc) return rc;
+  const int tv = (s.vale_dim + TILE - 1) / TILE;
+  const int tiles = FULL ? tv * tv : tv * (tv + 1) / 2;
+  k_ortho_w<REAL, FULL, TILE><<<dim3(tiles, s.nk, nterm), O::threads, O::smem, st>>>(
+      s, vv, y, x2, s_cv, packed, general, im);
+  IMAGO_CUDA(cudaGetLastError());
+  return IMAGO_OK;
+}
+
+// Both products of the tiled orthogonalisation, x2 null for X2 = Y.
+template <bool REAL, bool FULL>
+static int ortho_tiled(const DevSys &s, int nterm, const double2 *vv, const double2 *cv,
+                       const double2 *cc, const double2 *s_cv, double2 *y, double ycc,
+                       const double2 *x2, double *packed, bool general, double *im,
+                       cudaStream_t st) {
+  const double2 *b = x2 ? x2 : y;
+  if (s.vale_dim >= kOWideDim) {
+    const int rc = ortho_y<REAL, 64>(s, nterm, cv, cc, s_cv, y, ycc, st);
+    return rc ? rc : ortho_w<REAL, FULL, 64>(s, nterm, vv, y, b, s_cv, packed, general, im, st);
+  }
+  const int rc = ortho_y<REAL, 32>(s, nterm, cv, cc, s_cv, y, ycc, st);
+  return rc ? rc : ortho_w<REAL, FULL, 32>(s, nterm, vv, y, b, s_cv, packed, general, im, st);
 }
 
 // Small systems: the whole orthogonalisation of one (k, term) in one CTA.
@@ -1483,18 +1559,11 @@ int launch_ortho(const DevSys &s, int nterm, const double2 *vv,
     IMAGO_CUDA(cudaGetLastError());
     return IMAGO_OK;
   }
-  const int tcv = (C + kOT - 1) / kOT, tvv = (V + kOT - 1) / kOT;
-  dim3 gy(tcv * tvv, s.nk, nterm);
-  dim3 gw(tvv * (tvv + 1) / 2, s.nk, nterm);
-  if (s.real_k) {
-    k_ortho_y<true><<<gy, kOThreads, 0, st>>>(s, cv, cc, s_cv, y, 0.5);
-    k_ortho_w<true><<<gw, kOThreads, 0, st>>>(s, vv, y, y, s_cv, packed, false);
-  } else {
-    k_ortho_y<false><<<gy, kOThreads, 0, st>>>(s, cv, cc, s_cv, y, 0.5);
-    k_ortho_w<false><<<gw, kOThreads, 0, st>>>(s, vv, y, y, s_cv, packed, false);
-  }
-  IMAGO_CUDA(cudaGetLastError());
-  return IMAGO_OK;
+  if (s.real_k)
+    return ortho_tiled<true, false>(s, nterm, vv, cv, cc, s_cv, y, 0.5, nullptr, packed, false,
+                                    nullptr, st);
+  return ortho_tiled<false, false>(s, nterm, vv, cv, cc, s_cv, y, 0.5, nullptr, packed, false,
+                                   nullptr, st);
 }
 
 // The K-overlap phase sum (cmplxApplyPhaseFactors, intgSaving.F90:192-238;
@@ -1586,13 +1655,7 @@ int launch_ortho_full(const DevSys &s, const double2 *vv, const double2 *cv,
     IMAGO_CUDA(cudaGetLastError());
     return IMAGO_OK;
   }
-  const int tcv = (C + kOT - 1) / kOT, tvv = (V + kOT - 1) / kOT;
-  k_ortho_y<false><<<dim3(tcv * tvv, s.nk, 3), kOThreads, 0, st>>>(s, cv, cc, s_cv, y, 1.0);
-  IMAGO_CUDA(cudaGetLastError());
-  k_ortho_w<false, true><<<dim3(tvv * tvv, s.nk, 3), kOThreads, 0, st>>>(
-      s, vv, y, cv, s_cv, re, true, im);
-  IMAGO_CUDA(cudaGetLastError());
-  return IMAGO_OK;
+  return ortho_tiled<false, true>(s, 3, vv, cv, cc, s_cv, y, 1.0, cv, re, true, im, st);
 }
 
 // The orthogonalisation of a matrix whose core-core block is not Hermitian
@@ -1610,14 +1673,8 @@ int launch_ortho_general(const DevSys &s, int nterm, const double2 *vv,
   const int V = s.vale_dim, C = s.core_dim;
   if (nterm == 0) return IMAGO_OK;
   if (C == 0) return launch_ortho(s, nterm, vv, cv, cc, s_cv, y, packed, st);
-  const int tcv = (C + kOT - 1) / kOT, tvv = (V + kOT - 1) / kOT;
-  k_ortho_y<false><<<dim3(tcv * tvv, s.nk, nterm), kOThreads, 0, st>>>(s, cv, cc, s_cv,
-                                                                      y, 1.0);
-  IMAGO_CUDA(cudaGetLastError());
-  k_ortho_w<false><<<dim3(tvv * (tvv + 1) / 2, s.nk, nterm), kOThreads, 0, st>>>(
-      s, vv, y, cv, s_cv, packed, true);
-  IMAGO_CUDA(cudaGetLastError());
-  return IMAGO_OK;
+  return ortho_tiled<false, false>(s, nterm, vv, cv, cc, s_cv, y, 1.0, cv, packed, true, nullptr,
+                                   st);
 }
 
 // coreValeOL as the reference writes it: separate real and imaginary
