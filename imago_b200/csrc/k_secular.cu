@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <unordered_map>
 #include <vector>
 
 #include <cusolverDn.h>
@@ -59,6 +60,60 @@ __global__ void k_secular(int V, long long np, int nk, int pot_dim,
     const double2 o = make_double2(ol[pk], ol[pk + 1]);
     s[base + (long long)col * V + row] = o;
     s[base + (long long)row * V + col] = make_double2(o.x, -o.y);
+  }
+}
+
+// Hashes of each k-point's H and S, and of their conjugates, by which the
+// host finds k-points whose problem is another's conjugate (k and -k of an
+// integral build: the same bits with the imaginary parts negated).  Sums of
+// mixed bit patterns modulo 2^64 over the upper triangle, so the order of the
+// additions does not matter; H and S apart, 128 bits to agree on.  HBM-bound:
+// one pass over what k_secular wrote (Si8, 512 k: 0.18 GB).
+__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
+  x ^= x >> 30;
+  x *= 0xbf58476d1ce4e5b9ull;
+  x ^= x >> 27;
+  x *= 0x94d049bb133111ebull;
+  return x ^ (x >> 31);
+}
+
+__global__ void __launch_bounds__(256)
+    k_conj_hash(int V, const double2 *h, const double2 *s, unsigned long long *out) {
+  const int k = blockIdx.x;
+  const long long base = (long long)k * V * V;
+  unsigned long long sum[4] = {0, 0, 0, 0};  // H, conj H, S, conj S
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < V * V; e += gridDim.y * blockDim.x) {
+    const int col = e / V, row = e - col * V;
+    if (row > col) continue;
+    const unsigned long long at = 0x9e3779b97f4a7c15ull * (unsigned)(e + 1);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const double2 x = (m ? s : h)[base + e];
+      // + 0.0: -0 and +0 are one value
+      const unsigned long long re = mix64((unsigned long long)__double_as_longlong(x.x + 0.0) + at);
+      sum[2 * m] += mix64(re + (unsigned long long)__double_as_longlong(x.y + 0.0));
+      sum[2 * m + 1] += mix64(re + (unsigned long long)__double_as_longlong(0.0 - x.y));
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(out + 4 * k + m, sum[m]);
+  }
+}
+
+// out[k] = in[map[k]], or the conjugate of in[~map[k]] where map[k] < 0;
+// `per` complex values each.
+__global__ void __launch_bounds__(256)
+    k_conj_expand(long long per, const int *map, const double2 *in, double2 *out) {
+  const int k = blockIdx.x, m = map[k];
+  const double2 *src = in + (long long)(m < 0 ? ~m : m) * per;
+  const double sg = m < 0 ? -1.0 : 1.0;
+  for (long long e = blockIdx.y * (long long)blockDim.x + threadIdx.x; e < per;
+       e += (long long)gridDim.y * blockDim.x) {
+    const double2 x = src[e];
+    out[(long long)k * per + e] = make_double2(x.x, sg * x.y);
   }
 }
 
@@ -567,4 +622,57 @@ extern "C" int imago_secular_matrices(int vale_dim, int num_kpoints, int pot_dim
   return imago_secular_matrices_rel(vale_dim, num_kpoints, pot_dim, np_packed,
                                     ke_packed, nullptr, ep_packed, pot_coeffs,
                                     ol_packed, h_full, s_full, stream);
+}
+
+extern "C" int imago_secular_pairs(int n, int num_kpoints, const double *h_full,
+                                   const double *s_full, int *pair, void *stream) {
+  if (n <= 0 || num_kpoints < 0 || !h_full || !s_full || !pair) return IMAGO_ERR_INVALID;
+  if (n > 32767) return IMAGO_ERR_RANGE;
+  if (num_kpoints == 0) return IMAGO_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  const size_t bytes = sizeof(unsigned long long) * 4 * (size_t)num_kpoints;
+  void *d = nullptr;
+  if (imago::pool_alloc(&d, bytes, st) != cudaSuccess) {
+    cudaGetLastError();
+    return IMAGO_ERR_NOMEM;
+  }
+  std::vector<unsigned long long> hash(4 * (size_t)num_kpoints);
+  int rc = IMAGO_OK;
+  const unsigned per = (unsigned)std::max(1, std::min(64, 148 * 8 / num_kpoints));
+  if (cudaMemsetAsync(d, 0, bytes, st) != cudaSuccess) rc = IMAGO_ERR_CUDA;
+  if (!rc) {
+    imago::k_conj_hash<<<dim3(num_kpoints, per), 256, 0, st>>>(
+        n, reinterpret_cast<const double2 *>(h_full), reinterpret_cast<const double2 *>(s_full),
+        static_cast<unsigned long long *>(d));
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(hash.data(), d, bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+      rc = IMAGO_ERR_CUDA;
+  }
+  cudaFreeAsync(d, st);
+  cudaGetLastError();
+  if (rc) return rc;
+  // a k-point takes the first earlier one that is its conjugate
+  std::unordered_multimap<unsigned long long, int> seen;
+  for (int k = 0; k < num_kpoints; ++k) {
+    const unsigned long long *x = &hash[4 * (size_t)k];
+    int first = -1;
+    const auto range = seen.equal_range(x[1]);
+    for (auto it = range.first; it != range.second; ++it)
+      if (hash[4 * (size_t)it->second + 2] == x[3] && (first < 0 || it->second < first))
+        first = it->second;
+    pair[k] = first < 0 ? k : first;
+    if (first < 0) seen.emplace(x[0], k);
+  }
+  return IMAGO_OK;
+}
+
+extern "C" int imago_conj_expand(int num_kpoints, long long per, const int *map,
+                                 const double *in, double *out, void *stream) {
+  if (num_kpoints < 0 || per < 0 || !map || !in || !out) return IMAGO_ERR_INVALID;
+  if (num_kpoints == 0 || per == 0) return IMAGO_OK;
+  const unsigned grid = (unsigned)std::min<long long>((per + 255) / 256, 1024);
+  imago::k_conj_expand<<<dim3(num_kpoints, grid), 256, 0, (cudaStream_t)stream>>>(
+      per, map, reinterpret_cast<const double2 *>(in), reinterpret_cast<double2 *>(out));
+  return cudaGetLastError() == cudaSuccess ? (int)IMAGO_OK : (int)IMAGO_ERR_CUDA;
 }

@@ -417,6 +417,21 @@ IMAGO_API int imago_hermitian_eigh(int n, int batch, const double *a, double *w,
 IMAGO_API int imago_hermitian_set_solver(int mode);
 IMAGO_API int imago_hermitian_solver(int *mode);
 
+/* K-points whose secular problem is another's conjugate, H(k') = conj H(k)
+ * and S(k') = conj S(k) bit for bit (k and -k of an integral build):
+ * pair[k] (host, num_kpoints ints) is the first such k-point before k, or k
+ * itself.  Found by 128 bits of hashes of h_full and s_full (device,
+ * [num_kpoints][n][n] (re, im), upper triangle by columns as
+ * imago_secular_matrices writes them).  Waits for `stream`. */
+IMAGO_API int imago_secular_pairs(int n, int num_kpoints, const double *h_full,
+                                  const double *s_full, int *pair, void *stream);
+
+/* out[k] = in[map[k]], or the conjugate of in[-1 - map[k]] where map[k] < 0
+ * (map on the device), `per` (re, im) values each: results of the k-points
+ * solved spread over all of them.  Asynchronous on `stream`. */
+IMAGO_API int imago_conj_expand(int num_kpoints, long long per, const int *map,
+                                const double *in, double *out, void *stream);
+
 /* The Cholesky reduction of zhegv(1, 'V', 'U') (interfaces.F90:73-120:
  * zpotrf, then zhegst) for every k-point: S = L L^H (L = U^H, zpotrf's
  * factor) and A = L^-1 H L^-H.  h_full and s_full as

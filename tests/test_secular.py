@@ -186,3 +186,71 @@ def test_batched_eigensolver_beyond_the_jacobi_kernel(imago_lib, n):
         assert np.abs(np.conj(v[b].T) @ v[b] - np.eye(n)).max() < 1e-10
     assert np.abs(secular.hermitian_eigvals(at).cpu().numpy() - ref).max() < \
         1e-10 * np.abs(ref).max()
+
+
+def _hermitian(rng, nk, n):
+    a = rng.normal(size=(nk, n, n)) + 1j * rng.normal(size=(nk, n, n))
+    return a + a.conj().transpose(0, 2, 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 7, 64, 130])
+def test_conjugate_k_points_are_solved_once(imago_lib, monkeypatch, n):
+    # random problems, some of them another's conjugate (one twice, one real
+    # and its own conjugate): the pairs found, and the eigenvalues and the
+    # projectors equal to solving every k-point
+    import torch
+    from imago_b200 import secular
+    rng = np.random.default_rng(n)
+    h, g = _hermitian(rng, 4, n), _hermitian(rng, 4, n)
+    h[3], g[3] = h[3].real, g[3].real
+    s = g @ g.conj().transpose(0, 2, 1) + 2.0 * n * np.eye(n)
+    s = 0.5 * (s + s.conj().transpose(0, 2, 1))
+    order = [(0, 0), (1, 0), (0, 1), (2, 0), (3, 0), (1, 1), (0, 1), (2, 0)]
+    take = lambda x: np.stack([x[i].conj() if c else x[i] for i, c in order])
+    # for n = 1 every conjugate equals its original
+    expect = [0, 1, 0, 3, 4, 1, 0, 3 if n == 1 else 7]
+    pack = lambda x: torch.as_tensor(np.stack([x[:, r, c] for c in range(n) for r in range(c + 1)], 1)
+                                     .view(np.float64).reshape(len(order), -1, 2), device="cuda")
+    out = {"np_packed": pack(take(h)), "ol_packed": pack(take(s)), "ep_packed": None}
+    out["ke_packed"] = torch.zeros_like(out["np_packed"])
+    res = {}
+    for name, least in (("all", 1 << 60), ("pairs", 0)):
+        monkeypatch.setattr(secular, "PAIR_MIN", least)
+        if n > 128 and least:  # beyond 128 pairs are always looked for: one by one
+            lone = [secular.secular_eigensystem({k: None if v is None else v[i:i + 1]
+                                                 for k, v in out.items()}, np.zeros(0))
+                    for i in range(len(order))]
+            e, c = torch.cat([x[0] for x in lone]), torch.cat([x[1] for x in lone])
+        else:
+            e, c = secular.secular_eigensystem(out, np.zeros(0))
+            ev = secular.secular_eigenvalues(out, np.zeros(0))
+            assert np.abs((e - ev).cpu().numpy()).max() <= 1e-12 * np.abs(e.cpu().numpy()).max()
+        res[name] = (e.cpu().numpy(), c.cpu().numpy())
+    hs, ss = secular._secular_storage(out, np.zeros(0))
+    conj = secular._Conjugates(hs, ss)
+    assert list(conj.first) == [k for k in range(len(order)) if expect[k] == k]
+    (e0, c0), (e1, c1) = res["all"], res["pairs"]
+    assert np.abs(e0 - e1).max() <= 1e-12 * np.abs(e0).max()
+    # c diag(e) c^H S c = c diag(e): compare the phase-free H-like sums
+    p0, p1 = [(c * e[:, None, :]) @ c.conj().transpose(0, 2, 1) for e, c in ((e0, c0), (e1, c1))]
+    assert np.abs(p0 - p1).max() <= 1e-11 * np.abs(p0).max()
+
+
+@pytest.mark.gpu
+def test_failing_overlap_names_its_k_point_among_pairs(imago_lib, monkeypatch):
+    import torch
+    from imago_b200 import secular
+    rng = np.random.default_rng(5)
+    n, nk = 6, 5
+    a = _hermitian(rng, nk, n)
+    a[2] = a[0].conj()
+    s = np.stack([np.eye(n, dtype=complex)] * nk)
+    s[3, 1, 1] = -1.0
+    pack = lambda x: torch.as_tensor(np.stack([x[:, r, c] for c in range(n) for r in range(c + 1)], 1)
+                                     .view(np.float64).reshape(nk, -1, 2), device="cuda")
+    out = {"np_packed": pack(a), "ol_packed": pack(s), "ep_packed": None}
+    out["ke_packed"] = torch.zeros_like(out["np_packed"])
+    monkeypatch.setattr(secular, "PAIR_MIN", 0)
+    with pytest.raises(ValueError, match="k-point 3 .*leading minor 2"):
+        secular.secular_eigensystem(out, np.zeros(0))
