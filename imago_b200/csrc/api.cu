@@ -1107,6 +1107,9 @@ int upload(imago_ctx *c) {
   w.pairs = c->d_pairs.p; w.units = c->d_units.p; w.sps = c->d_sps.p;
   w.sp_by_cls = c->d_sp_by_cls.p;
   w.blk_total = c->blk_total;
+  w.blk_max = 4;
+  for (int k = 0; k < 16; ++k)
+    if (c->cls_beg[k + 1] > c->cls_beg[k]) w.blk_max = std::max(w.blk_max, blk_len(k / 4, k % 4));
   w.m_total = c->m_total;
   w.nbtile = (int)c->btile.size();
   w.btile = c->d_btile.p;

@@ -96,6 +96,7 @@ struct DevWork {
   const DSp *sps;
   const int *sp_by_cls;   // shell pairs sorted by class (la*4+lb), then unit
   long long blk_total;    // doubles of sh blocks per term
+  int blk_max;            // doubles of the largest one
   long long m_total;      // doubles of unit blocks per term
   int nbtile;             // phase-sum column tiles of kBlochCols: (pair, tile)
   const int2 *btile;

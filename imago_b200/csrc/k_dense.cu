@@ -1,5 +1,5 @@
-// k_dense.cu -- contraction, lattice-to-k phase sums, scatter and core
-// orthogonalisation of one integral build.
+// k_dense.cu -- lattice-to-k phase sums, scatter and core orthogonalisation
+// of one integral build.
 //
 // The phase sums and the orthogonalisation are dense complex contractions
 // and run on the FP64 tensor cores (mma.sync m8n8k4 f64), tiled through
@@ -78,148 +78,6 @@ __device__ __forceinline__ void cp_async8z(void *smem, const void *gmem,
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst),
                "l"(gmem), "r"(n)
                : "memory");
-}
-
-// 8-byte global-to-shared copy that does not pass through registers.
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
-  const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(gmem)
-               : "memory");
-}
-
-// ---------------------------------------------------------- contract --
-// One CTA per (unit, group of terms), threads over the block elements:
-//   M_t(m1, m2) = sum_{(a,b) in unit} C1(a, m1) C2(b, m2) sh_t,ab(lm1, lm2),
-// the pairXBasisFn2 / multWithBasisFn1 contraction (integrals.F90:555-563,
-// intgSaving.F90:56-89).  Entries whose lm lies beyond a primitive's class
-// carry a zero coefficient in the reference and are skipped.  Blocks are
-// stored column-major, e = m2 * ni + m1.  A unit's primitive blocks of one
-// term are contiguous in `blk`: they are staged through shared memory in
-// chunks of whole shell pairs with coalesced loads, together with the
-// chunk's shell-pair list and both atoms' coefficient tables; the
-// coefficient product of an (element, shell pair) serves every term of
-// the group.  T = 4 or 8 terms per CTA, picked by measurement: eight halve
-// the per-(element, shell pair) work of a many-term build but give fewer
-// CTAs and a smaller staging chunk.
-constexpr int kContractThreads = 128;
-constexpr int kElemsPerThread = 3;          // n_i n_j <= 384 per pass
-constexpr int kSpStage = 256;               // shell pairs staged at a time
-constexpr int kCoefMax = 1024;              // alphas x states per atom
-
-template <int T>
-__global__ void __launch_bounds__(kContractThreads, 4)
-    k_contract(DevSys s, DevWork w, int nterm, const double *blk, double *M) {
-  constexpr int kTermsPerCta = T;
-  constexpr int kBlkStage = T >= 8 ? 384 : 768;  // block doubles per term staged
-  __shared__ int sp_ab[kSpStage];            // a | b << 16
-  __shared__ int sp_cls[kSpStage];           // nsh(la) | nsh(lb) << 8
-  __shared__ int sp_rel[kSpStage];           // block offset from the chunk's
-  __shared__ double c1s[kCoefMax], c2s[kCoefMax];
-  __shared__ double bs[kTermsPerCta][kBlkStage];
-  __shared__ long long chunk_base;
-  const int ntg = (nterm + kTermsPerCta - 1) / kTermsPerCta;
-  const int ui = blockIdx.x / ntg;
-  const int t0 = (blockIdx.x % ntg) * kTermsPerCta;
-  const int tn = min(kTermsPerCta, nterm - t0);
-  const int tid = threadIdx.x;
-  const DUnit u = w.units[ui];
-  const DPair p = w.pairs[u.pair];
-  const int ni = p.ni, nj = p.nj, ne = ni * nj;
-  const int na1 = s.type_nalpha[p.ti], na2 = s.type_nalpha[p.tj];
-  const long long base = p.moff + (long long)(ui - p.ubeg) * ne;
-  const int so1 = s.type_state_off[p.ti], so2 = s.type_state_off[p.tj];
-  const double *c1 = s.basis + s.type_basis_off[p.ti];
-  const double *c2 = s.basis + s.type_basis_off[p.tj];
-  const bool stage_coef = na1 * ni <= kCoefMax && na2 * nj <= kCoefMax;
-  if (stage_coef) {
-    for (int i = tid; i < na1 * ni; i += kContractThreads) c1s[i] = c1[i];
-    for (int i = tid; i < na2 * nj; i += kContractThreads) c2s[i] = c2[i];
-  }
-  const double *cf1 = stage_coef ? c1s : c1;
-  const double *cf2 = stage_coef ? c2s : c2;
-  const double *bt = blk + (long long)t0 * w.blk_total;
-  for (int e0 = 0; e0 < ne; e0 += kContractThreads * kElemsPerThread) {
-    int lm1[kElemsPerThread], lm2[kElemsPerThread], m1[kElemsPerThread],
-        m2[kElemsPerThread];
-    double acc[kElemsPerThread][kTermsPerCta];
-#pragma unroll
-    for (int j = 0; j < kElemsPerThread; ++j) {
-      const int e = e0 + tid + j * kContractThreads;
-      m2[j] = e < ne ? e / ni : 0;
-      m1[j] = e < ne ? e - m2[j] * ni : 0;
-      lm1[j] = e < ne ? s.state_lm[so1 + m1[j]] : 1 << 20;
-      lm2[j] = e < ne ? s.state_lm[so2 + m2[j]] : 1 << 20;
-#pragma unroll
-      for (int t = 0; t < kTermsPerCta; ++t) acc[j][t] = 0.0;
-    }
-    for (int q0 = u.spbeg; q0 < u.spend;) {
-      const int nq = min(kSpStage, u.spend - q0);
-      __syncthreads();
-      // shell pairs of the chunk: those whose blocks end within kBlkStage
-      // doubles of the first one's start (at least one: a block has <= 256)
-      int fit = 0;
-      for (int i = tid; i < kSpStage; i += kContractThreads) {
-        if (i < nq) {
-          const DSp sp = w.sps[q0 + i];
-          const long long b0 = w.sps[q0].boff;
-          const int rel = (int)(sp.boff - b0);
-          sp_ab[i] = sp.a | (sp.b << 16);
-          sp_cls[i] = nsh(sp.la) | (nsh(sp.lb) << 8);
-          sp_rel[i] = rel;
-          fit += rel + nsh(sp.la) * nsh(sp.lb) <= kBlkStage;
-          if (i == 0) chunk_base = b0;
-        }
-      }
-      const int cnt = max(1, __syncthreads_count(fit > 0 && tid < nq) +
-                                 __syncthreads_count(fit > 1));
-      const int last = cnt - 1;
-      const int len = sp_rel[last] + (sp_cls[last] & 0xff) * (sp_cls[last] >> 8);
-      const double *src = bt + chunk_base;
-      for (int t = 0; t < tn; ++t)
-        for (int i = tid; i < len; i += kContractThreads)
-          cp_async8(&bs[t][i], src + (long long)t * w.blk_total + i);
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      __syncthreads();
-      for (int q = 0; q < cnt; ++q) {
-        const int ab = sp_ab[q], cl = sp_cls[q];
-        const int a = ab & 0xffff, b = ab >> 16, na = cl & 0xff, nb = cl >> 8;
-        const int rel = sp_rel[q];
-#pragma unroll
-        for (int j = 0; j < kElemsPerThread; ++j) {
-          if (lm1[j] >= na || lm2[j] >= nb) continue;
-          const double cw = cf1[a * ni + m1[j]] * cf2[b * nj + m2[j]];
-          const int o = rel + lm1[j] * nb + lm2[j];
-#pragma unroll
-          for (int t = 0; t < kTermsPerCta; ++t)
-            if (t < tn) acc[j][t] += cw * bs[t][o];
-        }
-      }
-      q0 += cnt;
-    }
-#pragma unroll
-    for (int j = 0; j < kElemsPerThread; ++j) {
-      const int e = e0 + tid + j * kContractThreads;
-      if (e >= ne) continue;
-#pragma unroll
-      for (int t = 0; t < kTermsPerCta; ++t)
-        if (t < tn) M[(long long)(t0 + t) * w.m_total + base + e] = acc[j][t];
-    }
-  }
-}
-
-int launch_contract(const DevSys &s, const DevWork &w, int nterm,
-                    const double *blk, double *M, cudaStream_t st, int terms_per_cta) {
-  if (w.nunits == 0 || nterm == 0) return IMAGO_OK;
-  if (terms_per_cta >= 8 && nterm > 4) {
-    const long long grid = (long long)w.nunits * ((nterm + 7) / 8);
-    k_contract<8><<<(unsigned)grid, kContractThreads, 0, st>>>(s, w, nterm, blk, M);
-  } else {
-    const long long grid = (long long)w.nunits * ((nterm + 3) / 4);
-    k_contract<4><<<(unsigned)grid, kContractThreads, 0, st>>>(s, w, nterm, blk, M);
-  }
-  IMAGO_CUDA(cudaGetLastError());
-  return IMAGO_OK;
 }
 
 // ------------------------------------------------------------- bloch --
