@@ -58,10 +58,16 @@ __global__ void __launch_bounds__(128, LA + LB >= 4 ? 3 : 4)
     __syncwarp();
     const float tf = __double2float_ru(tmax);
     const UnitWalk uw = unit_walk(s, w, sp.unit, pt);
+    ImageRef en = uw.beg + sub < uw.end ? uw.at(uw.beg + sub) : ImageRef{0, 0.f};
+    double4 Cn = w.ipos[en.idx];
     for (int r = uw.beg + sub; r < uw.end; r += T) {
-      const ImageRef e = uw.at(r);
+      const ImageRef e = en;
       if (beyond(e.d1, c.pmf, tf)) break;
-      const double4 C = w.ipos[e.idx];
+      const double4 C = Cn;
+      if (r + T < uw.end) {  // one image ahead
+        en = uw.at(r + T);
+        Cn = w.ipos[en.idx];
+      }
       const double d2 = image_d2(c.Ps, C);
       if (d2 > tmax) continue;
       const double X[3] = {c.Pt[0] - C.x, c.Pt[1] - C.y, c.Pt[2] - C.z};

@@ -101,10 +101,16 @@ __device__ __forceinline__ void prim3c_item(const DevSys &s, const DevWork &w, i
         c.reach2(s.T, NUC ? s.ptype_nucalpha[ps] : s.palpha[s.ptype_alpha_off[ps] + tm.j]);
     const float tf = __double2float_ru(t);
     const UnitWalk uw = unit_walk(s, w, sp.unit, pt);
+    ImageRef en = uw.beg < uw.end ? uw.at(uw.beg) : ImageRef{0, 0.f};
+    double4 Cn = w.ipos[en.idx];
     for (int r = uw.beg; r < uw.end; ++r) {
-      const ImageRef e = uw.at(r);
+      const ImageRef e = en;
       if (beyond(e.d1, c.pmf, tf)) break;
-      const double4 C = w.ipos[e.idx];
+      const double4 C = Cn;
+      if (r + 1 < uw.end) {  // one image ahead
+        en = uw.at(r + 1);
+        Cn = w.ipos[en.idx];
+      }
       if (image_d2(c.Ps, C) > t) continue;
       if constexpr (CNT) {
         ++*ntrip;
