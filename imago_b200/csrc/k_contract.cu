@@ -127,20 +127,22 @@ __global__ void __launch_bounds__(kContractThreads, T == 8 ? 3 : 4)
           if (t < tn) M[(long long)(t0 + t) * w.m_total + base + e] = acc[j][t];
       }
     };
-    // chunk ch of group g into buffer b: 16-byte copies, the blocks start on
-    // 32 bytes and are padded
+    // chunk ch of group g into buffer b: 16-byte copies (the blocks start on
+    // 32 bytes and are padded), 128 / T threads to a term so that a thread
+    // forms one address
     auto issue = [&](int g, int ch, int b) {
-      const int t0 = g * T, tn = min(T, nterm - t0);
-      const int q = cb[ch + 1] - 1, r0 = sp_rel[cb[ch]];
-      const int len = (sp_rel[q] + (sp_cls[q] & 0xff) * (sp_cls[q] >> 8) - r0 + 1) / 2;
-      const double *src = blk + (long long)t0 * w.blk_total + boff0 + r0;
-      for (int t = 0; t < tn; ++t)
-        for (int i = tid; i < len; i += kContractThreads) {
-          const unsigned dst = (unsigned)__cvta_generic_to_shared(bs + (b * T + t) * buf + 2 * i);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst),
-                       "l"(src + (long long)t * w.blk_total + 2 * i)
+      constexpr int per = kContractThreads / T;
+      const int t = tid / per;
+      if (t < nterm - g * T) {
+        const int q = cb[ch + 1] - 1, r0 = sp_rel[cb[ch]];
+        const int len = (sp_rel[q] + (sp_cls[q] & 0xff) * (sp_cls[q] >> 8) - r0 + 1) / 2;
+        const double *src = blk + (long long)(g * T + t) * w.blk_total + boff0 + r0;
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(bs + (b * T + t) * buf);
+        for (int i = tid % per; i < len; i += per)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * i),
+                       "l"(src + 2 * i)
                        : "memory");
-        }
+      }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
     // groups [ga, gb) over the current list
