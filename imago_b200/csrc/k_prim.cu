@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(128)
   if (g >= end) return;
   const DSp sp = w.sps[w.sp_by_cls[g]];
   const SpGeom q = sp_geom(s, w, sp);
-  prim2c<LA, LB, KIN>(q.a1, q.a2, q.A, q.B, blk + sp.boff);
+  prim2c<LA, LB, KIN, true>(q.a1, q.a2, q.A, q.B, blk + sp.boff);
 }
 
 // Mass velocity (built once per SCF run, rel = 1): s/p/d classes unrolled,
@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(128)
   if (g >= end) return;
   const DSp sp = w.sps[w.sp_by_cls[g]];
   const SpGeom q = sp_geom(s, w, sp);
-  prim_mv<LA, LB>(q.a1, q.a2, q.A, q.B, -kMassVelPref, blk + sp.boff);
+  prim_mv<LA, LB, true>(q.a1, q.a2, q.A, q.B, -kMassVelPref, blk + sp.boff);
 }
 
 __global__ void __launch_bounds__(128)
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128)
   const DSp sp = w.sps[w.sp_by_cls[g]];
   const SpGeom q = sp_geom(s, w, sp);
   const double C[3] = {center.x, center.y, center.z};
-  prim_vec<LA, LB, DIP>(q.a1, q.a2, q.A, q.B, C, blk + sp.boff, w.blk_total);
+  prim_vec<LA, LB, DIP, true>(q.a1, q.a2, q.A, q.B, C, blk + sp.boff, w.blk_total);
 }
 
 template <bool DIP>

@@ -111,6 +111,20 @@ __device__ __forceinline__ void os1d(double PA, double PB, double inv2p,
     }
 }
 
+// f(0), f(1), ... f(N - 1) with the index as a type, so that everything
+// derived from it is a constant and small arrays stay in registers.
+template <int I>
+struct Idx {
+  static constexpr int value = I;
+};
+template <int N, int I = 0, class F>
+__device__ __forceinline__ void static_for(F &&f) {
+  if constexpr (I < N) {
+    f(Idx<I>{});
+    static_for<N, I + 1>(f);
+  }
+}
+
 // Four doubles in one 32-byte store (one whole sector; 32-byte aligned).
 __device__ __forceinline__ void store4(double *p, const double v[4]) {
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]),
@@ -118,27 +132,56 @@ __device__ __forceinline__ void store4(double *p, const double v[4]) {
                : "memory");
 }
 
-// Write the real-solid-harmonic block from a Cartesian block
-// pc[p * ncart(LB) + q].
-template <int LA, int LB>
-__device__ __forceinline__ void cart_to_sh(const double *pc, double *out) {
-#pragma unroll
-  for (int s1 = 0; s1 < nsh(LA); ++s1)
-#pragma unroll
-    for (int s2 = 0; s2 < nsh(LB); ++s2) {
-      double v = 0.0;
-#pragma unroll
-      for (int k1 = 0; k1 < 3; ++k1) {
-        if (k1 >= sh_nterm(s1)) break;
-#pragma unroll
-        for (int k2 = 0; k2 < 3; ++k2) {
-          if (k2 >= sh_nterm(s2)) break;
-          v += sh_coef(s1, k1) * sh_coef(s2, k2) *
-               pc[sh_cart(s1, k1) * ncart(LB) + sh_cart(s2, k2)];
-        }
+// A block's rows as they are finished: to `out`, or (PAD) to a build's
+// block buffer, where every block starts on 32 bytes and has blk_len
+// doubles: each thread writes its own block, so single 8-byte stores would
+// send one partial sector each (162-atom quartz EP: 2.0 G of them; whole
+// sectors are a quarter; overlap and kinetic blocks of that cell 0.43 and
+// 0.33 ms with 8-byte stores and the Cartesian block in local memory, 0.11
+// and 0.12 so).
+template <int N, bool PAD>
+struct BlockWriter {
+  double *out;
+  double quad[4];
+  template <int R, int M>
+  __device__ __forceinline__ void row(const double (&v)[M]) {
+    static_for<M>([&](auto im) {
+      constexpr int m = decltype(im)::value, o = R * M + m;
+      if constexpr (!PAD) {
+        out[o] = v[m];
+      } else {
+        quad[o & 3] = v[m];
+        if constexpr (o == N - 1)
+          for (int i = (o & 3) + 1; i < 4; ++i) quad[i] = 0.0;
+        if constexpr (o == N - 1 || (o & 3) == 3) store4(out + (o & ~3), quad);
       }
-      out[s1 * nsh(LB) + s2] = v;
-    }
+    });
+  }
+};
+
+// A block from its Cartesian products cart(p, q), each formed where a
+// harmonic needs it.
+template <int LA, int LB, bool PAD, class F>
+__device__ __forceinline__ void write_sh_block(F &&cart, double *out) {
+  BlockWriter<nsh(LA) * nsh(LB), PAD> w{out, {}};
+  static_for<nsh(LA)>([&](auto i1) {
+    constexpr int s1 = decltype(i1)::value;
+    double row[nsh(LB)];
+    static_for<nsh(LB)>([&](auto i2) {
+      constexpr int s2 = decltype(i2)::value;
+      double v = 0.0;
+      static_for<sh_nterm(s1)>([&](auto j1) {
+        static_for<sh_nterm(s2)>([&](auto j2) {
+          constexpr int k1 = decltype(j1)::value, k2 = decltype(j2)::value;
+          constexpr int p = sh_cart(s1, k1), q = sh_cart(s2, k2);
+          constexpr double f = sh_coef(s1, k1) * sh_coef(s2, k2);
+          v += f * cart(p, q);
+        });
+      });
+      row[s2] = v;
+    });
+    w.template row<s1>(row);
+  });
 }
 
 // Two-centre overlap (KIN = false) or kinetic energy (KIN = true) between
@@ -148,8 +191,8 @@ __device__ __forceinline__ void cart_to_sh(const double *pc, double *out) {
 //   T_{i+1,j} = PA T_ij + (i T_{i-1,j} + j T_{i,j-1})/(2p)
 //               + 2 xi (S_{i+1,j} - i/(2 a1) S_{i-1,j})   (and j likewise),
 //   KE = pref (Tx Sy Sz + Sx Ty Sz + Sx Sy Tz).
-template <int LA, int LB, bool KIN>
-__device__ void prim2c(double a1, double a2, const double *A, const double *B,
+template <int LA, int LB, bool KIN, bool PAD = false>
+__device__ __forceinline__ void prim2c(double a1, double a2, const double *A, const double *B,
                        double *out) {
   const double zeta = a1 + a2, xi = a1 * a2 / zeta, inv2p = 1.0 / (2.0 * zeta);
   double S[3][LA + 1][LB + 1];
@@ -185,23 +228,20 @@ __device__ void prim2c(double a1, double a2, const double *A, const double *B,
     }
   }
   const double pref = pow(kPi / zeta, 1.5) * exp(-xi * d2);
-  double pc[ncart(LA) * ncart(LB)];
-#pragma unroll
-  for (int p = 0; p < ncart(LA); ++p)
-#pragma unroll
-    for (int q = 0; q < ncart(LB); ++q) {
-      const int ax = cart_exp(p, 0), ay = cart_exp(p, 1), az = cart_exp(p, 2);
-      const int bx = cart_exp(q, 0), by = cart_exp(q, 1), bz = cart_exp(q, 2);
-      double v;
-      if (KIN)
-        v = T[0][ax][bx] * S[1][ay][by] * S[2][az][bz] +
-            S[0][ax][bx] * T[1][ay][by] * S[2][az][bz] +
-            S[0][ax][bx] * S[1][ay][by] * T[2][az][bz];
-      else
-        v = S[0][ax][bx] * S[1][ay][by] * S[2][az][bz];
-      pc[p * ncart(LB) + q] = pref * v;
-    }
-  cart_to_sh<LA, LB>(pc, out);
+  write_sh_block<LA, LB, PAD>(
+      [&](int p, int q) {
+        const int ax = cart_exp(p, 0), ay = cart_exp(p, 1), az = cart_exp(p, 2);
+        const int bx = cart_exp(q, 0), by = cart_exp(q, 1), bz = cart_exp(q, 2);
+        double v;
+        if (KIN)
+          v = T[0][ax][bx] * S[1][ay][by] * S[2][az][bz] +
+              S[0][ax][bx] * T[1][ay][by] * S[2][az][bz] +
+              S[0][ax][bx] * S[1][ay][by] * T[2][az][bz];
+        else
+          v = S[0][ax][bx] * S[1][ay][by] * S[2][az][bz];
+        return pref * v;
+      },
+      out);
 }
 
 // (alpha^2 / 8) with alpha the fine structure constant 7.2973525693e-3,
@@ -246,8 +286,8 @@ __device__ __forceinline__ double d2_both(const double S[IA + 1][JB + 1],
 // whose terms carry the size of the result; the reference's recursion seeds
 // on 16 a2^4 <r_B^4> - 80 a2^3 <r_B^2> + 60 a2^2, which cancels to a value
 // of order a1 a2 when a1 << a2.  s, p and d classes only (registers).
-template <int LA, int LB>
-__device__ void prim_mv(double a1, double a2, const double *A, const double *B,
+template <int LA, int LB, bool PAD = false>
+__device__ __forceinline__ void prim_mv(double a1, double a2, const double *A, const double *B,
                         double scale, double *out) {
   const double zeta = a1 + a2, xi = a1 * a2 / zeta, inv2p = 1.0 / (2.0 * zeta);
   // per axis: S, L (left d^2), R (right d^2), U (both) for i <= LA, j <= LB;
@@ -284,22 +324,7 @@ __device__ void prim_mv(double a1, double a2, const double *A, const double *B,
     v += (l0 * r1 + r0 * l1) * s2 + (l0 * r2 + r0 * l2) * s1 + (l1 * r2 + r1 * l2) * s0;
     return pref * v;
   };
-#pragma unroll
-  for (int s1 = 0; s1 < nsh(LA); ++s1)
-#pragma unroll
-    for (int s2 = 0; s2 < nsh(LB); ++s2) {
-      double v = 0.0;
-#pragma unroll
-      for (int k1 = 0; k1 < 3; ++k1) {
-        if (k1 >= sh_nterm(s1)) break;
-#pragma unroll
-        for (int k2 = 0; k2 < 3; ++k2) {
-          if (k2 >= sh_nterm(s2)) break;
-          v += sh_coef(s1, k1) * sh_coef(s2, k2) * cart(sh_cart(s1, k1), sh_cart(s2, k2));
-        }
-      }
-      out[s1 * nsh(LB) + s2] = v;
-    }
+  write_sh_block<LA, LB, PAD>(cart, out);
 }
 
 // Momentum <a|d/dx_c|b> (DIP = false) or dipole <a|(r - C)_c|b> (DIP =
@@ -321,8 +346,8 @@ __device__ __forceinline__ double vec_factor(const double S[IA + 1][JB + 1],
 }
 
 // s, p and d classes: bounds known at compile time, tables in registers.
-template <int LA, int LB, bool DIP>
-__device__ void prim_vec(double a1, double a2, const double *A, const double *B,
+template <int LA, int LB, bool DIP, bool PAD = false>
+__device__ __forceinline__ void prim_vec(double a1, double a2, const double *A, const double *B,
                          const double *C, double *out, long long cstride) {
   const double zeta = a1 + a2, xi = a1 * a2 / zeta, inv2p = 1.0 / (2.0 * zeta);
   const bool left = a1 <= a2;
@@ -356,22 +381,7 @@ __device__ void prim_vec(double a1, double a2, const double *A, const double *B,
       }
       return v;
     };
-#pragma unroll
-    for (int s1 = 0; s1 < nsh(LA); ++s1)
-#pragma unroll
-      for (int s2 = 0; s2 < nsh(LB); ++s2) {
-        double v = 0.0;
-#pragma unroll
-        for (int k1 = 0; k1 < 3; ++k1) {
-          if (k1 >= sh_nterm(s1)) break;
-#pragma unroll
-          for (int k2 = 0; k2 < 3; ++k2) {
-            if (k2 >= sh_nterm(s2)) break;
-            v += sh_coef(s1, k1) * sh_coef(s2, k2) * cart(sh_cart(s1, k1), sh_cart(s2, k2));
-          }
-        }
-        out[c * cstride + s1 * nsh(LB) + s2] = v;
-      }
+    write_sh_block<LA, LB, PAD>(cart, out + c * cstride);
   }
 }
 
@@ -494,20 +504,6 @@ __host__ __device__ constexpr int cart_index(int x, int y, int z) {
   return t[9 * x + 3 * y + z];
 }
 
-// f(0), f(1), ... f(N - 1) with the index as a type, so that everything
-// derived from it is a constant and small arrays stay in registers.
-template <int I>
-struct Idx {
-  static constexpr int value = I;
-};
-template <int N, int I = 0, class F>
-__device__ __forceinline__ void static_for(F &&f) {
-  if constexpr (I < N) {
-    f(Idx<I>{});
-    static_for<N, I + 1>(f);
-  }
-}
-
 // One axis's Hermite coefficients E^{ij}_t for one i and every j <= LB:
 // E[j][t], t <= i + j.
 template <int I, int LB>
@@ -605,31 +601,6 @@ __device__ __forceinline__ void hermite_row(const double (&PA0)[3], const double
     row[m] = v;
   });
 }
-
-// A block's rows as they are finished: to `out`, or (PAD) to a build's
-// block buffer, where every block starts on 32 bytes and has blk_len
-// doubles: each thread writes its own block, so single 8-byte stores would
-// send one partial sector each (162-atom quartz EP: 2.0 G of them; whole
-// sectors are a quarter).
-template <int N, bool PAD>
-struct BlockWriter {
-  double *out;
-  double quad[4];
-  template <int R, int M>
-  __device__ __forceinline__ void row(const double (&v)[M]) {
-    static_for<M>([&](auto im) {
-      constexpr int m = decltype(im)::value, o = R * M + m;
-      if constexpr (!PAD) {
-        out[o] = v[m];
-      } else {
-        quad[o & 3] = v[m];
-        if constexpr (o == N - 1)
-          for (int i = (o & 3) + 1; i < 4; ++i) quad[i] = 0.0;
-        if constexpr (o == N - 1 || (o & 3) == 3) store4(out + (o & ~3), quad);
-      }
-    });
-  }
-};
 
 // Turn accumulated Hermite integrals Q into the sh block, one Cartesian row
 // of atom 1 at a time: a d-d block as a whole (100 Cartesian values beside
@@ -926,26 +897,30 @@ __device__ void prim_kov_t(double a1, double a2, const double *A, const double *
     fr[x] = mag * cs;
     fi[x] = -mag * sn;
   }
-  double pcr[ncart(LA) * ncart(LB)], pci[ncart(LA) * ncart(LB)];
+  // the phases into the tables, then a pass for each part
 #pragma unroll
-  for (int p = 0; p < ncart(LA); ++p)
+  for (int x = 0; x < 3; ++x)
 #pragma unroll
-    for (int c = 0; c < ncart(LB); ++c) {
-      double vr = 1.0, vi = 0.0;
+    for (int i = 0; i <= LA; ++i)
 #pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        const int i = cart_exp(p, x), j = cart_exp(c, x);
-        const double gr = Sr[x][i][j] * fr[x] - Si[x][i][j] * fi[x];
-        const double gi = Sr[x][i][j] * fi[x] + Si[x][i][j] * fr[x];
-        const double nr = vr * gr - vi * gi, ni = vr * gi + vi * gr;
-        vr = nr;
-        vi = ni;
+      for (int j = 0; j <= LB; ++j) {
+        const double r = Sr[x][i][j];
+        Sr[x][i][j] = r * fr[x] - Si[x][i][j] * fi[x];
+        Si[x][i][j] = r * fi[x] + Si[x][i][j] * fr[x];
       }
-      pcr[p * ncart(LB) + c] = vr;
-      pci[p * ncart(LB) + c] = vi;
+  auto part = [&](int p, int c, bool imag) {
+    double vr = 1.0, vi = 0.0;
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      const int i = cart_exp(p, x), j = cart_exp(c, x);
+      const double nr = vr * Sr[x][i][j] - vi * Si[x][i][j];
+      vi = vr * Si[x][i][j] + vi * Sr[x][i][j];
+      vr = nr;
     }
-  cart_to_sh<LA, LB>(pcr, out_re);
-  cart_to_sh<LA, LB>(pci, out_im);
+    return imag ? vi : vr;
+  };
+  write_sh_block<LA, LB, true>([&](int p, int c) { return part(p, c, false); }, out_re);
+  write_sh_block<LA, LB, true>([&](int p, int c) { return part(p, c, true); }, out_im);
 }
 
 
