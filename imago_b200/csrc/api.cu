@@ -1731,7 +1731,7 @@ int do_ep(imago_ctx *c, double *packed, int first = 0, int count = -1) {
 // spin), then the kinetic, mass-velocity (rel) and nuclear blocks added.
 // The contraction, phase sum and orthogonalisation are linear, so they then
 // run once per spin instead of once per term.  The potential terms are
-// summed in registers per shell pair (k_prim3c_ham, once per spin);
+// summed in registers per shell pair (k_prim3c_ham, both spins at once);
 // imago_intg_set_ham_mode selects the EP build's per-term blocks added with
 // their weights (k_block_axpy) instead.  Lanes per shell pair: Si8 (62k
 // shell pairs) 1.72 / 0.84 / 0.78 ms of primitives with 1 / 4 / 8 lanes
@@ -1754,22 +1754,37 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
   const int lanes = c->ham_mode == 3 ? 1 : (long long)c->sps.size() >= kHamWidePairs ? 4 : 8;
   const int chunk = fused ? 0 : ep_chunk_size(c);
   if (!fused && (rc = ensure_scratch(c, std::max(chunk, spin)))) return rc;
-  if (!fused)
-    IMAGO_CUDA(cudaMemsetAsync(c->ham_blk.p, 0, sizeof(double) * n * spin, st));
   if (c->pot_dim > 0)
     IMAGO_CUDA(cudaMemcpyAsync(c->ham_w.p, coeffs, sizeof(double) * c->pot_dim * spin,
                                cudaMemcpyHostToDevice, st));
   const int nchunk = fused || c->pot_dim == 0 ? 0 : (c->pot_dim + chunk - 1) / chunk;
-  c->launches += class_launches(c) * (2 + (rel ? 1 : 0) + (fused ? spin : nchunk)) +
-                 (2 + (rel ? 1 : 0) + nchunk) + 2 + (c->core_dim > 0 ? 2 : 1);
+  c->launches += class_launches(c) * (2 + (rel ? 1 : 0) + (fused ? 1 : nchunk)) + nchunk + 3 +
+                 (c->core_dim > 0 ? 2 : 1);
   mark(c);
+  // the kinetic, mass-velocity (written negatively, the sign the reference
+  // subtracts it with) and nuclear blocks, each added as it is stored, beside
+  // the potential terms on the kinetic lane
+  const int lane = c->lane;
+  c->lane = KIND_KE;
+  cudaStream_t bst = c->cur();
+  double *base = nullptr;
+  rc = cudaStreamWaitEvent(bst, c->kfork, 0) == cudaSuccess ? ensure_scratch(c, 1)
+                                                            : (int)IMAGO_ERR_CUDA;
+  if (!rc) {
+    base = c->scr[KIND_KE].blk.p;
+    rc = launch_prim2c(s, w, c->cls_beg, kPrim2cKinetic, base, bst);
+  }
+  if (!rc && rel) rc = launch_prim2c(s, w, c->cls_beg, kPrim2cMassVel, base, bst, true);
+  if (!rc) rc = launch_prim3c_nuc(s, w, c->cls_beg, base, bst, true);
+  if (cudaEventRecord(c->kjoin[KIND_KE], bst) != cudaSuccess && !rc) rc = IMAGO_ERR_CUDA;
+  c->lane = lane;
+  if (rc) return rc;
   if (fused) {
-    for (int h = 0; h < spin; ++h)
-      if ((rc = launch_prim3c_ham(s, w, c->cls_beg, c->d_terms.p, c->pot_dim,
-                                  c->ham_w.p + (size_t)h * c->pot_dim, lanes,
-                                  c->ham_blk.p + (size_t)h * n, st)))
-        return rc;
+    if ((rc = launch_prim3c_ham(s, w, c->cls_beg, c->d_terms.p, c->pot_dim, c->ham_w.p, spin, lanes,
+                                c->ham_blk.p, st)))
+      return rc;
   } else {
+    IMAGO_CUDA(cudaMemsetAsync(c->ham_blk.p, 0, sizeof(double) * n * spin, st));
     for (int t0 = 0; t0 < c->pot_dim; t0 += chunk) {
       const int nt = std::min(chunk, c->pot_dim - t0);
       if ((rc = launch_prim3c_terms(s, w, c->cls_beg, c->d_terms.p + t0,
@@ -1780,16 +1795,8 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
         return rc;
     }
   }
-  if ((rc = launch_prim2c(s, w, c->cls_beg, kPrim2cKinetic, S.blk.p, st))) return rc;
-  if ((rc = launch_block_axpy(S.blk.p, 1, n, nullptr, 0, spin, c->ham_blk.p, st))) return rc;
-  if (rel) {
-    // written negatively, the sign the reference subtracts it with
-    if ((rc = launch_prim2c(s, w, c->cls_beg, kPrim2cMassVel, S.blk.p, st))) return rc;
-    if ((rc = launch_block_axpy(S.blk.p, 1, n, nullptr, 0, spin, c->ham_blk.p, st)))
-      return rc;
-  }
-  if ((rc = launch_prim3c_nuc(s, w, c->cls_beg, S.blk.p, st))) return rc;
-  if ((rc = launch_block_axpy(S.blk.p, 1, n, nullptr, 0, spin, c->ham_blk.p, st))) return rc;
+  IMAGO_CUDA(cudaStreamWaitEvent(st, c->kjoin[KIND_KE], 0));
+  if ((rc = launch_block_axpy(base, 1, n, nullptr, 0, spin, c->ham_blk.p, st))) return rc;
   mark(c);
   if ((rc = launch_contract(s, w, spin, c->ham_blk.p, S.M.p, st))) return rc;
   mark(c);

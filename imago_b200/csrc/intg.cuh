@@ -145,12 +145,12 @@ cudaMemPool_t device_scratch_pool();
 
 // Launchers (kernels.cu).  All take the stream to run on.
 int launch_prim2c(const DevSys &s, const DevWork &w, const int *cls_beg,
-                  int op, double *blk, cudaStream_t st);
-// The PSCF Hamiltonian's potential terms for one spin, summed in registers
-// per shell pair: H = sum_t coef[t] EP_t (sh blocks, written, not added).
+                  int op, double *blk, cudaStream_t st, bool add = false);
+// The PSCF Hamiltonian's potential terms for one or two spins, summed in
+// registers per shell pair: H[h] = sum_t coef[h][t] EP_t (sh blocks).
 // lanes (1, 4 or 8) threads share a shell pair's images (s, p, d classes).
 int launch_prim3c_ham(const DevSys &s, const DevWork &w, const int *cls_beg,
-                      const Term3c *terms_dev, int nterm, const double *coef,
+                      const Term3c *terms_dev, int nterm, const double *coef, int spin,
                       int lanes, double *H, cudaStream_t st);
 // The three wave vectors of a K-overlap build, q[3 * axis + xyz].
 struct KovWaves {
@@ -220,14 +220,15 @@ int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
 // The f classes of the EP terms (terms_dev) or of the nuclear term.
 int launch_prim3c_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
                      const Term3c *terms_dev, int nterm, bool nuclear, double *blk,
-                     cudaStream_t st);
+                     cudaStream_t st, bool add = false);
 // The f classes of launch_prim3c_ham.
 int launch_prim3c_ham_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
-                         const Term3c *terms_dev, int nterm, const double *coef, double *H,
-                         cudaStream_t st);
-// The nuclear term (all potential types), several lanes per shell pair.
+                         const Term3c *terms_dev, int nterm, const double *coef, int spin,
+                         double *H, cudaStream_t st);
+// The nuclear term (all potential types), several lanes per shell pair;
+// add: onto blk's blocks, as launch_prim2c's mass velocity.
 int launch_prim3c_nuc(const DevSys &s, const DevWork &w, const int *cls_beg, double *blk,
-                      cudaStream_t st);
+                      cudaStream_t st, bool add = false);
 // terms_per_cta: 4 or 8 EP terms per CTA (builds of up to 4 terms use 4)
 int launch_contract(const DevSys &s, const DevWork &w, int nterm,
                     const double *blk, double *M, cudaStream_t st, int terms_per_cta = 4);

@@ -14,7 +14,7 @@ namespace imago {
 // (0.7 of the 0.75 ms of the two-atom diamond cell's nuclear term).
 template <int LA, int LB, int T>
 __global__ void __launch_bounds__(128, LA + LB >= 4 ? 3 : 4)
-    k_prim3c_nuc(DevSys s, DevWork w, int beg, int n, double *blk) {
+    k_prim3c_nuc(DevSys s, DevWork w, int beg, int n, double *blk, bool add) {
   constexpr int L = LA + LB;
   static_assert(32 % T == 0, "a shell pair's lanes stay in one warp");
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -53,7 +53,8 @@ __global__ void __launch_bounds__(128, LA + LB >= 4 ? 3 : 4)
   }
   team_sum<L, T>(Q);
   if (live && sub == 0)
-    hermite_to_sh<LA, LB, true>(q.A, q.B, q.a1, q.a2, exp(-c.xi * q.r2), Q, blk + sp.boff);
+    hermite_to_sh<LA, LB, true>(q.A, q.B, q.a1, q.a2, exp(-c.xi * q.r2), Q, blk + sp.boff,
+                                add ? blk + sp.boff : nullptr);
 }
 
 // Lanes per shell pair: enough threads to fill the GPU, no more, since each
@@ -67,29 +68,29 @@ constexpr long long kNucThreadsWanted = 320000;
 
 template <int LA, int LB>
 static int nuc_one(const DevSys &s, const DevWork &w, int beg, int n, int lanes, double *blk,
-                   cudaStream_t st) {
+                   cudaStream_t st, bool add) {
   if (n <= 0) return IMAGO_OK;
   const unsigned grid = (unsigned)(((long long)n * lanes + 127) / 128);
   switch (lanes) {
-    case 8: k_prim3c_nuc<LA, LB, 8><<<grid, 128, 0, st>>>(s, w, beg, n, blk); break;
-    case 4: k_prim3c_nuc<LA, LB, 4><<<grid, 128, 0, st>>>(s, w, beg, n, blk); break;
-    case 2: k_prim3c_nuc<LA, LB, 2><<<grid, 128, 0, st>>>(s, w, beg, n, blk); break;
-    default: k_prim3c_nuc<LA, LB, 1><<<grid, 128, 0, st>>>(s, w, beg, n, blk);
+    case 8: k_prim3c_nuc<LA, LB, 8><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
+    case 4: k_prim3c_nuc<LA, LB, 4><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
+    case 2: k_prim3c_nuc<LA, LB, 2><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
+    default: k_prim3c_nuc<LA, LB, 1><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add);
   }
   IMAGO_CUDA(cudaGetLastError());
   return IMAGO_OK;
 }
 
 int launch_prim3c_nuc(const DevSys &s, const DevWork &w, const int *cls_beg, double *blk,
-                      cudaStream_t st) {
+                      cudaStream_t st, bool add) {
   int lanes = 1, rc = IMAGO_OK;
   while (lanes < 8 && 2LL * lanes * w.nsp <= kNucThreadsWanted) lanes *= 2;
 #define IMAGO_PN(a, b) \
   if (!rc) rc = nuc_one<a, b>(s, w, cls_beg[a * 4 + b], \
-                              cls_beg[a * 4 + b + 1] - cls_beg[a * 4 + b], lanes, blk, st);
+                              cls_beg[a * 4 + b + 1] - cls_beg[a * 4 + b], lanes, blk, st, add);
   IMAGO_FOR_SPD_CLASSES(IMAGO_PN)
 #undef IMAGO_PN
-  return rc ? rc : launch_prim3c_rt(s, w, cls_beg, nullptr, 1, true, blk, st);
+  return rc ? rc : launch_prim3c_rt(s, w, cls_beg, nullptr, 1, true, blk, st, add);
 }
 
 }  // namespace imago

@@ -24,22 +24,24 @@ __global__ void __launch_bounds__(128)
 // the f classes through one runtime-class kernel.
 template <int LA, int LB>
 __global__ void __launch_bounds__(128)
-    k_prim_mv(DevSys s, DevWork w, int beg, int end, double *blk) {
+    k_prim_mv(DevSys s, DevWork w, int beg, int end, double *blk, bool add) {
   const int g = beg + blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= end) return;
   const DSp sp = w.sps[w.sp_by_cls[g]];
   const SpGeom q = sp_geom(s, w, sp);
-  prim_mv<LA, LB, true>(q.a1, q.a2, q.A, q.B, -kMassVelPref, blk + sp.boff);
+  prim_mv<LA, LB, true>(q.a1, q.a2, q.A, q.B, -kMassVelPref, blk + sp.boff,
+                        add ? blk + sp.boff : nullptr);
 }
 
 __global__ void __launch_bounds__(128)
     k_prim_mv_rt(DevSys s, DevWork w, int beg, int end, int la, int lb,
-                 double *blk) {
+                 double *blk, bool add) {
   const int g = beg + blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= end) return;
   const DSp sp = w.sps[w.sp_by_cls[g]];
   const SpGeom q = sp_geom(s, w, sp);
-  prim_mv_rt(la, lb, q.a1, q.a2, q.A, q.B, -kMassVelPref, blk + sp.boff);
+  prim_mv_rt(la, lb, q.a1, q.a2, q.A, q.B, -kMassVelPref, blk + sp.boff,
+             add ? blk + sp.boff : nullptr);
 }
 
 // Momentum / dipole: three component blocks per shell pair, component c at
@@ -199,7 +201,7 @@ __global__ void __launch_bounds__(128)
 template <bool NUC>
 __device__ __noinline__ void prim3c_item_rt(const DevSys &s, const DevWork &w, int beg,
                                             int n, const Term3c *terms, int la, int lb,
-                                            double *blk, long long g) {
+                                            double *blk, long long g, bool add) {
   const int L = la + lb;
   const int tl = (int)(g / n);
   const DSp sp = w.sps[w.sp_by_cls[beg + (int)(g % n)]];
@@ -235,17 +237,17 @@ __device__ __noinline__ void prim3c_item_rt(const DevSys &s, const DevWork &w, i
   }
   const double ex = exp(-c.xi * q.r2);
   const double pref = NUC ? ex : pow(kPi / (c.zeta + a3e), 1.5) * ex;
-  hermite_to_sh_rt(la, lb, q.A, q.B, q.a1, q.a2, pref, Q,
-                   blk + (long long)tl * w.blk_total + sp.boff);
+  double *out = blk + (long long)tl * w.blk_total + sp.boff;
+  hermite_to_sh_rt(la, lb, q.A, q.B, q.a1, q.a2, pref, Q, out, add ? out : nullptr);
 }
 
 template <bool NUC>
 __global__ void __launch_bounds__(128)
     k_prim3c_rt(DevSys s, DevWork w, int beg, int n, const Term3c *terms,
-                int nterm, int la, int lb, double *blk) {
+                int nterm, int la, int lb, double *blk, bool add) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (long long)n * nterm) return;
-  prim3c_item_rt<NUC>(s, w, beg, n, terms, la, lb, blk, g);
+  prim3c_item_rt<NUC>(s, w, beg, n, terms, la, lb, blk, g, add);
 }
 
 // ------------------------------------------------------- work queue --
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(128, 3)
       IMAGO_QC(1, 2) IMAGO_QC(2, 0) IMAGO_QC(2, 1) IMAGO_QC(2, 2)
 #undef IMAGO_QC
       default:
-        prim3c_item_rt<false>(s, w, beg, n, terms, qc.cls[c] / 4, qc.cls[c] % 4, blk, g);
+        prim3c_item_rt<false>(s, w, beg, n, terms, qc.cls[c] / 4, qc.cls[c] % 4, blk, g, false);
     }
   }
 }
@@ -331,14 +333,15 @@ int launch_prim3c_count(const DevSys &s, const DevWork &w, const int *cls_beg,
 }
 
 int launch_prim2c(const DevSys &s, const DevWork &w, const int *cls_beg,
-                  int op, double *blk, cudaStream_t st) {
+                  int op, double *blk, cudaStream_t st, bool add) {
   int rc = IMAGO_OK;
+  if (add && op != kPrim2cMassVel) return IMAGO_ERR_INVALID;
   if (op == kPrim2cMassVel) {
 #define IMAGO_MV(a, b)                                                        \
   {                                                                          \
     const int beg = cls_beg[a * 4 + b], n = cls_beg[a * 4 + b + 1] - beg;    \
     if (n > 0) {                                                             \
-      k_prim_mv<a, b><<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, beg + n, blk); \
+      k_prim_mv<a, b><<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, beg + n, blk, add); \
       IMAGO_CUDA(cudaGetLastError());                                        \
     }                                                                        \
   }
@@ -349,7 +352,7 @@ int launch_prim2c(const DevSys &s, const DevWork &w, const int *cls_beg,
       if (la < 3 && lb < 3) continue;
       const int beg = cls_beg[c], n = cls_beg[c + 1] - beg;
       if (n <= 0) continue;
-      k_prim_mv_rt<<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, beg + n, la, lb, blk);
+      k_prim_mv_rt<<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, beg + n, la, lb, blk, add);
       IMAGO_CUDA(cudaGetLastError());
     }
     return IMAGO_OK;
@@ -410,16 +413,19 @@ int launch_prim2c_vec(const DevSys &s, const DevWork &w, const int *cls_beg,
 }
 
 int launch_prim3c_ham_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
-                         const Term3c *terms_dev, int nterm, const double *coef, double *H,
-                         cudaStream_t st) {
+                         const Term3c *terms_dev, int nterm, const double *coef, int spin,
+                         double *H, cudaStream_t st) {
   for (int c = 0; c < 16; ++c) {
     const int la = c / 4, lb = c % 4;
     if (la < 3 && lb < 3) continue;
     const int beg = cls_beg[c], n = cls_beg[c + 1] - beg;
     if (n <= 0) continue;
-    k_prim3c_ham_rt<<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm,
-                                                     coef, la, lb, H);
-    IMAGO_CUDA(cudaGetLastError());
+    for (int h = 0; h < spin; ++h) {
+      k_prim3c_ham_rt<<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm,
+                                                       coef + (size_t)h * nterm, la, lb,
+                                                       H + h * w.blk_total);
+      IMAGO_CUDA(cudaGetLastError());
+    }
   }
   return IMAGO_OK;
 }
@@ -537,7 +543,7 @@ int launch_prim3c(const DevSys &s, const DevWork &w, const int *cls_beg,
 
 int launch_prim3c_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
                      const Term3c *terms_dev, int nterm, bool nuclear, double *blk,
-                     cudaStream_t st) {
+                     cudaStream_t st, bool add) {
   for (int c = 0; c < 16; ++c) {
     const int la = c / 4, lb = c % 4;
     if (la < 3 && lb < 3) continue;
@@ -545,9 +551,10 @@ int launch_prim3c_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
     if (n <= 0 || nterm <= 0) continue;
     const unsigned grid = (unsigned)(((long long)n * nterm + 127) / 128);
     if (nuclear)
-      k_prim3c_rt<true><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, la, lb, blk);
+      k_prim3c_rt<true><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, la, lb, blk, add);
     else
-      k_prim3c_rt<false><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, la, lb, blk);
+      k_prim3c_rt<false><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, la, lb, blk,
+                                               false);
     IMAGO_CUDA(cudaGetLastError());
   }
   return IMAGO_OK;

@@ -111,6 +111,17 @@ __device__ __forceinline__ void os1d(double PA, double PB, double inv2p,
     }
 }
 
+// v += four doubles from 32-byte aligned p.
+__device__ __forceinline__ void add4(const double *p, double v[4]) {
+  double x[4];
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3])
+               : "l"(p)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] += x[i];
+}
+
 // f(0), f(1), ... f(N - 1) with the index as a type, so that everything
 // derived from it is a constant and small arrays stay in registers.
 template <int I>
@@ -138,10 +149,11 @@ __device__ __forceinline__ void store4(double *p, const double v[4]) {
 // send one partial sector each (162-atom quartz EP: 2.0 G of them; whole
 // sectors are a quarter; overlap and kinetic blocks of that cell 0.43 and
 // 0.33 ms with 8-byte stores and the Cartesian block in local memory, 0.11
-// and 0.12 so).
+// and 0.12 so).  With `base`, base's block is added (base may be out).
 template <int N, bool PAD>
 struct BlockWriter {
   double *out;
+  const double *base;
   double quad[4];
   template <int R, int M>
   __device__ __forceinline__ void row(const double (&v)[M]) {
@@ -153,7 +165,10 @@ struct BlockWriter {
         quad[o & 3] = v[m];
         if constexpr (o == N - 1)
           for (int i = (o & 3) + 1; i < 4; ++i) quad[i] = 0.0;
-        if constexpr (o == N - 1 || (o & 3) == 3) store4(out + (o & ~3), quad);
+        if constexpr (o == N - 1 || (o & 3) == 3) {
+          if (base) add4(base + (o & ~3), quad);
+          store4(out + (o & ~3), quad);
+        }
       }
     });
   }
@@ -162,8 +177,9 @@ struct BlockWriter {
 // A block from its Cartesian products cart(p, q), each formed where a
 // harmonic needs it.
 template <int LA, int LB, bool PAD, class F>
-__device__ __forceinline__ void write_sh_block(F &&cart, double *out) {
-  BlockWriter<nsh(LA) * nsh(LB), PAD> w{out, {}};
+__device__ __forceinline__ void write_sh_block(F &&cart, double *out,
+                                               const double *base = nullptr) {
+  BlockWriter<nsh(LA) * nsh(LB), PAD> w{out, base, {}};
   static_for<nsh(LA)>([&](auto i1) {
     constexpr int s1 = decltype(i1)::value;
     double row[nsh(LB)];
@@ -288,7 +304,8 @@ __device__ __forceinline__ double d2_both(const double S[IA + 1][JB + 1],
 // of order a1 a2 when a1 << a2.  s, p and d classes only (registers).
 template <int LA, int LB, bool PAD = false>
 __device__ __forceinline__ void prim_mv(double a1, double a2, const double *A, const double *B,
-                        double scale, double *out) {
+                                        double scale, double *out,
+                                        const double *base = nullptr) {
   const double zeta = a1 + a2, xi = a1 * a2 / zeta, inv2p = 1.0 / (2.0 * zeta);
   // per axis: S, L (left d^2), R (right d^2), U (both) for i <= LA, j <= LB;
   // the extended overlap table lives only while its axis is formed
@@ -324,7 +341,7 @@ __device__ __forceinline__ void prim_mv(double a1, double a2, const double *A, c
     v += (l0 * r1 + r0 * l1) * s2 + (l0 * r2 + r0 * l2) * s1 + (l1 * r2 + r1 * l2) * s0;
     return pref * v;
   };
-  write_sh_block<LA, LB, PAD>(cart, out);
+  write_sh_block<LA, LB, PAD>(cart, out, base);
 }
 
 // Momentum <a|d/dx_c|b> (DIP = false) or dipole <a|(r - C)_c|b> (DIP =
@@ -611,11 +628,12 @@ __device__ __forceinline__ void hermite_row(const double (&PA0)[3], const double
 template <int LA, int LB, bool PAD = false>
 __device__ __forceinline__ void hermite_to_sh(const double (&PA)[3], const double (&PB)[3],
                                               double inv2p, double pref,
-                                              const double Q[nherm(LA + LB)], double *out) {
+                                              const double Q[nherm(LA + LB)], double *out,
+                                              const double *base = nullptr) {
   double H[nherm(LA + LB)];
 #pragma unroll
   for (int i = 0; i < nherm(LA + LB); ++i) H[i] = pref * Q[i];
-  BlockWriter<nsh(LA) * nsh(LB), PAD> w{out, {}};
+  BlockWriter<nsh(LA) * nsh(LB), PAD> w{out, base, {}};
   double row[nsh(LB)];
   hermite_row<LA, LB, 0>(PA, PB, inv2p, H, row);
   w.template row<0>(row);
@@ -656,7 +674,8 @@ __device__ __forceinline__ void hermite_to_sh(const double (&PA)[3], const doubl
 template <int LA, int LB, bool PAD = false>
 __device__ __forceinline__ void hermite_to_sh(const double *A, const double *B, double a1,
                                               double a2, double pref,
-                                              const double Q[nherm(LA + LB)], double *out) {
+                                              const double Q[nherm(LA + LB)], double *out,
+                                              const double *base = nullptr) {
   const double zeta = a1 + a2;
   double PA[3], PB[3];
 #pragma unroll
@@ -665,7 +684,7 @@ __device__ __forceinline__ void hermite_to_sh(const double *A, const double *B, 
     PA[x] = P - A[x];
     PB[x] = P - B[x];
   }
-  hermite_to_sh<LA, LB, PAD>(PA, PB, 1.0 / (2.0 * zeta), pref, Q, out);
+  hermite_to_sh<LA, LB, PAD>(PA, PB, 1.0 / (2.0 * zeta), pref, Q, out, base);
 }
 
 // ------------------------------------------------ f classes, runtime loops --
@@ -676,7 +695,7 @@ constexpr int kMaxL = 6;
 constexpr int kMaxHerm = nherm(kMaxL);  // 84
 
 static __device__ __forceinline__ void cart_to_sh_rt(int la, int lb, const double *pc,
-                                              double *out) {
+                                              double *out, const double *base = nullptr) {
   const int ncb = ncart(lb), nsa = nsh(la), nsb = nsh(lb);
 #pragma unroll 1
   for (int s1 = 0; s1 < nsa; ++s1)
@@ -687,7 +706,7 @@ static __device__ __forceinline__ void cart_to_sh_rt(int la, int lb, const doubl
         for (int k2 = 0; k2 < sh_nterm(s2); ++k2)
           v += sh_coef(s1, k1) * sh_coef(s2, k2) *
                pc[sh_cart(s1, k1) * ncb + sh_cart(s2, k2)];
-      out[s1 * nsb + s2] = v;
+      out[s1 * nsb + s2] = base ? v + base[s1 * nsb + s2] : v;
     }
 }
 
@@ -756,7 +775,7 @@ static __device__ __noinline__ void prim2c_rt(int la, int lb, bool kin, double a
 static __device__ __noinline__ void prim_mv_rt(int la, int lb, double a1,
                                                double a2, const double *A,
                                                const double *B, double scale,
-                                               double *out) {
+                                               double *out, const double *base = nullptr) {
   const double zeta = a1 + a2, xi = a1 * a2 / zeta, inv2p = 1.0 / (2.0 * zeta);
   double t[4][3][4][4];
   double d2 = 0.0;
@@ -797,7 +816,7 @@ static __device__ __noinline__ void prim_mv_rt(int la, int lb, double a1,
            (l[1] * r[2] + r[1] * l[2]) * s[0];
       pc[p * ncb + q] = pref * v;
     }
-  cart_to_sh_rt(la, lb, pc, out);
+  cart_to_sh_rt(la, lb, pc, out, base);
 }
 
 // prim_vec for the f classes: runtime loops, tables in local memory.
@@ -1061,7 +1080,8 @@ static __device__ __noinline__ void accumulate_nuclear_q_rt(int L, const double 
 static __device__ __noinline__ void hermite_to_sh_rt(int la, int lb, const double *A,
                                               const double *B, double a1,
                                               double a2, double pref,
-                                              const double *Q, double *out) {
+                                              const double *Q, double *out,
+                                              const double *base = nullptr) {
   const int L = la + lb;
   const double zeta = a1 + a2, inv2p = 1.0 / (2.0 * zeta);
   double E[3][4][4][kMaxL + 1];
@@ -1101,7 +1121,7 @@ static __device__ __noinline__ void hermite_to_sh_rt(int la, int lb, const doubl
         }
       pc[p * ncb + q] = pref * s;
     }
-  cart_to_sh_rt(la, lb, pc, out);
+  cart_to_sh_rt(la, lb, pc, out, base);
 }
 
 }  // namespace imago
