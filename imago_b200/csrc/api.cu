@@ -737,11 +737,13 @@ void build_pairs(const imago_ctx *c, const std::vector<int2> &ij, size_t lo,
 }
 
 // Runs f(lo, hi) over [0, n) in chunks on up to hardware_concurrency
-// threads (one thread for small n).
+// threads (one thread where `work`, in steps of tens of nanoseconds, would
+// not pay for starting them).
 template <class F>
-void parallel_ranges(size_t n, size_t nchunk, F f) {
-  const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  if (n < 512 || hw == 1) {
+void parallel_ranges(size_t n, size_t nchunk, size_t work, F f) {
+  const unsigned hw = (unsigned)std::max<size_t>(
+      1, std::min<size_t>({16, nchunk, std::thread::hardware_concurrency()}));
+  if (work < 30000 || hw == 1) {
     for (size_t c = 0; c < nchunk; ++c) f(c, n * c / nchunk, n * (c + 1) / nchunk);
     return;
   }
@@ -764,9 +766,12 @@ int build_work(imago_ctx *c) {
   ij.reserve((size_t)c->ns * (c->ns + 1) / 2);
   for (int i = 0; i < c->ns; ++i)
     for (int j = i; j < c->ns; ++j) ij.push_back(make_int2(i, j));
-  const size_t nchunk = std::max<size_t>(1, std::min<size_t>(256, ij.size() / 8));
+  // a pair of a small cell has hundreds of images and thousands of shell
+  // pairs: chunks of single pairs there (16-atom diamond cell, 136 pairs:
+  // staging 6.0 -> 3.75 ms)
+  const size_t nchunk = std::max<size_t>(1, std::min<size_t>(256, ij.size()));
   std::vector<PairWork> part(nchunk);
-  parallel_ranges(ij.size(), nchunk, [&](size_t k, size_t lo, size_t hi) {
+  parallel_ranges(ij.size(), nchunk, ij.size() * c->ncell, [&](size_t k, size_t lo, size_t hi) {
     build_pairs(c, ij, lo, hi, part[k]);
   });
   // offsets of each part in the merged arrays, then the parts copied (and
@@ -807,7 +812,7 @@ int build_work(imago_ctx *c) {
       }
   }
   c->sp_by_cls.resize(sb[nparts]);
-  parallel_ranges(sb[nparts], nparts, [&](size_t k, size_t, size_t) {
+  parallel_ranges(sb[nparts], nparts, sb[nparts], [&](size_t k, size_t, size_t) {
     const PairWork &w = part[k];
     for (size_t q = 0; q < w.pairs.size(); ++q) {
       DPair p = w.pairs[q];
