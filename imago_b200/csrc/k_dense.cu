@@ -161,6 +161,10 @@ __device__ __forceinline__ void scatter_full(const DevSys &s, const DPair &p,
 // 2 x BC/16 warps, each a 16 k x 16 column tile.  Rows of m_s are BC + 4
 // doubles and rows of ph_s 34 complex values, both 8 mod 32 bank words, so
 // the 4 k rows of a fragment read fall on distinct banks in each wavefront.
+// The MMAs bound it (Si8: 0.63 of 1.0 ms, padding included): a warp without
+// a k-point or a column leaves the tensor cores to the SM's others (Si16, 14
+// computed k-points, EP: 0.31 -> 0.25 ms).  Leaving out single fragments too
+// costs the full tiles registers: Si8 1.01 -> 1.03.
 constexpr int kBKP = kBK + 2;
 
 // KOV: the plane-wave overlap's complex blocks, the real and imaginary
@@ -190,6 +194,7 @@ __global__ void __launch_bounds__(4 * BC, (KOV ? 128 : 256) / BC)
   const int nu = p.uend - p.ubeg;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wk = (warp / NWC) * 16, wc = (warp % NWC) * 16;  // warp tile origin
+  const bool on = k0 + wk < nk && c0 + wc < ne;
   constexpr int NP = KOV ? 2 : 1;
   const double *Mt = nullptr;
   double ar[NP][2][2][2] = {}, ai[NP][2][2][2] = {};
@@ -226,23 +231,25 @@ __global__ void __launch_bounds__(4 * BC, (KOV ? 128 : 256) / BC)
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
+    if (on) {
 #pragma unroll
-    for (int ks = 0; ks < kBU; ks += 4) {
-      const int ku = ks + (lane & 3);
-      double b[2];
-      double2 a[2];
+      for (int ks = 0; ks < kBU; ks += 4) {
+        const int ku = ks + (lane & 3);
+        double b[2];
+        double2 a[2];
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        b[t] = m_s[buf][ku][wc + t * 8 + (lane >> 2)];
-        a[t] = ph_s[buf][ku][wk + t * 8 + (lane >> 2)];
-      }
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          dmma(ar[part][mt][nt][0], ar[part][mt][nt][1], a[mt].x, b[nt]);
-          dmma(ai[part][mt][nt][0], ai[part][mt][nt][1], a[mt].y, b[nt]);
+        for (int t = 0; t < 2; ++t) {
+          b[t] = m_s[buf][ku][wc + t * 8 + (lane >> 2)];
+          a[t] = ph_s[buf][ku][wk + t * 8 + (lane >> 2)];
         }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            dmma(ar[part][mt][nt][0], ar[part][mt][nt][1], a[mt].x, b[nt]);
+            dmma(ai[part][mt][nt][0], ai[part][mt][nt][1], a[mt].y, b[nt]);
+          }
+      }
     }
     __syncthreads();  // this stage's buffer is refilled two stages on
   }
