@@ -147,25 +147,33 @@ class ClockSampler:
 
 
 # ------------------------------------------------------------ algorithmic --
-def algorithmic_flops(g):
-    """Per-build FLOPs of the dense stages, from the screened work counts:
+def computed_kpoints(system):
+    """K-points whose matrices a build forms: one of each k and -k (modulo a
+    reciprocal vector), whose matrices are each other's conjugates."""
+    k = np.mod(np.round(np.asarray(system.kpoints_abc) * 2**20), 2**20).astype(np.int64)
+    return len({min(tuple(q), tuple(np.mod(-q, 2**20))) for q in k})
+
+
+def algorithmic_flops(g, nk):
+    """Per-build FLOPs of the dense stages over `nk` computed k-points, from
+    the screened work counts:
     lattice-to-k sum: 4 flops per (k, unit block element), per matrix;
     orthogonalisation: Y = X_cv - X_cc S/2 (8 C^2 V per k) and the packed
     update S^H Y + Y^H S (16 C per packed element per k), per matrix."""
     nmat = 3 + g.pot_dim
-    V, C, nk = g.vale_dim, g.core_dim, g.nk
+    V, C = g.vale_dim, g.core_dim
     m_elems = g.block_elements
     bloch = 4.0 * nk * m_elems * nmat
     ortho = nk * (8.0 * C * C * V + 16.0 * C * g.npacked) * nmat
     return {"bloch": bloch, "ortho": ortho}
 
 
-# DRAM bytes (read + write) per (k-point, matrix) of the fused
-# orthogonalisation, from one ncu capture of its Si8 4x4x4 EP launch: 243.66 MB
-# read and 83.76 MB written for 64 k x 20 terms.  The kernel's traffic grows
-# in proportion to the (k, matrix) pairs, so the build's figure is this times
-# nk x (3 + potDim).
-ORTHO_FUSED_BYTES_PER_KMAT = (243.658496e6 + 83.760128e6) / 1280
+# DRAM bytes (read + write) per (computed k-point, matrix) of the fused
+# orthogonalisation, from one ncu capture of its Si8 4x4x4 EP launch: 121.32 MB
+# read and 66.15 MB written for 32 computed k x 20 terms.  The kernel's traffic
+# grows in proportion to the (k, matrix) pairs, so the build's figure is this
+# times computed k x (3 + potDim).
+ORTHO_FUSED_BYTES_PER_KMAT = (121.320960e6 + 66.147584e6) / 640
 
 
 def fp64_peak_tflops(torch):
@@ -986,7 +994,7 @@ def run_ours(args):
         adjacent = adjacent_builds(g, bufs, stream, torch, dev, ham_mode=args.ham_mode)
     e2e = time_e2e(system, local, stream, bufs, 5, torch)
 
-    flops = algorithmic_flops(g)
+    flops = algorithmic_flops(g, computed_kpoints(system))
     fp64 = fp64_peak_tflops(torch) if rank == 0 else None
     prim3c = prim3c_roofline(g, bufs, stream, flush, torch, fp64) if rank == 0 else None
     top = int(np.argmax(kms))
@@ -996,7 +1004,7 @@ def run_ours(args):
         achieved = flops[top_name] / (kms[top] / 1e3) / 1e12
         traffic = None
         if top_name == "ortho" and args.workload == "si8":
-            traffic = ORTHO_FUSED_BYTES_PER_KMAT * nk * (3 + P)
+            traffic = ORTHO_FUSED_BYTES_PER_KMAT * computed_kpoints(system) * (3 + P)
         roofline = {"bound": "tensor", "achieved": achieved, "peak": fp64,
                     "unit": "TFLOP/s", "frac": achieved / fp64, "traffic": traffic,
                     "traffic_unit": "bytes per build (ncu, scaled by (k, matrix) pairs)",

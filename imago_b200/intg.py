@@ -361,7 +361,8 @@ class IntegralSetup:
         (imago_intg_set_schedule): "auto" (all measured on the first EP
         build, the fastest kept), "per_class" (one launch per class),
         "queue" (one persistent launch fed by a device work queue) or
-        "pairs" (one launch per class, two EP terms of a type per thread)."""
+        "pairs" (a thread takes several EP terms of a type in one walk over
+        the images; all classes in one launch on small systems)."""
         m = {"auto": -1, "per_class": 0, "queue": 1, "pairs": 2}[mode]
         _check(lib().imago_intg_set_schedule(self._ctx, m), "imago_intg_set_schedule")
 
@@ -414,8 +415,8 @@ class IntegralSetup:
     def set_ham_mode(self, mode):
         """How ham_pscf sums the potential terms (imago_intg_set_ham_mode):
         "auto", "blocks" (per-term blocks added with their weights),
-        "fused" (all terms of a shell pair in registers, a pass per spin,
-        four lanes per shell pair on small systems) or "fused1" (one lane)."""
+        "fused" (all terms of a shell pair and both spins in registers, four
+        or eight lanes per shell pair) or "fused1" (one lane)."""
         m = {"auto": 0, "blocks": 1, "fused": 2, "fused1": 3}[mode]
         _check(lib().imago_intg_set_ham_mode(self._ctx, m), "imago_intg_set_ham_mode")
 

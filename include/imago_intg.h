@@ -278,10 +278,10 @@ IMAGO_API int imago_ham_pscf(imago_ctx *ctx, int spin, const double *coeffs, int
                              double *packed);
 
 /* How imago_ham_pscf sums the potential terms (no counterpart in the
- * reference): 0 chooses by spin count and system size, 1 builds each
+ * reference): 0 (the default) is 2, 1 builds each
  * term's primitive blocks and adds them with their weights, 2 sums all
- * terms of a shell pair in registers (one pass per spin; several lanes per
- * shell pair on small systems), 3 as 2 with one lane per shell pair.  The
+ * terms of a shell pair in registers (both spins in one pass; four or
+ * eight lanes per shell pair), 3 as 2 with one lane per shell pair.  The
  * results agree to rounding; the choice is a matter of speed. */
 IMAGO_API int imago_intg_set_ham_mode(imago_ctx *ctx, int mode);
 
@@ -477,13 +477,12 @@ IMAGO_API int imago_packed_density(int n, int num_kpoints, int ld_states, int nu
  * classes in one persistent launch whose warps take 32 items at a time
  * from a device work queue (one atomic counter), the classes ordered by
  * cost so that the cheap ones fill in behind the expensive ones; mode 2:
- * one launch per class with two EP terms of a potential type per thread
- * for the classes up to d-p (k_prim3c_pair), which walk the sites and
- * images once for both; mode -1 (the default): all run once on the
- * context's first EP build and the fastest is kept.  NP is the same bit for
- * bit under every mode, EP the same to rounding (mode 2 may enumerate an
- * item's images from another lattice vector).  A captured graph of the
- * context is dropped. */
+ * a thread takes several EP terms of a potential type in one walk over the
+ * images (k_prim3c_terms: a launch per class, or all classes in one launch
+ * on small systems); mode -1 (the default): all run once on the context's
+ * first EP build and the fastest is kept.  NP has one kernel of its own and
+ * is the same bit for bit under every mode, EP the same to rounding.  A
+ * captured graph of the context is dropped. */
 IMAGO_API int imago_intg_set_schedule(imago_ctx *ctx, int mode);
 /* The schedule in use (0, 1 or 2) and the trial times of the measurement
  * (ms, in mode order; zero when not measured). */
