@@ -15,9 +15,9 @@ namespace imago {
 // distance from M, less the margin that bounds the float error, is within
 // that reach.  Images come in chunks of 32 neighbours, most of which their
 // bounding spheres rule out (162-atom quartz: staging 17.5 ms with every
-// image tested, 12.0 without lists).  Entries are placed in kListBins steps of the reach, in table
-// order inside a step, and carry the lower edge of their step: a walk may
-// stop at the first entry whose edge is beyond its own reach.  The list
+// image tested, 12.0 without lists).  Entries are placed in kListBins steps of
+// the reach and carry the lower edge of their step: a walk may stop at the
+// first entry whose edge is beyond its own reach.  The list
 // replaces a nearest-image search per (shell pair, term, site) and the loop
 // over lattice cells behind it (the walk alone was 15 of the 35 ms of the
 // 162-atom quartz EP primitives).
@@ -111,58 +111,78 @@ __global__ void __launch_bounds__(32 * kListWarps)
   }
 }
 
-__global__ void __launch_bounds__(32 * kListWarps)
+// Lane-private counters per step (row b, column lane, a column over for the
+// step's first entry): counting and placing need neither atomics nor a match
+// across the warp, whose latency bound the form with both (64-atom graphite
+// 0.93 ms, short scoreboard; staging 6.43 -> 6.10 ms, 162-atom quartz 14.6 ->
+// 13.8), and the order of a list is always the same: by step, lane, chunk.
+constexpr int kFillWarps = 4, kFillRow = 33;
+
+__global__ void __launch_bounds__(32 * kFillWarps)
     k_list_fill(DevSys s, DevWork w, float margin, const float *rad, ImageRef *list) {
-  __shared__ int bins[kListWarps][kListBins];
+  __shared__ int bins[kFillWarps][kListBins * kFillRow];
+  static_assert(kListBins == 64, "two steps per lane");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = gridDim.x * kListWarps;
+  const int nw = gridDim.x * kFillWarps;
   int *bin = bins[warp];
-  for (int ui = blockIdx.x * kListWarps + warp; ui < w.nunits; ui += nw) {
+  for (int ui = blockIdx.x * kFillWarps + warp; ui < w.nunits; ui += nw) {
     const DUnit u = w.units[ui];
     const float3 m = unit_mid(s, w, u);
     const float R = rad[ui], step = R / kListBins, inv = kListBins / R;
     const float lim = R + margin, lim2 = lim * lim;
     for (int pt = 0; pt < s.npt; ++pt) {
+      const int2 range = w.uoff[(long long)ui * s.npt + pt];
+      if (range.x == range.y) continue;
       const int i1 = w.img_off[pt + 1];
-      // the step of an image: its distance less the margin
-      auto place = [&](int i, int &b) {
+      // the step of an image, its distance less the margin; -1 outside
+      auto place = [&](int i) {
         const float d2 = i < i1 ? list_d2(w.ftab[i], m) : 0.f;
-        const bool in = i < i1 && d2 <= lim2;
-        b = in ? min(kListBins - 1, (int)(fmaxf(0.f, sqrtf(d2) - margin) * inv)) : -1 - lane;
-        return in;
+        return i < i1 && d2 <= lim2
+                   ? min(kListBins - 1, (int)(fmaxf(0.f, sqrtf(d2) - margin) * inv))
+                   : -1;
       };
-      bin[lane] = bin[lane + 32] = 0;
+      for (int i = lane; i < kListBins * kFillRow; i += 32) bin[i] = 0;
       __syncwarp();
       near_chunks(w, pt, m, lim, lane, [&](int ib) {
-        int b;
-        if (place(ib + lane, b)) atomicAdd(&bin[b], 1);
+        const int b = place(ib + lane);
+        if (b >= 0) ++bin[b * kFillRow + lane];
       });
       __syncwarp();
-      // exclusive prefix over the steps, two per lane
-      const int c0 = bin[2 * lane], c1 = bin[2 * lane + 1];
-      int sum = c0 + c1;
+      // exclusive prefix over the lanes of steps `lane` and `lane + 32`, then
+      // over the steps
+      int sum[2] = {0, 0};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        int *row = bin + (lane + 32 * q) * kFillRow;
+#pragma unroll 8
+        for (int l = 0; l < 32; ++l) {
+          const int n = row[l];
+          row[l] = sum[q];
+          sum[q] += n;
+        }
+      }
+      int end[2] = {sum[0], sum[1]};
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, sum, o);
-        if (lane >= o) sum += x;
-      }
-      __syncwarp();
-      bin[2 * lane] = sum - c0 - c1;
-      bin[2 * lane + 1] = sum - c1;
-      __syncwarp();
-      ImageRef *out = list + w.uoff[(long long)ui * s.npt + pt].x;
-      near_chunks(w, pt, m, lim, lane, [&](int ib) {
-        int b;
-        const bool in = place(ib + lane, b);
-        const unsigned peers = __match_any_sync(0xffffffffu, b);
-        if (in) {
-          const int pos = bin[b] + __popc(peers & ((1u << lane) - 1));
-          // the step's lower edge, rounded to stay below the distance
-          out[pos] = ImageRef{ib + lane, b * step * (1.f - 1e-5f)};
+        const int x0 = __shfl_up_sync(0xffffffffu, end[0], o);
+        const int x1 = __shfl_up_sync(0xffffffffu, end[1], o);
+        if (lane >= o) {
+          end[0] += x0;
+          end[1] += x1;
         }
-        __syncwarp();
-        if (in && (peers >> lane) == 1u) bin[b] += __popc(peers);
-        __syncwarp();
+      }
+      const int half = __shfl_sync(0xffffffffu, end[0], 31);
+      bin[lane * kFillRow + 32] = end[0] - sum[0];
+      bin[(lane + 32) * kFillRow + 32] = half + end[1] - sum[1];
+      __syncwarp();
+      ImageRef *out = list + range.x;
+      near_chunks(w, pt, m, lim, lane, [&](int ib) {
+        const int b = place(ib + lane);
+        if (b >= 0) {
+          // the step's lower edge, rounded to stay below the distance
+          out[bin[b * kFillRow + 32] + bin[b * kFillRow + lane]++] =
+              ImageRef{ib + lane, b * step * (1.f - 1e-5f)};
+        }
       });
       __syncwarp();
     }
@@ -182,8 +202,8 @@ int launch_list_count(const DevSys &s, const DevWork &w, float margin, int2 *uof
 int launch_list_fill(const DevSys &s, const DevWork &w, float margin, const float *rad,
                      ImageRef *list, cudaStream_t st) {
   if (w.nunits == 0) return IMAGO_OK;
-  const int grid = std::min((w.nunits + kListWarps - 1) / kListWarps, 148 * 8);
-  k_list_fill<<<grid, 32 * kListWarps, 0, st>>>(s, w, margin, rad, list);
+  const int grid = std::min((w.nunits + kFillWarps - 1) / kFillWarps, 148 * 12);
+  k_list_fill<<<grid, 32 * kFillWarps, 0, st>>>(s, w, margin, rad, list);
   IMAGO_CUDA(cudaGetLastError());
   return IMAGO_OK;
 }
