@@ -480,9 +480,10 @@ IMAGO_API int imago_packed_density(int n, int num_kpoints, int ld_states, int nu
  * a thread takes several EP terms of a potential type in one walk over the
  * images (k_prim3c_terms: a launch per class, or all classes in one launch
  * on small systems); mode -1 (the default): all run once on the context's
- * first EP build and the fastest is kept.  NP has one kernel of its own and
- * is the same bit for bit under every mode, EP the same to rounding.  A
- * captured graph of the context is dropped. */
+ * first EP build and the fastest is kept (mode 0 unless another is faster by
+ * a tenth).  NP has one kernel of its own and is the same bit for bit under
+ * every mode, EP the same to rounding.  A captured graph of the context is
+ * dropped. */
 IMAGO_API int imago_intg_set_schedule(imago_ctx *ctx, int mode);
 /* The schedule in use (0, 1 or 2) and the trial times of the measurement
  * (ms, in mode order; zero when not measured). */
