@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(4 * BC, (KOV ? 128 : 256) / BC)
 // of images, so what a thread reads besides its columns (the pair, the
 // images' cells and phases, the origin shift) is shared by its TT terms:
 // 162-atom quartz EP 3.29 -> 1.05 ms at Gamma, 4.63 -> 4.38 at 2x2x2 k
-// (four computed k-points; the scattered stores bound that).  REAL: every
-// phase is 1.
+// (four computed k-points; the scattered stores bound that).  REAL: one
+// k-point whose every phase is 1.
 template <int NK, int TT, bool REAL>
 __global__ void __launch_bounds__(kBC)
     k_bloch_small(DevSys s, DevWork w, int nterm, const double *M, double2 *vv,
@@ -409,10 +409,13 @@ int launch_bloch(const DevSys &s, const DevWork &w, int nterm, const double *M,
                  double2 *vv, double2 *cv, double2 *cc, cudaStream_t st) {
   if (w.nbtile == 0 || nterm == 0) return IMAGO_OK;
   if (s.nkt <= kBlochSmallNk) {
-    // terms per thread: as many as the build has, within 32 sums
-    if (s.real_k && nterm > 4)
+    // terms per thread: as many as the build has, within 32 sums.  A list of
+    // three or more Gamma points has every phase 1 too, but several computed
+    // k-points to write
+    const bool gamma = s.real_k && s.nk == 1;
+    if (gamma && nterm > 4)
       bloch_small<1, 8, true>(s, w, nterm, M, vv, cv, cc, st);
-    else if (s.real_k)
+    else if (gamma)
       bloch_small<1, 1, true>(s, w, nterm, M, vv, cv, cc, st);
     else if (s.nk <= 4 && nterm > 2)
       bloch_small<4, 4, false>(s, w, nterm, M, vv, cv, cc, st);
