@@ -64,11 +64,13 @@ __global__ void k_secular(int V, long long np, int nk, int pot_dim,
 }
 
 // Hashes of each k-point's H and S, and of their conjugates, by which the
-// host finds k-points whose problem is another's conjugate (k and -k of an
-// integral build: the same bits with the imaginary parts negated).  Sums of
-// mixed bit patterns modulo 2^64 over the upper triangle, so the order of the
-// additions does not matter; H and S apart, 128 bits to agree on.  HBM-bound:
-// one pass over what k_secular wrote (Si8, 512 k: 0.18 GB).
+// host finds the k-points whose problem may be another's conjugate (k and -k
+// of an integral build: the same values with the imaginary parts negated);
+// k_conj_check then compares the matrices themselves.  Sums of mixed bit
+// patterns modulo 2^64 over the upper triangle, so the order of the additions
+// does not matter; H and S apart.  HBM-bound: one pass over what k_secular
+// wrote (Si8, 512 k: 0.18 GB).  mix64 and the constant below are the
+// finaliser and the increment of SplitMix64 (Steele, Lea and Flood 2014).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
   x ^= x >> 30;
   x *= 0xbf58476d1ce4e5b9ull;
@@ -101,6 +103,26 @@ __global__ void __launch_bounds__(256)
     for (int o = 16; o > 0; o >>= 1) sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], o);
     if ((threadIdx.x & 31) == 0) atomicAdd(out + 4 * k + m, sum[m]);
   }
+}
+
+// Whether k-point k is value for value the conjugate of pair[k] < k: bad[k]
+// is set where an element of an upper triangle is not (a NaN never is).
+__global__ void __launch_bounds__(256)
+    k_conj_check(int V, const double2 *h, const double2 *s, const int *pair, int *bad) {
+  const int k = blockIdx.x, o = pair[k];
+  if (o == k) return;
+  const long long base = (long long)k * V * V, other = (long long)o * V * V;
+  bool same = true;
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < V * V; e += gridDim.y * blockDim.x) {
+    const int col = e / V, row = e - col * V;
+    if (row > col) continue;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const double2 x = (m ? s : h)[base + e], y = (m ? s : h)[other + e];
+      same = same && x.x == y.x && x.y == -y.y;
+    }
+  }
+  if (!same) bad[k] = 1;
 }
 
 // out[k] = in[map[k]], or the conjugate of in[~map[k]] where map[k] < 0;
@@ -630,41 +652,66 @@ extern "C" int imago_secular_pairs(int n, int num_kpoints, const double *h_full,
   if (n > 32767) return IMAGO_ERR_RANGE;
   if (num_kpoints == 0) return IMAGO_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t bytes = sizeof(unsigned long long) * 4 * (size_t)num_kpoints;
+  // the hashes; then, in the same memory, the candidates and their verdicts
+  const size_t nk = (size_t)num_kpoints, bytes = sizeof(unsigned long long) * 4 * nk;
   void *d = nullptr;
   if (imago::pool_alloc(&d, bytes, st) != cudaSuccess) {
     cudaGetLastError();
     return IMAGO_ERR_NOMEM;
   }
-  std::vector<unsigned long long> hash(4 * (size_t)num_kpoints);
+  const double2 *h = reinterpret_cast<const double2 *>(h_full);
+  const double2 *s = reinterpret_cast<const double2 *>(s_full);
+  std::vector<unsigned long long> hash(4 * nk);
   int rc = IMAGO_OK;
   const unsigned per = (unsigned)std::max(1, std::min(64, 148 * 8 / num_kpoints));
   if (cudaMemsetAsync(d, 0, bytes, st) != cudaSuccess) rc = IMAGO_ERR_CUDA;
   if (!rc) {
     imago::k_conj_hash<<<dim3(num_kpoints, per), 256, 0, st>>>(
-        n, reinterpret_cast<const double2 *>(h_full), reinterpret_cast<const double2 *>(s_full),
-        static_cast<unsigned long long *>(d));
+        n, h, s, static_cast<unsigned long long *>(d));
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpyAsync(hash.data(), d, bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       rc = IMAGO_ERR_CUDA;
   }
+  if (!rc) {
+    // a k-point's candidate is the first earlier one with its conjugate's
+    // hashes
+    bool any = false;
+    std::unordered_multimap<unsigned long long, int> seen;
+    for (int k = 0; k < num_kpoints; ++k) {
+      const unsigned long long *x = &hash[4 * (size_t)k];
+      int first = -1;
+      const auto range = seen.equal_range(x[1]);
+      for (auto it = range.first; it != range.second; ++it)
+        if (hash[4 * (size_t)it->second + 2] == x[3] && (first < 0 || it->second < first))
+          first = it->second;
+      pair[k] = first < 0 ? k : first;
+      any |= first >= 0;
+      if (first < 0) seen.emplace(x[0], k);
+    }
+    if (any) {
+      int *cand = static_cast<int *>(d), *bad = cand + nk;
+      std::vector<int> differs(nk);
+      if (cudaMemcpyAsync(cand, pair, sizeof(int) * nk, cudaMemcpyHostToDevice, st) !=
+              cudaSuccess ||
+          cudaMemsetAsync(bad, 0, sizeof(int) * nk, st) != cudaSuccess)
+        rc = IMAGO_ERR_CUDA;
+      if (!rc) {
+        imago::k_conj_check<<<dim3(num_kpoints, per), 256, 0, st>>>(n, h, s, cand, bad);
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(differs.data(), bad, sizeof(int) * nk, cudaMemcpyDeviceToHost, st) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+          rc = IMAGO_ERR_CUDA;
+      }
+      // one whose hashes alone agreed stands for itself
+      for (int k = 0; k < num_kpoints && !rc; ++k)
+        if (differs[k]) pair[k] = k;
+    }
+  }
   cudaFreeAsync(d, st);
   cudaGetLastError();
-  if (rc) return rc;
-  // a k-point takes the first earlier one that is its conjugate
-  std::unordered_multimap<unsigned long long, int> seen;
-  for (int k = 0; k < num_kpoints; ++k) {
-    const unsigned long long *x = &hash[4 * (size_t)k];
-    int first = -1;
-    const auto range = seen.equal_range(x[1]);
-    for (auto it = range.first; it != range.second; ++it)
-      if (hash[4 * (size_t)it->second + 2] == x[3] && (first < 0 || it->second < first))
-        first = it->second;
-    pair[k] = first < 0 ? k : first;
-    if (first < 0) seen.emplace(x[0], k);
-  }
-  return IMAGO_OK;
+  return rc;
 }
 
 extern "C" int imago_conj_expand(int num_kpoints, long long per, const int *map,

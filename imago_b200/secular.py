@@ -239,7 +239,8 @@ def hermitian_eigh(a):
 
 class _Conjugates:
     """The k-points whose H and S are an earlier k-point's conjugates, as k
-    and -k of an integral build are (imago_secular_pairs): their eigenvalues
+    and -k of an integral build are (imago_secular_pairs, which compares the
+    matrices themselves): their eigenvalues
     are the same and their vectors the conjugates, so only `first` are
     solved.  Finding and spreading them costs 0.23 ms, and below one matrix
     per SM a smaller batch is no faster, so it is tried for n > REDUCE_MAX_N
