@@ -240,12 +240,12 @@ def hermitian_eigh(a):
 class _Conjugates:
     """The k-points whose H and S are an earlier k-point's conjugates, as k
     and -k of an integral build are (imago_secular_pairs, which compares the
-    matrices themselves): their eigenvalues
-    are the same and their vectors the conjugates, so only `first` are
-    solved.  Finding and spreading them costs 0.23 ms, and below one matrix
-    per SM a smaller batch is no faster, so it is tried for n > REDUCE_MAX_N
-    or from PAIR_MIN rows in all.  One B200, eigensystems in ms with every
-    k-point solved / with pairs: n = 104, 512 k 9.7 / 5.4, 216 k 4.70 / 3.09,
+    matrices themselves): their eigenvalues are the same and their vectors the
+    conjugates, so only `first` are solved.  Finding them takes 0.24 ms (n =
+    104, 512 k; 0.19 by their hashes alone), and below one matrix per SM a
+    smaller batch is no faster, so it is tried for n > REDUCE_MAX_N or from
+    PAIR_MIN rows in all.  One B200, eigensystems in ms with every k-point
+    solved / with pairs: n = 104, 512 k 9.7 / 5.4, 216 k 4.70 / 3.09,
     125 k 2.94 / 2.71, 64 k 2.46 / 2.40, 27 k 2.10 / 2.26; n = 64, 216 k 1.54
     / 1.33, 64 k 0.94 / 1.09; n = 208, 64 k 14.2 / 12.6, 8 k 11.9 / 10.4."""
 
@@ -297,6 +297,20 @@ class _Conjugates:
         return out
 
 
+def _cholesky(s, kpoints):
+    """torch.linalg.cholesky of the overlaps of `kpoints`, its error naming
+    the k-point itself rather than its place among them."""
+    lo, info = torch.linalg.cholesky_ex(s)
+    bad = torch.nonzero(info).flatten()
+    if bad.numel():
+        i = int(bad[0])
+        raise torch.linalg.LinAlgError(
+            f"linalg.cholesky: (Batch element {int(kpoints[i])}): The factorization could not be "
+            "completed because the input is not positive-definite (the leading minor of order "
+            f"{int(info[i])} is not positive-definite).")
+    return lo
+
+
 def secular_eigenvalues(out, pot_coeffs, num_states=None):
     """Eigenvalues of H c = E S c per k-point, ascending, [nk, num_states]:
     the Cholesky factor L of S, A = L^-1 H L^-H (cholesky_reduce up to n =
@@ -311,7 +325,7 @@ def secular_eigenvalues(out, pot_coeffs, num_states=None):
         _check_info(info, conj.first)
     else:
         h, s = hs.transpose(-2, -1), ss.transpose(-2, -1)
-        lo = torch.linalg.cholesky(s)
+        lo = _cholesky(s, conj.first)
         y = torch.linalg.solve_triangular(lo, h, upper=False)          # L^-1 H
         a = torch.linalg.solve_triangular(lo, y.mH, upper=False)       # L^-1 H L^-H
         ev = hermitian_eigvals(a)
@@ -339,7 +353,7 @@ def secular_eigensystem(out, pot_coeffs, num_states=None):
         _check_info(info, conj.first)
         return conj.values(ev)[:, :ns], conj.vectors(c).transpose(-2, -1)
     h, s = hs.transpose(-2, -1), ss.transpose(-2, -1)
-    lo = torch.linalg.cholesky(s)
+    lo = _cholesky(s, conj.first)
     y = torch.linalg.solve_triangular(lo, h, upper=False)
     a = torch.linalg.solve_triangular(lo, y.mH, upper=False)
     ev, vec = hermitian_eigh(a)

@@ -112,3 +112,31 @@ def test_equal_hashes_of_different_problems_are_told_apart(imago_lib, monkeypatc
     # the one that is the first one's conjugate is still solved with it
     hs, ss = secular._secular_storage(out, np.zeros(0))
     assert list(secular._Conjugates(hs, ss).first) == [0, 1, 3]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solve", ["secular_eigenvalues", "secular_eigensystem"])
+@pytest.mark.parametrize("paired", [True, False])
+def test_large_failing_overlap_names_its_k_point(imago_lib, solve, paired):
+    # n > 128, factorised by torch: the message of torch.linalg.cholesky over
+    # every k-point, whether or not some were left out as another's conjugate
+    import torch
+    from imago_b200 import secular
+    rng = np.random.default_rng(6)
+    n, nk = 130, 5
+    a = rng.normal(size=(nk, n, n)) + 1j * rng.normal(size=(nk, n, n))
+    a = a + a.conj().transpose(0, 2, 1)
+    if paired:
+        a[1] = a[0].conj()
+    s = np.stack([np.eye(n, dtype=complex)] * nk)
+    s[3, 6, 6] = -1.0
+    with pytest.raises(torch.linalg.LinAlgError) as ref:
+        torch.linalg.cholesky(torch.as_tensor(s, device="cuda"))
+    assert "3" in str(ref.value) and "7" in str(ref.value)
+    pack = lambda x: torch.as_tensor(np.stack([x[:, r, c] for c in range(n) for r in range(c + 1)], 1)
+                                     .view(np.float64).reshape(nk, -1, 2), device="cuda")
+    out = {"np_packed": pack(a), "ol_packed": pack(s), "ep_packed": None}
+    out["ke_packed"] = torch.zeros_like(out["np_packed"])
+    with pytest.raises(torch.linalg.LinAlgError) as err:
+        getattr(secular, solve)(out, np.zeros(0))
+    assert str(err.value) == str(ref.value)
