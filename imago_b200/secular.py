@@ -282,9 +282,10 @@ class _Conjugates:
         return e if self.all else e.index_select(0, self._place)
 
     def vectors(self, c):
-        """c [solved, a, b] (contiguous) spread over every k-point."""
+        """c [solved, a, b] spread over every k-point."""
         if self.all:
             return c
+        c = c.contiguous()
         nk, per = self._map.numel(), c[0].numel()
         out = torch.empty((nk,) + c.shape[1:], dtype=c.dtype, device=c.device)
         L = intg.lib()
@@ -360,4 +361,4 @@ def secular_eigensystem(out, pot_coeffs, num_states=None):
     c = torch.linalg.solve_triangular(lo.mH, vec, upper=True)
     if num_states is not None:
         ev, c = ev[:, :num_states], c[:, :, :num_states]
-    return conj.values(ev), conj.vectors(c.contiguous())
+    return conj.values(ev), conj.vectors(c)

@@ -140,3 +140,23 @@ def test_large_failing_overlap_names_its_k_point(imago_lib, solve, paired):
     with pytest.raises(torch.linalg.LinAlgError) as err:
         getattr(secular, solve)(out, np.zeros(0))
     assert str(err.value) == str(ref.value)
+
+
+@pytest.mark.gpu
+def test_large_vectors_are_not_copied_where_nothing_is_paired(imago_lib):
+    # n > 128: the vectors come as the triangular solve stores them, by columns
+    import torch
+    from imago_b200 import secular
+    rng = np.random.default_rng(7)
+    n, nk = 131, 2
+    a = rng.normal(size=(nk, n, n)) + 1j * rng.normal(size=(nk, n, n))
+    a = a + a.conj().transpose(0, 2, 1)
+    pack = lambda x: torch.as_tensor(np.stack([x[:, r, c] for c in range(n) for r in range(c + 1)], 1)
+                                     .view(np.float64).reshape(nk, -1, 2), device="cuda")
+    out = {"np_packed": pack(a), "ol_packed": pack(np.stack([np.eye(n, dtype=complex)] * nk)),
+           "ep_packed": None}
+    out["ke_packed"] = torch.zeros_like(out["np_packed"])
+    e, c = secular.secular_eigensystem(out, np.zeros(0))
+    assert c.stride(-2) == 1
+    e, c = e.cpu().numpy(), c.cpu().numpy()
+    assert np.abs(a @ c - c * e[:, None, :]).max() <= 1e-11 * np.abs(e).max()
