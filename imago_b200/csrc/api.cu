@@ -177,6 +177,7 @@ struct imago_ctx {
   std::vector<int2> kout;
   int vale_dim = 0, core_dim = 0, pot_dim = 0;
   double T = 0.0;
+  double cell_lim = 0.0;  // |R|^2 within which the cell list was asked for
   double rv[9], recip[9], inv[9];
   std::vector<double> site_pos, psite_pos, cells, csize, kxyz;
   std::vector<int> site_type, psite_ptype, cum_vale, cum_core;
@@ -238,6 +239,7 @@ struct imago_ctx {
   DBuf<int2> d_uoff;
   DBuf<ImageRef> d_ulist;
   DBuf<float> d_rad;
+  DBuf<unsigned char> d_listed;  // bounded systems only (DevSys)
 
   // scratch
   // Each build kind (OL, KE, NP, EP) has its own scratch and stream (a
@@ -317,7 +319,7 @@ struct imago_ctx {
     d_ipos.release(st); d_ftab.release(st); d_img_off.release(st);
     d_chunk.release(st); d_chunk_off.release(st);
     d_ptype_ascends.release(st); d_uoff.release(st); d_ulist.release(st);
-    d_rad.release(st);
+    d_rad.release(st); d_listed.release(st);
     d_queue.release(st);
     d_flag.release(st);
     d_kout.release(st);
@@ -396,6 +398,7 @@ int make_cells(imago_ctx *c, double min_atom_alpha, double min_pot_alpha) {
   }
   lim = lim + 0.75 * maxsq + std::sqrt(3.0 * maxsq * lim);
   lim = std::max(lim, 2.0 * c->T / min_atom_alpha);
+  c->cell_lim = lim;
   lattice_points(c->rv, lim, c->cells, c->csize);
   c->ncell = (int)c->csize.size();
   return IMAGO_OK;
@@ -882,6 +885,8 @@ constexpr size_t kMaxImageListBytes = size_t(4) << 30;
 // lies within sqrt(T / xi) of atom 1 and an image within sqrt(T / mu) of it,
 // the two sharing T, so that |C - A|^2 <= T (1 / xi + 1 / zeta + 1 / a3) <=
 // T (5 / (2 a) + 1 / a3) (screening exponents); atom 1 is in the home cell.
+// In a bounded system (DevSys) an image is also within reach_cap of the
+// product centre.
 struct ImageTable {
   std::vector<double4> pos;
   std::vector<float4> fpos;
@@ -889,18 +894,86 @@ struct ImageTable {
   std::vector<int> off, chunk_off;
   double a3_min = 0.0;
   float margin = 0.f;
+  bool bounded = false;
+  double reach_cap = 1e300;
+  int span[3] = {0, 0, 0};
+  std::vector<unsigned char> listed;  // bounded only
 };
+
+// The length up to which the cell list holds every lattice vector: all of
+// those within cell_lim that lattice_points' box along the axes has.
+double cells_sure(const imago_ctx *c) {
+  double r = std::sqrt(c->cell_lim);
+  for (int i = 0; i < 3; ++i) {
+    double v = 0.0, n = 0.0;
+    for (int x = 0; x < 3; ++x) {
+      v += c->rv[3 * i + x] * c->rv[3 * i + x];
+      n += c->inv[3 * i + x] * c->inv[3 * i + x];
+    }
+    r = std::min(r, (std::ceil(std::sqrt(c->cell_lim) / std::sqrt(v)) + 1.0) / std::sqrt(n));
+  }
+  return r * (1.0 - 1e-9);
+}
+
+// A bound of the distance from any point to the nearest lattice point: half
+// the cell's longest diagonal.
+double half_diagonal(const imago_ctx *c) {
+  double d2 = 0.0;
+  for (int s = 0; s < 4; ++s) {
+    double d = 0.0;
+    for (int x = 0; x < 3; ++x) {
+      const double v = c->rv[x] + (s & 1 ? -1 : 1) * c->rv[3 + x] + (s & 2 ? -1 : 1) * c->rv[6 + x];
+      d += v * v;
+    }
+    d2 = std::max(d2, d);
+  }
+  return 0.5 * std::sqrt(d2) * (1.0 + 1e-9);
+}
+
+// A closer bound for skewed cells: the largest distance on a grid over the
+// cell and half a grid cell's diagonal.
+double grid_distance(const imago_ctx *c) {
+  constexpr int kGrid = 12;
+  double far2 = 0.0;
+  for (int g = 0; g < kGrid * kGrid * kGrid; ++g) {
+    const double f[3] = {(g % kGrid + 0.5) / kGrid - 0.5, (g / kGrid % kGrid + 0.5) / kGrid - 0.5,
+                         (g / (kGrid * kGrid) + 0.5) / kGrid - 0.5};
+    double near2 = 1e300;
+    for (int n = 0; n < 27; ++n) {
+      const double q[3] = {f[0] + n % 3 - 1, f[1] + n / 3 % 3 - 1, f[2] + n / 9 - 1};
+      double d = 0.0;
+      for (int x = 0; x < 3; ++x) {
+        const double v = q[0] * c->rv[x] + q[1] * c->rv[3 + x] + q[2] * c->rv[6 + x];
+        d += v * v;
+      }
+      near2 = std::min(near2, d);
+    }
+    far2 = std::max(far2, near2);
+  }
+  return std::sqrt(far2) + half_diagonal(c) / kGrid;
+}
 
 void make_images(const imago_ctx *c, ImageTable &tab) {
   double amin = 1e300, a3 = 1e300;
   for (int t = 0; t < c->nt; ++t)
     for (double a : c->types[c->type_screen[t]].alphas) amin = std::min(amin, a);
+  // (the third centres whose screens let an image through: a negative radius
+  // takes none, and neutral sites have no nuclear term)
   for (int t = 0; t < c->npt; ++t) {
     const HPType &p = c->ptypes[c->ptype_screen[t]];
-    for (double a : p.alphas) a3 = std::min(a3, a);
-    a3 = std::min(a3, p.nucalpha);
+    for (double a : p.alphas)
+      if (a >= 0.0) a3 = std::min(a3, a);
+    if (!(c->ptypes[t].z < kSmallThresh)) a3 = std::min(a3, p.nucalpha);
   }
   tab.a3_min = a3;
+  // bounded where the list is shorter than the largest screening radius and
+  // the distance to the nearest lattice point together
+  const double radius = std::sqrt(c->T * (0.5 / amin + 1.0 / a3)), sure = cells_sure(c);
+  double nearest = half_diagonal(c);
+  if (!(radius + nearest <= sure)) {
+    nearest = std::min(nearest, grid_distance(c));
+    tab.bounded = !(radius + nearest <= sure);
+  }
   double mid[3] = {0, 0, 0}, rho = 0.0, rho_p = 0.0;
   for (int i = 0; i < c->ns; ++i)
     for (int x = 0; x < 3; ++x) mid[x] += c->site_pos[3 * i + x] / c->ns;
@@ -911,7 +984,27 @@ void make_images(const imago_ctx *c, ImageTable &tab) {
   };
   for (int i = 0; i < c->ns; ++i) rho = std::max(rho, from_mid(&c->site_pos[3 * i]));
   for (int i = 0; i < c->nps; ++i) rho_p = std::max(rho_p, from_mid(&c->psite_pos[3 * i]));
-  const double rad = (rho + std::sqrt(c->T * (2.5 / amin + 1.0 / a3))) * (1.0 + 1e-9) + 1e-6;
+  double reach = std::sqrt(c->T * (2.5 / amin + 1.0 / a3));
+  if (tab.bounded) {
+    tab.reach_cap = (nearest + std::sqrt(c->csize[c->ncell - 1])) * (1.0 + 1e-9);
+    reach = std::min(reach, std::sqrt(2.0 * c->T / amin) + tab.reach_cap);
+    std::vector<std::array<int, 3>> ns(c->ncell);
+    for (int q = 0; q < c->ncell; ++q)
+      for (int i = 0; i < 3; ++i) {
+        const double *R = &c->cells[3 * q];
+        ns[q][i] = (int)std::lround(R[0] * c->inv[3 * i] + R[1] * c->inv[3 * i + 1] +
+                                    R[2] * c->inv[3 * i + 2]);
+        tab.span[i] = std::max(tab.span[i], std::abs(ns[q][i]));
+      }
+    tab.listed.assign((2 * (size_t)tab.span[0] + 1) * (2 * tab.span[1] + 1) * (2 * tab.span[2] + 1),
+                      0);
+    for (const auto &n : ns) {
+      size_t at = 0;
+      for (int i = 0; i < 3; ++i) at = at * (2 * tab.span[i] + 1) + n[i] + tab.span[i];
+      tab.listed[at] = 1;
+    }
+  }
+  const double rad = (rho + reach) * (1.0 + 1e-9) + 1e-6;
   // lattice vectors that bring some site into the sphere
   int lim[3];
   for (int i = 0; i < 3; ++i) {
@@ -1077,6 +1170,7 @@ int upload(imago_ctx *c) {
   UP(d_btile, c->btile) UP(d_btile_w, c->btile_w) UP(d_kout, c->kout)
   UP(d_ptype_ascends, pasc) UP(d_ipos, tab.pos) UP(d_ftab, tab.fpos) UP(d_img_off, tab.off)
   UP(d_chunk, tab.chunk) UP(d_chunk_off, tab.chunk_off)
+  if (tab.bounded) UP(d_listed, tab.listed)
 #undef UP
   if ((rc = c->d_queue.alloc(4, st))) return rc;
   if ((rc = c->d_flag.alloc(1, st))) return rc;
@@ -1099,6 +1193,21 @@ int upload(imago_ctx *c) {
   std::memcpy(s.rv, c->rv, sizeof s.rv);
   std::memcpy(s.inv, c->inv, sizeof s.inv);
   s.a3_min = tab.a3_min;
+  s.bounded = tab.bounded;
+  s.reach_cap = tab.reach_cap;
+  for (int i = 0; i < 3; ++i) s.span[i] = tab.span[i];
+  s.listed = c->d_listed.p;
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) {
+      s.gram[3 * i + j] = 0.0;
+      for (int x = 0; x < 3; ++x) s.gram[3 * i + j] += c->rv[3 * i + x] * c->rv[3 * j + x];
+    }
+  for (int m = 1; m <= 13; ++m) {
+    const int d[3] = {(13 + m) / 9 - 1, (13 + m) / 3 % 3 - 1, (13 + m) % 3 - 1};
+    s.neighbour[m - 1] = 0.0;
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j) s.neighbour[m - 1] += d[i] * d[j] * s.gram[3 * i + j];
+  }
   s.ptype_ascends = c->d_ptype_ascends.p;
   s.real_k = 1;
   for (double x : c->kxyz) s.real_k &= x == 0.0;

@@ -39,6 +39,53 @@ __device__ __forceinline__ double image_d2(const double Ps[3], const double4 &C)
   return x * x + y * y + z * z;
 }
 
+// A bounded system's d2 = |Ps - C|^2 of an image: the least screening radius^2
+// at which the reference's walk around Ps (integrals.F90:2632-2660, 2791-2819)
+// comes to image C.  The site's image closest to Ps has to pass the screen
+// too, and the lattice vector from there to C has to be in the cell list (else
+// infinity).  The closest image (findLatticeVector, lattice.f90:784-888) is
+// the one that rounding the fractional coordinates gives or one of its 26
+// neighbours: with residual r, |r - d|^2 = |r|^2 + d.G d - 2 d.G r, G the
+// lattice's Gram matrix, so a pair of neighbours +-d costs one comparison.
+__device__ __forceinline__ double listed_d2(const DevSys &s, const double Ps[3], const double4 &C,
+                                            double d2) {
+  const double v[3] = {Ps[0] - C.x, Ps[1] - C.y, Ps[2] - C.z};
+  double r[3], g[3];
+  int n[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const double f = v[0] * s.inv[3 * i] + v[1] * s.inv[3 * i + 1] + v[2] * s.inv[3 * i + 2];
+    n[i] = __double2int_rn(f);
+    r[i] = f - n[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    g[i] = s.gram[3 * i] * r[0] + s.gram[3 * i + 1] * r[1] + s.gram[3 * i + 2] * r[2];
+  const double r2 = r[0] * g[0] + r[1] * g[1] + r[2] * g[2];
+  double best = -1e-12 * r2;
+  int step = 0;  // code of the neighbour taken: 13 itself, less 13
+#pragma unroll
+  for (int m = 1; m <= 13; ++m) {
+    const int d0 = (13 + m) / 9 - 1, d1 = (13 + m) / 3 % 3 - 1, d2_ = (13 + m) % 3 - 1;
+    const double dg = d0 * g[0] + d1 * g[1] + d2_ * g[2];
+    const double x = s.neighbour[m - 1] - 2.0 * fabs(dg);
+    if (x < best) {
+      best = x;
+      step = dg > 0.0 ? m : -m;
+    }
+  }
+  n[0] += (13 + step) / 9 - 1;
+  n[1] += (13 + step) / 3 % 3 - 1;
+  n[2] += (13 + step) % 3 - 1;
+  // C lies at -n from the closest image
+  if (abs(n[0]) > s.span[0] || abs(n[1]) > s.span[1] || abs(n[2]) > s.span[2]) return INFINITY;
+  const long long at = ((long long)(s.span[0] - n[0]) * (2 * s.span[1] + 1) + s.span[1] - n[1]) *
+                           (2 * s.span[2] + 1) + s.span[2] - n[2];
+  if (!s.listed[at]) return INFINITY;
+  const double c0 = r2 + (step ? best : 0.0);
+  return c0 > d2 * (1.0 + 1e-9) ? c0 : d2;
+}
+
 struct SpGeom {
   double A[3], B[3];   // atom 1, shifted atom 2
   double a1, a2;       // primitive exponents

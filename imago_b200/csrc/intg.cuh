@@ -47,6 +47,17 @@ struct DevSys {
   // that the screening radius falls from term to term
   const int *ptype_ascends;
   double a3_min;          // smallest screening exponent of any third centre
+  // Some three-centre screen may reach beyond the lattice cell list, with
+  // which the reference's sums over a site's images end: each image is then
+  // looked up (listed_d2) in `listed`, one byte per lattice vector with
+  // coefficients within +-span.  No image that counts is further than
+  // reach_cap from the product centre; gram is the lattice's Gram matrix,
+  // neighbour[m - 1] the squared length of the lattice vector with
+  // coefficients (digits of 13 + m in base 3) - 1
+  int bounded;
+  int span[3];
+  double reach_cap, gram[9], neighbour[13];
+  const unsigned char *listed;
   // lattice cells sorted by |R|^2, k-points, phase table
   const double *cell;     // [n*3]
   const double *csize;    // [n]
@@ -209,7 +220,10 @@ int launch_prim3c_count(const DevSys &s, const DevWork &w, const int *cls_beg,
                         const Term3c *terms_dev, int nterm, bool nuclear,
                         unsigned long long *count16, cudaStream_t st);
 
-// EP terms, one launch per class, one (shell pair, term) per thread.
+// EP terms, one launch per class, one (shell pair, term) per thread; the
+// other forms come here for a bounded system, whose look-ups cost about as
+// much as an image's integrals (8 Si atoms in a cell sheared to 17 degrees:
+// EP 7.4 ms of primitives, 4.3 without them).
 int launch_prim3c(const DevSys &s, const DevWork &w, const int *cls_beg,
                   const Term3c *terms_dev, int nterm, double *blk, cudaStream_t st);
 // EP terms, one launch per class, a thread taking several terms of a type

@@ -22,7 +22,7 @@ namespace imago {
 template <int T>
 constexpr int kHamTerms = T >= 4 ? 32 : 8;
 
-template <int LA, int LB, int T, int SPIN>
+template <int LA, int LB, int T, int SPIN, bool BND>
 __global__ void __launch_bounds__(128, LA + LB >= 4 ? (SPIN == 2 ? 2 : 3) : (SPIN == 2 ? 3 : 4))
     k_prim3c_ham(DevSys s, DevWork w, int beg, int n, const Term3c *terms, int nterm,
                  const double *coef, double *H) {
@@ -75,8 +75,12 @@ __global__ void __launch_bounds__(128, LA + LB >= 4 ? (SPIN == 2 ? 2 : 3) : (SPI
         en = uw.at(r + T);
         Cn = w.ipos[en.idx];
       }
-      const double d2 = image_d2(c.Ps, C);
+      double d2 = image_d2(c.Ps, C);
       if (d2 > tmax) continue;
+      if constexpr (BND) {
+        d2 = listed_d2(s, c.Ps, C, d2);
+        if (d2 > tmax) continue;
+      }
       const double X[3] = {c.Pt[0] - C.x, c.Pt[1] - C.y, c.Pt[2] - C.z};
       const double x2 = X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
       double G[SPIN][L + 1];
@@ -120,13 +124,16 @@ static int ham_one(const DevSys &s, const DevWork &w, int beg, int n, const Term
                    const double *coef, int lanes, double *H,
                    cudaStream_t st) {
   if (n <= 0) return IMAGO_OK;
+  if (s.bounded) lanes = 4;
   const unsigned grid = (unsigned)(((long long)n * lanes + 127) / 128);
-  if (lanes == 8)
-    k_prim3c_ham<LA, LB, 8, SPIN><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
+  if (s.bounded)
+    k_prim3c_ham<LA, LB, 4, SPIN, true><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
+  else if (lanes == 8)
+    k_prim3c_ham<LA, LB, 8, SPIN, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
   else if (lanes == 4)
-    k_prim3c_ham<LA, LB, 4, SPIN><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
+    k_prim3c_ham<LA, LB, 4, SPIN, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
   else
-    k_prim3c_ham<LA, LB, 1, SPIN><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
+    k_prim3c_ham<LA, LB, 1, SPIN, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
   IMAGO_CUDA(cudaGetLastError());
   return IMAGO_OK;
 }

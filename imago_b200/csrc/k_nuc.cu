@@ -12,7 +12,7 @@ namespace imago {
 // hundreds of images, at some 300 FP64 operations each for the nuclear
 // term: one lane per pair left the GPU waiting for the longest of them
 // (0.7 of the 0.75 ms of the two-atom diamond cell's nuclear term).
-template <int LA, int LB, int T>
+template <int LA, int LB, int T, bool BND>
 __global__ void __launch_bounds__(128, LA + LB >= 4 ? 3 : 4)
     k_prim3c_nuc(DevSys s, DevWork w, int beg, int n, double *blk, bool add) {
   constexpr int L = LA + LB;
@@ -46,7 +46,11 @@ __global__ void __launch_bounds__(128, LA + LB >= 4 ? 3 : 4)
         en = uw.at(r + T);
         Cn = w.ipos[en.idx];
       }
-      if (image_d2(c.Ps, C) > t) continue;
+      const double d2 = image_d2(c.Ps, C);
+      if (d2 > t) continue;
+      if constexpr (BND) {
+        if (listed_d2(s, c.Ps, C, d2) > t) continue;
+      }
       const double X[3] = {c.Pt[0] - C.x, c.Pt[1] - C.y, c.Pt[2] - C.z};
       accumulate_nuclear_q<L>(X, mu, nu, w0, Q);
     }
@@ -70,12 +74,18 @@ template <int LA, int LB>
 static int nuc_one(const DevSys &s, const DevWork &w, int beg, int n, int lanes, double *blk,
                    cudaStream_t st, bool add) {
   if (n <= 0) return IMAGO_OK;
+  if (s.bounded) lanes = 4;
   const unsigned grid = (unsigned)(((long long)n * lanes + 127) / 128);
   switch (lanes) {
-    case 8: k_prim3c_nuc<LA, LB, 8><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
-    case 4: k_prim3c_nuc<LA, LB, 4><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
-    case 2: k_prim3c_nuc<LA, LB, 2><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
-    default: k_prim3c_nuc<LA, LB, 1><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add);
+    case 8: k_prim3c_nuc<LA, LB, 8, false><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
+    case 4:
+      if (s.bounded)
+        k_prim3c_nuc<LA, LB, 4, true><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add);
+      else
+        k_prim3c_nuc<LA, LB, 4, false><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add);
+      break;
+    case 2: k_prim3c_nuc<LA, LB, 2, false><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
+    default: k_prim3c_nuc<LA, LB, 1, false><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add);
   }
   IMAGO_CUDA(cudaGetLastError());
   return IMAGO_OK;

@@ -78,8 +78,8 @@ __global__ void __launch_bounds__(128)
 // the class's list.  Shared by the per-class launches and the work queue.
 // CNT: the same walk, of EP terms or (NUC) of the nuclear term, counting
 // the screened (site, image) triples into *ntrip instead of integrating
-// (nothing is written).
-template <int LA, int LB, bool NUC, bool CNT = false>
+// (nothing is written).  BND: a bounded system (DevSys).
+template <int LA, int LB, bool NUC, bool CNT = false, bool BND = false>
 __device__ __forceinline__ void prim3c_item(const DevSys &s, const DevWork &w, int beg,
                                             int n, const Term3c *terms, double *blk,
                                             long long g, unsigned *ntrip = nullptr) {
@@ -113,7 +113,11 @@ __device__ __forceinline__ void prim3c_item(const DevSys &s, const DevWork &w, i
         en = uw.at(r + 1);
         Cn = w.ipos[en.idx];
       }
-      if (image_d2(c.Ps, C) > t) continue;
+      const double d2 = image_d2(c.Ps, C);
+      if (d2 > t) continue;
+      if constexpr (BND) {
+        if (listed_d2(s, c.Ps, C, d2) > t) continue;
+      }
       if constexpr (CNT) {
         ++*ntrip;
       } else {
@@ -138,19 +142,23 @@ __global__ void __launch_bounds__(128)
                    unsigned long long *count) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned c = 0;
-  if (g < (long long)n * nterm)
-    prim3c_item<LA, LB, NUC, true>(s, w, beg, n, terms, nullptr, g, &c);
+  if (g < (long long)n * nterm) {
+    if (s.bounded)
+      prim3c_item<LA, LB, NUC, true, true>(s, w, beg, n, terms, nullptr, g, &c);
+    else
+      prim3c_item<LA, LB, NUC, true>(s, w, beg, n, terms, nullptr, g, &c);
+  }
   c = __reduce_add_sync(0xffffffffu, c);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
 }
 
-template <int LA, int LB>
+template <int LA, int LB, bool BND>
 __global__ void __launch_bounds__(128, LA + LB >= 4 ? 3 : (LA + LB >= 3 ? 4 : (LA + LB == 2 ? 5 : 6)))
     k_prim3c(DevSys s, DevWork w, int beg, int n, const Term3c *terms,
              int nterm, double *blk) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (long long)n * nterm) return;
-  prim3c_item<LA, LB, false>(s, w, beg, n, terms, blk, g);
+  prim3c_item<LA, LB, false, false, BND>(s, w, beg, n, terms, blk, g);
 }
 
 // f classes of k_prim3c_ham, runtime loops.
@@ -178,7 +186,8 @@ __global__ void __launch_bounds__(128)
       const ImageRef e = uw.at(r);
       if (beyond(e.d1, c.pmf, tf)) break;
       const double4 C = w.ipos[e.idx];
-      if (image_d2(c.Ps, C) > t) continue;
+      const double d2 = image_d2(c.Ps, C);
+      if (d2 > t || (s.bounded && listed_d2(s, c.Ps, C, d2) > t)) continue;
       const double X[3] = {c.Pt[0] - C.x, c.Pt[1] - C.y, c.Pt[2] - C.z};
       accumulate_overlap_q_rt(L, X, mu, wt, Q);
     }
@@ -227,7 +236,8 @@ __device__ __noinline__ void prim3c_item_rt(const DevSys &s, const DevWork &w, i
       const ImageRef e = uw.at(r);
       if (beyond(e.d1, c.pmf, tf)) break;
       const double4 C = w.ipos[e.idx];
-      if (image_d2(c.Ps, C) > t) continue;
+      const double d2 = image_d2(c.Ps, C);
+      if (d2 > t || (s.bounded && listed_d2(s, c.Ps, C, d2) > t)) continue;
       const double X[3] = {c.Pt[0] - C.x, c.Pt[1] - C.y, c.Pt[2] - C.z};
       if (NUC)
         accumulate_nuclear_q_rt(L, X, mu, nu, w0, Q);
@@ -483,6 +493,7 @@ int launch_prim3c_queue(const DevSys &s, const DevWork &w, const int *cls_beg,
                         const Term3c *terms_dev, int nterm, double *blk,
                         unsigned long long *counter, int ctas, cudaStream_t st) {
   if (nterm <= 0) return IMAGO_OK;
+  if (s.bounded) return launch_prim3c(s, w, cls_beg, terms_dev, nterm, blk, st);
   Prim3cQueue qc{};
   // highest l_a + l_b first, then the larger l_a
   int order[16], m = 0;
@@ -532,7 +543,12 @@ int launch_prim3c(const DevSys &s, const DevWork &w, const int *cls_beg,
     const int beg = cls_beg[a * 4 + b], n = cls_beg[a * 4 + b + 1] - beg;           \
     if (n > 0) {                                                                    \
       const unsigned grid = (unsigned)(((long long)n * nterm + 127) / 128);         \
-      k_prim3c<a, b><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, blk);    \
+      if (s.bounded)                                                                \
+        k_prim3c<a, b, true><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm,  \
+                                                   blk);                            \
+      else                                                                          \
+        k_prim3c<a, b, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, \
+                                                    blk);                           \
       IMAGO_CUDA(cudaGetLastError());                                               \
     }                                                                               \
   }

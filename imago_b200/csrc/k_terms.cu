@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(32 * kListWarps)
       const double a = as1[sp.a], b = as2[sp.b], z = a + b;
       const double frac = fmax(0.0, 1.0 - u.r2 * (a * b / z) / s.T);
       const double t = frac * s.T * (z + s.a3_min) / (z * s.a3_min);
-      reach = fmax(reach, fabs(a / z - 0.5) * r + sqrt(t));
+      reach = fmax(reach, fabs(a / z - 0.5) * r + fmin(sqrt(t), s.reach_cap));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) reach = fmax(reach, __shfl_xor_sync(0xffffffffu, reach, o));
@@ -384,6 +384,7 @@ constexpr long long kTermThreadsMerged = 400000, kTermThreadsWanted = 800000;
 int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
                         const Term3c *terms_dev, const Term3c *terms_host, int nterm,
                         double *blk, cudaStream_t st) {
+  if (s.bounded) return launch_prim3c(s, w, cls_beg, terms_dev, nterm, blk, st);
   int runs = 0;
   for (int i = 0; i < nterm; ++i) runs += i == 0 || terms_host[i].ptype != terms_host[i - 1].ptype;
   const long long base = std::max(1LL, (long long)w.nsp * std::max(1, runs));
