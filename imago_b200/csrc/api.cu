@@ -1893,27 +1893,30 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
                  (c->core_dim > 0 ? 2 : 1);
   mark(c);
   // the kinetic, mass-velocity (written negatively, the sign the reference
-  // subtracts it with) and nuclear blocks, each added as it is stored, beside
-  // the potential terms on the kinetic lane
-  const int lane = c->lane;
-  c->lane = KIND_KE;
-  cudaStream_t bst = c->cur();
-  double *base = nullptr;
-  rc = cudaStreamWaitEvent(bst, c->kfork, 0) == cudaSuccess ? ensure_scratch(c, 1)
-                                                            : (int)IMAGO_ERR_CUDA;
-  if (!rc) {
-    base = c->scr[KIND_KE].blk.p;
-    rc = launch_prim2c(s, w, c->cls_beg, kPrim2cKinetic, base, bst);
-  }
-  if (!rc && rel) rc = launch_prim2c(s, w, c->cls_beg, kPrim2cMassVel, base, bst, true);
-  if (!rc) rc = launch_prim3c_nuc(s, w, c->cls_beg, base, bst, true);
-  if (cudaEventRecord(c->kjoin[KIND_KE], bst) != cudaSuccess && !rc) rc = IMAGO_ERR_CUDA;
-  c->lane = lane;
-  if (rc) return rc;
+  // subtracts it with) and nuclear blocks, each added as it is stored
+  double *base = S.blk.p;
+  auto base_blocks = [&](cudaStream_t bst) {
+    int r = launch_prim2c(s, w, c->cls_beg, kPrim2cKinetic, base, bst);
+    if (!r && rel) r = launch_prim2c(s, w, c->cls_beg, kPrim2cMassVel, base, bst, true);
+    return r ? r : launch_prim3c_nuc(s, w, c->cls_beg, base, bst, true);
+  };
   if (fused) {
+    // beside the potential terms, on the kinetic lane's stream (kfork: after
+    // this lane's scratch is there)
+    const int lane = c->lane;
+    c->lane = KIND_KE;
+    cudaStream_t bst = c->cur();
+    c->lane = lane;
+    if (cudaEventRecord(c->kfork, st) != cudaSuccess ||
+        cudaStreamWaitEvent(bst, c->kfork, 0) != cudaSuccess)
+      return IMAGO_ERR_CUDA;
+    rc = base_blocks(bst);
+    if (cudaEventRecord(c->kjoin[KIND_KE], bst) != cudaSuccess && !rc) rc = IMAGO_ERR_CUDA;
+    if (rc) return rc;
     if ((rc = launch_prim3c_ham(s, w, c->cls_beg, c->d_terms.p, c->pot_dim, c->ham_w.p, spin, lanes,
                                 c->ham_blk.p, st)))
       return rc;
+    IMAGO_CUDA(cudaStreamWaitEvent(st, c->kjoin[KIND_KE], 0));
   } else {
     IMAGO_CUDA(cudaMemsetAsync(c->ham_blk.p, 0, sizeof(double) * n * spin, st));
     for (int t0 = 0; t0 < c->pot_dim; t0 += chunk) {
@@ -1925,8 +1928,8 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
                                   c->ham_blk.p, st)))
         return rc;
     }
+    if ((rc = base_blocks(st))) return rc;
   }
-  IMAGO_CUDA(cudaStreamWaitEvent(st, c->kjoin[KIND_KE], 0));
   if ((rc = launch_block_axpy(base, 1, n, nullptr, 0, spin, c->ham_blk.p, st))) return rc;
   mark(c);
   if ((rc = launch_contract(s, w, spin, c->ham_blk.p, S.M.p, st))) return rc;
