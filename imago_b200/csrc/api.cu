@@ -1095,26 +1095,46 @@ void set_bloch_width(imago_ctx *c, int wi) {
   c->work.nbtile_w = c->btile_off[wi + 1] - c->btile_off[wi];
 }
 
-// The units' image lists; without memory for them (or beyond
-// kMaxImageListBytes) the kernels test every image of a type.
+// Bytes the image lists and their ranges may take together: IMAGO_TUNING's
+// lists=off, lists=<MiB>, or kMaxImageListBytes.
+size_t image_list_limit() {
+  const char *env = std::getenv("IMAGO_TUNING");
+  const char *at = env ? std::strstr(env, "lists=") : nullptr;
+  if (!at) return kMaxImageListBytes;
+  at += std::strlen("lists=");
+  if (!std::strncmp(at, "off", 3)) return 0;
+  char *end = nullptr;
+  const unsigned long mib = std::strtoul(at, &end, 10);
+  return end == at ? kMaxImageListBytes : std::min(kMaxImageListBytes, (size_t)mib << 20);
+}
+
+// The units' image lists; without memory for them, or beyond
+// image_list_limit, the kernels test every image of a type.
 int build_lists(imago_ctx *c, float margin) {
   cudaStream_t st = c->stream;
   DevWork &w = c->work;
-  const size_t nu = (size_t)w.nunits;
-  const char *env = std::getenv("IMAGO_TUNING");
-  if (env && std::strstr(env, "lists=off")) return IMAGO_OK;
-  if (nu == 0 || c->d_uoff.alloc(nu * c->npt, st) || c->d_rad.alloc(nu, st)) return IMAGO_OK;
+  const size_t nu = (size_t)w.nunits, limit = image_list_limit();
+  const size_t ranges = nu * c->npt * sizeof(int2);
+  if (nu == 0 || ranges > limit) return IMAGO_OK;
+  auto none = [&] {
+    c->d_uoff.release(st);
+    c->d_rad.release(st);
+    return (int)IMAGO_OK;
+  };
+  if (c->d_uoff.alloc(nu * c->npt, st) || c->d_rad.alloc(nu, st)) return none();
   int rc = launch_list_count(c->sys, w, margin, c->d_uoff.p, c->d_rad.p, c->d_queue.p, st);
   if (rc) return rc;
   unsigned long long total = 0;
   IMAGO_CUDA(cudaMemcpyAsync(&total, c->d_queue.p, sizeof total, cudaMemcpyDeviceToHost, st));
   IMAGO_CUDA(cudaStreamSynchronize(st));
-  if (total * sizeof(ImageRef) > kMaxImageListBytes ||
+  if (total * sizeof(ImageRef) > limit - ranges ||
       c->d_ulist.alloc(std::max<size_t>(total, 1), st))
-    return IMAGO_OK;
+    return none();
   w.uoff = c->d_uoff.p;
   w.ulist = c->d_ulist.p;
-  return launch_list_fill(c->sys, w, margin, c->d_rad.p, c->d_ulist.p, st);
+  rc = launch_list_fill(c->sys, w, margin, c->d_rad.p, c->d_ulist.p, st);
+  c->d_rad.release(st);
+  return rc;
 }
 
 int upload(imago_ctx *c) {
@@ -1427,7 +1447,7 @@ void tune_apply(imago_ctx *c) {
 // runs (a profiler's serialised replays distort the trial timings): a
 // comma-separated list of bloch=32|48|64, sched=per_class|queue|pairs,
 // ortho=per_item|piped, contract=4|8; lists=off does without the image
-// lists (build_lists).  Unknown entries are ignored.
+// lists, lists=<MiB> bounds them (build_lists).  Unknown entries are ignored.
 void tune_from_env(imago_ctx *c) {
   const char *env = std::getenv("IMAGO_TUNING");
   if (!env) return;
