@@ -2342,18 +2342,19 @@ int imago_batch_create(int n, const imago_system *systems,
   co.device = b->device;
   co.outputs_on_device = 1;
   co.scratch_bytes = opts ? opts->scratch_bytes : 0;
-  if (co.scratch_bytes == 0) {
-    // every cell keeps its scratch for the graph: a third of free memory
-    // shared out over the cells
-    size_t fr = 0, tot = 0;
-    cudaMemGetInfo(&fr, &tot);
-    co.scratch_bytes = std::max<size_t>(fr / 3 / (size_t)n, 1);
-  }
   int rc = IMAGO_OK;
   for (int i = 0; i < n && !rc; ++i) {
     imago_ctx *c = nullptr;
     rc = imago_intg_create(&systems[i], &co, &c);
     if (!rc) b->cells.push_back(c);
+  }
+  if (co.scratch_bytes == 0) {
+    // every cell keeps its scratch for the graph: a third of the memory their
+    // tables and image lists leave free, shared out over the cells
+    size_t fr = 0, tot = 0;
+    cudaMemGetInfo(&fr, &tot);
+    for (imago_ctx *c : b->cells)
+      c->scratch_bytes = std::max<size_t>(fr / 3 / (size_t)n, 1);
   }
   if (!rc) {
     if (opts && opts->stream) {
