@@ -251,13 +251,24 @@ __device__ __noinline__ void prim3c_item_rt(const DevSys &s, const DevWork &w, i
   hermite_to_sh_rt(la, lb, q.A, q.B, q.a1, q.a2, pref, Q, out, add ? out : nullptr);
 }
 
+// Every f class in one launch, costliest first: cta[c] is the first CTA of
+// the c-th class.  A cell's f classes are a few CTAs each and last as long as
+// their longest thread, so in turn their times add up (two atoms with f
+// functions, nuclear term: 6.3 ms one class after another, 3.7 together).
+struct RtClasses {
+  int ncls;
+  int la[7], lb[7], beg[7], n[7], cta[8];
+};
+
 template <bool NUC>
 __global__ void __launch_bounds__(128)
-    k_prim3c_rt(DevSys s, DevWork w, int beg, int n, const Term3c *terms,
-                int nterm, int la, int lb, double *blk, bool add) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= (long long)n * nterm) return;
-  prim3c_item_rt<NUC>(s, w, beg, n, terms, la, lb, blk, g, add);
+    k_prim3c_rt(DevSys s, DevWork w, RtClasses rc, const Term3c *terms, int nterm, double *blk,
+                bool add) {
+  int c = 0;
+  while ((int)blockIdx.x >= rc.cta[c + 1]) ++c;
+  const long long g = (long long)((int)blockIdx.x - rc.cta[c]) * blockDim.x + threadIdx.x;
+  if (g >= (long long)rc.n[c] * nterm) return;
+  prim3c_item_rt<NUC>(s, w, rc.beg[c], rc.n[c], terms, rc.la[c], rc.lb[c], blk, g, add);
 }
 
 // ------------------------------------------------------- work queue --
@@ -560,19 +571,25 @@ int launch_prim3c(const DevSys &s, const DevWork &w, const int *cls_beg,
 int launch_prim3c_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
                      const Term3c *terms_dev, int nterm, bool nuclear, double *blk,
                      cudaStream_t st, bool add) {
-  for (int c = 0; c < 16; ++c) {
-    const int la = c / 4, lb = c % 4;
-    if (la < 3 && lb < 3) continue;
-    const int beg = cls_beg[c], n = cls_beg[c + 1] - beg;
-    if (n <= 0 || nterm <= 0) continue;
-    const unsigned grid = (unsigned)(((long long)n * nterm + 127) / 128);
-    if (nuclear)
-      k_prim3c_rt<true><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, la, lb, blk, add);
-    else
-      k_prim3c_rt<false><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, la, lb, blk,
-                                               false);
-    IMAGO_CUDA(cudaGetLastError());
+  if (nterm <= 0) return IMAGO_OK;
+  RtClasses rc{};
+  for (int c : {15, 11, 14, 7, 13, 3, 12}) {  // la * 4 + lb, la or lb = 3
+    const int n = cls_beg[c + 1] - cls_beg[c];
+    if (n <= 0) continue;
+    const int i = rc.ncls++;
+    rc.la[i] = c / 4;
+    rc.lb[i] = c % 4;
+    rc.beg[i] = cls_beg[c];
+    rc.n[i] = n;
+    rc.cta[i + 1] = rc.cta[i] + (int)(((long long)n * nterm + 127) / 128);
   }
+  if (rc.ncls == 0) return IMAGO_OK;
+  const unsigned grid = (unsigned)rc.cta[rc.ncls];
+  if (nuclear)
+    k_prim3c_rt<true><<<grid, 128, 0, st>>>(s, w, rc, terms_dev, nterm, blk, add);
+  else
+    k_prim3c_rt<false><<<grid, 128, 0, st>>>(s, w, rc, terms_dev, nterm, blk, false);
+  IMAGO_CUDA(cudaGetLastError());
   return IMAGO_OK;
 }
 
