@@ -196,8 +196,8 @@ struct imago_ctx {
   float bloch_ms[kNumBlochWidths] = {};
   int cls_beg[17];
   // three-centre schedule: per-class launches (0), one persistent launch
-  // fed by a work queue (1), or per-class launches with two EP terms of a
-  // type per thread (2); mode -1 measures all on the first EP build
+  // fed by a work queue (1), or several EP terms of a type per thread (2);
+  // mode -1 measures all on the first EP build
   int sched_mode = -1, sched = 0;
   bool sched_tuned = false;
   float sched_ms[kNumSchedules] = {};
@@ -1334,12 +1334,6 @@ void mark(imago_ctx *c) {
   if (e) cudaEventRecord(e, c->cur());
 }
 
-int class_launches(const imago_ctx *c) {
-  int n = 0;
-  for (int k = 0; k < 16; ++k) n += c->cls_beg[k + 1] > c->cls_beg[k];
-  return n;
-}
-
 // The tensor-core phase sum's column-tile width is picked by measurement:
 // on the context's first phase sum each width runs once on the real blocks
 // (every run writes the same values) and the fastest is kept.  Narrower
@@ -1370,7 +1364,6 @@ int tune_bloch(imago_ctx *c, int nterm) {
   for (auto &x : e) cudaEventDestroy(x);
   cudaGetLastError();
   set_bloch_width(c, best);
-  c->launches += kNumBlochWidths;
   c->bloch_tuned = !rc;
   return rc;
 }
@@ -1510,7 +1503,6 @@ int tune_contract(imago_ctx *c, const DevSys &s, const DevWork &w, int nterm,
   for (auto &x : e) cudaEventDestroy(x);
   cudaGetLastError();
   c->contract_tpc = (!rc && c->contract_ms[1] < c->contract_ms[0]) ? 8 : 4;
-  c->launches += 2;
   c->contract_tuned = !rc;
   if (!rc) tune_store(c);
   return rc;
@@ -1560,7 +1552,6 @@ int tune_sched(imago_ctx *c, const DevSys &s, const DevWork &w, const Term3c *te
   for (int k = 1; k < kNumSchedules && !rc; ++k)
     if (c->sched_ms[k] < (best ? c->sched_ms[best] : kSchedMargin * c->sched_ms[0])) best = k;
   c->sched = best;
-  c->launches += 2 * class_launches(c) + 1;
   c->sched_tuned = !rc;
   if (!rc) tune_store(c);
   return rc;
@@ -1590,7 +1581,6 @@ int tune_ortho(imago_ctx *c, const DevSys &s, int nterm, double *packed_dev,
   for (auto &x : e) cudaEventDestroy(x);
   cudaGetLastError();
   c->ortho = (!rc && c->ortho_ms[1] < c->ortho_ms[0]) ? 1 : 0;
-  c->launches += 2;
   c->ortho_tuned = !rc;
   if (!rc) tune_store(c);
   return rc;
@@ -1610,7 +1600,6 @@ int run_build(imago_ctx *c, Kind kind, int term0, int nterm,
   }
   const DevSys &s = sv;
   const DevWork &w = c->work;
-  c->launches += class_launches(c) + 2 + (c->core_dim > 0 ? 2 : 1);
   mark(c);
   if (kind == KIND_OL || kind == KIND_KE || kind == KIND_MV) {
     const int op = kind == KIND_OL   ? kPrim2cOverlap
@@ -1751,7 +1740,6 @@ int do_ol(imago_ctx *c, double *packed, double *cv_re, double *cv_im) {
       if (!im) im = scratch;
     }
     if ((rc = launch_split_cv(c->sys, c->s_cv.p, re, im, c->cur()))) return rc;
-    c->launches += 1;
     if (!c->outputs_on_device) {
       if ((rc = copy_out(c, cv_re, re, ncv))) return rc;
       if ((rc = copy_out(c, cv_im, im, ncv))) return rc;
@@ -1817,7 +1805,6 @@ int do_kov(imago_ctx *c, const double *dk, double *re, double *im) {
   s.nk = c->nk;
   s.kout = c->d_kout.p + c->nka;
   const DevWork &w = c->work;
-  c->launches += class_launches(c) + 2 + (c->core_dim > 0 ? 2 : 1) + (c->npair > 0 ? 1 : 0);
   mark(c);
   if ((rc = launch_prim_kov(s, w, c->cls_beg, q, S.blk.p, st))) return rc;
   mark(c);
@@ -1908,9 +1895,6 @@ int do_ham(imago_ctx *c, int spin, const double *coeffs, bool rel, double *packe
   if (c->pot_dim > 0)
     IMAGO_CUDA(cudaMemcpyAsync(c->ham_w.p, coeffs, sizeof(double) * c->pot_dim * spin,
                                cudaMemcpyHostToDevice, st));
-  const int nchunk = fused || c->pot_dim == 0 ? 0 : (c->pot_dim + chunk - 1) / chunk;
-  c->launches += class_launches(c) * (2 + (rel ? 1 : 0) + (fused ? 1 : nchunk)) + nchunk + 3 +
-                 (c->core_dim > 0 ? 2 : 1);
   mark(c);
   // the kinetic, mass-velocity (written negatively, the sign the reference
   // subtracts it with) and nuclear blocks, each added as it is stored
@@ -2025,6 +2009,7 @@ int enqueue_build(imago_ctx *c, unsigned which, const imago_out *out,
                   int ep_first = 0, int ep_count = -1) {
   IMAGO_CUDA(cudaEventRecord(c->kfork, c->stream));
   c->ol_in_call = (which & IMAGO_OL) != 0;
+  const long long l0 = launch_count;
   int rc = IMAGO_OK;
   // stage times are kept for the four kinds of the lanes; MV follows KE on
   // the kinetic lane and is not timed
@@ -2055,6 +2040,7 @@ int enqueue_build(imago_ctx *c, unsigned which, const imago_out *out,
   if (!rc && (which & IMAGO_EP))
     rc = run(KIND_EP, [&] { return do_ep(c, out->ep_packed, ep_first, ep_count); });
   c->ol_in_call = false;
+  c->launches += launch_count - l0;
   return rc;
 }
 
@@ -2092,7 +2078,9 @@ int on_lane(imago_ctx *c, int lane, Body body) {
   if (cudaEventRecord(c->kfork, c->stream) != cudaSuccess ||
       cudaStreamWaitEvent(ks, c->kfork, 0) != cudaSuccess)
     rc = IMAGO_ERR_CUDA;
+  const long long l0 = launch_count;
   if (!rc) rc = body();
+  c->launches += launch_count - l0;
   if (cudaEventRecord(c->kjoin[lane], ks) != cudaSuccess ||
       cudaStreamWaitEvent(c->stream, c->kjoin[lane], 0) != cudaSuccess)
     rc = rc ? rc : IMAGO_ERR_CUDA;

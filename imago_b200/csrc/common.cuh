@@ -92,3 +92,15 @@ __host__ __device__ constexpr int herm_index(int t, int u, int v) {
       return IMAGO_ERR_CUDA;                                               \
     }                                                                      \
   } while (0)
+
+// After each kernel launch: its error, and the count of launches that the
+// calling thread has made, from which a call's own are taken
+// (imago_intg_kernel_stats).
+namespace imago {
+inline thread_local long long launch_count = 0;
+}
+#define IMAGO_LAUNCHED()             \
+  do {                               \
+    ++imago::launch_count;           \
+    IMAGO_CUDA(cudaGetLastError());  \
+  } while (0)

@@ -217,7 +217,7 @@ static int contract_one(const DevSys &s, const DevWork &w, int nterm, const doub
       1, std::min<long long>(ntg, (kContractCtas + w.nunits - 1) / w.nunits));
   k_contract<T><<<(unsigned)((long long)w.nunits * gsplit), kContractThreads, bytes, st>>>(
       s, w, nterm, gsplit, blk, M);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 

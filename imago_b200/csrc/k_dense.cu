@@ -423,7 +423,7 @@ int launch_bloch(const DevSys &s, const DevWork &w, int nterm, const double *M,
       bloch_small<4, 1, false>(s, w, nterm, M, vv, cv, cc, st);
     else
       bloch_small<8, 1, false>(s, w, nterm, M, vv, cv, cc, st);
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
     return IMAGO_OK;
   }
   dim3 grid(w.nbtile_w, (s.nk + kBK - 1) / kBK, nterm);
@@ -441,7 +441,7 @@ int launch_bloch(const DevSys &s, const DevWork &w, int nterm, const double *M,
     default:
       return IMAGO_ERR_INVALID;
   }
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -720,7 +720,7 @@ static int ortho_y(const DevSys &s, int nterm, const double2 *cv, const double2 
   const int tc = (s.core_dim + TILE - 1) / TILE, tv = (s.vale_dim + TILE - 1) / TILE;
   k_ortho_y<REAL, TILE><<<dim3(tc * tv, s.nk, nterm), O::threads, O::smem, st>>>(s, cv, cc, s_cv, y,
                                                                                ycc);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -736,7 +736,7 @@ static int ortho_w(const DevSys &s, int nterm, const double2 *vv, const double2 
   const int tiles = FULL ? tv * tv : tv * (tv + 1) / 2;
   k_ortho_w<REAL, FULL, TILE><<<dim3(tiles, s.nk, nterm), O::threads, O::smem, st>>>(
       s, vv, y, x2, s_cv, packed, general, im);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -1336,7 +1336,7 @@ __global__ void k_wait_check(int *flag, unsigned long long limit_ns) {
 int launch_wait_check(int *flag, double limit_ms, cudaStream_t st) {
   const unsigned long long ns = (unsigned long long)(limit_ms * 1e6);
   k_wait_check<<<1, 128, 0, st>>>(flag, ns);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -1408,7 +1408,7 @@ int launch_ortho_pipe(const DevSys &s, int nterm, const double2 *vv, const doubl
     k_ortho_pipe<true><<<grid, kFThreads, smem, st>>>(s, mx, mc, ms, vv, nterm, packed);
   else
     k_ortho_pipe<false><<<grid, kFThreads, smem, st>>>(s, mx, mc, ms, vv, nterm, packed);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   *launched = true;
   return IMAGO_OK;
 }
@@ -1442,7 +1442,7 @@ int launch_ortho(const DevSys &s, int nterm, const double2 *vv,
     const long long np = (long long)V * (V + 1) / 2;
     dim3 g((unsigned)std::min<long long>((np + 255) / 256, 128), s.nk, nterm);
     k_pack_plain<<<g, 256, 0, st>>>(s, vv, packed);
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
     return IMAGO_OK;
   }
   if (pipe) {
@@ -1468,7 +1468,7 @@ int launch_ortho(const DevSys &s, int nterm, const double2 *vv,
     else
       k_ortho_fused<false><<<dim3(s.nk, nterm), kFThreads, smem, st>>>(s, vv, cv, cc,
                                                                       s_cv, packed);
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
     return IMAGO_OK;
   }
   if (s.real_k)
@@ -1534,13 +1534,13 @@ int launch_bloch_kov(const DevSys &s, const DevWork &w, const double *M, double2
       default:
         return IMAGO_ERR_INVALID;
     }
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
     return IMAGO_OK;
   }
   constexpr int kPerBlock = 256 / kBlochCols;
   dim3 grid(w.nbtile, (s.nk + kPerBlock - 1) / kPerBlock, 3);
   k_bloch_kov<<<grid, 256, 0, st>>>(s, w, M, vv, cv, cc);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -1564,7 +1564,7 @@ int launch_ortho_full(const DevSys &s, const double2 *vv, const double2 *cv,
     const long long n = 3LL * s.nk * V * V;
     k_vv_planes<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
         s, n, vv, re, im);
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
     return IMAGO_OK;
   }
   return ortho_tiled<false, true>(s, 3, vv, cv, cc, s_cv, y, 1.0, cv, re, true, im, st);
@@ -1620,7 +1620,7 @@ int launch_conj_cv(const DevSys &s, int npair, double2 *cv, cudaStream_t st) {
   if (n == 0) return IMAGO_OK;
   k_conj_cv<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(
       n, cv, cv + s.nk * per);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -1630,7 +1630,7 @@ int launch_split_cv(const DevSys &s, const double2 *cv, double *re, double *im,
   if (n == 0) return IMAGO_OK;
   k_split_cv<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(
       s, (long long)s.vale_dim * s.core_dim, cv, re, im);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -1660,7 +1660,7 @@ int launch_block_axpy(const double *blk, int nterm, long long n, const double *w
   if (spin < 1 || spin > 2) return IMAGO_ERR_INVALID;
   k_block_axpy<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
       blk, nterm, n, w, wstride, spin, H);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -1682,7 +1682,7 @@ __global__ void k_phase(DevSys s, double2 *phase) {
 int launch_phase(const DevSys &s, double2 *phase, cudaStream_t st) {
   const long long n = (long long)s.ncell * s.nkt;
   k_phase<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(s, phase);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 

@@ -134,7 +134,7 @@ static int ham_one(const DevSys &s, const DevWork &w, int beg, int n, const Term
     k_prim3c_ham<LA, LB, 4, SPIN, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
   else
     k_prim3c_ham<LA, LB, 1, SPIN, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms, nterm, coef, H);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 

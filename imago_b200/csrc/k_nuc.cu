@@ -87,7 +87,7 @@ static int nuc_one(const DevSys &s, const DevWork &w, int beg, int n, int lanes,
     case 2: k_prim3c_nuc<LA, LB, 2, false><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add); break;
     default: k_prim3c_nuc<LA, LB, 1, false><<<grid, 128, 0, st>>>(s, w, beg, n, blk, add);
   }
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 

@@ -327,7 +327,7 @@ static int prim2c_one(const DevSys &s, const DevWork &w, int beg, int end,
     k_prim2c<LA, LB, true><<<(n + tb - 1) / tb, tb, 0, st>>>(s, w, beg, end, blk);
   else
     k_prim2c<LA, LB, false><<<(n + tb - 1) / tb, tb, 0, st>>>(s, w, beg, end, blk);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -345,7 +345,7 @@ int launch_prim3c_count(const DevSys &s, const DevWork &w, const int *cls_beg,
       else                                                                          \
         k_prim3c_count<a, b, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev,  \
                                                           nterm, count16 + a * 4 + b); \
-      IMAGO_CUDA(cudaGetLastError());                                               \
+      IMAGO_LAUNCHED();                                                             \
     }                                                                               \
   }
   IMAGO_FOR_SPD_CLASSES(IMAGO_PC)
@@ -363,7 +363,7 @@ int launch_prim2c(const DevSys &s, const DevWork &w, const int *cls_beg,
     const int beg = cls_beg[a * 4 + b], n = cls_beg[a * 4 + b + 1] - beg;    \
     if (n > 0) {                                                             \
       k_prim_mv<a, b><<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, beg + n, blk, add); \
-      IMAGO_CUDA(cudaGetLastError());                                        \
+      IMAGO_LAUNCHED();                                                      \
     }                                                                        \
   }
     IMAGO_FOR_SPD_CLASSES(IMAGO_MV)
@@ -374,7 +374,7 @@ int launch_prim2c(const DevSys &s, const DevWork &w, const int *cls_beg,
       const int beg = cls_beg[c], n = cls_beg[c + 1] - beg;
       if (n <= 0) continue;
       k_prim_mv_rt<<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, beg + n, la, lb, blk, add);
-      IMAGO_CUDA(cudaGetLastError());
+      IMAGO_LAUNCHED();
     }
     return IMAGO_OK;
   }
@@ -394,7 +394,7 @@ int launch_prim2c(const DevSys &s, const DevWork &w, const int *cls_beg,
       k_prim2c_rt<true><<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, end, la, lb, blk);
     else
       k_prim2c_rt<false><<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, end, la, lb, blk);
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
   }
   return rc;
 }
@@ -413,7 +413,7 @@ int launch_prim2c_vec(const DevSys &s, const DevWork &w, const int *cls_beg,
         k_prim_vec<a, b, true><<<grid, 128, 0, st>>>(s, w, beg, beg + n, c3, blk);  \
       else                                                                    \
         k_prim_vec<a, b, false><<<grid, 128, 0, st>>>(s, w, beg, beg + n, c3, blk); \
-      IMAGO_CUDA(cudaGetLastError());                                         \
+      IMAGO_LAUNCHED();                                                       \
     }                                                                         \
   }
   IMAGO_FOR_SPD_CLASSES(IMAGO_PV)
@@ -428,7 +428,7 @@ int launch_prim2c_vec(const DevSys &s, const DevWork &w, const int *cls_beg,
       k_prim_vec_rt<true><<<grid, 128, 0, st>>>(s, w, beg, beg + n, la, lb, c3, blk);
     else
       k_prim_vec_rt<false><<<grid, 128, 0, st>>>(s, w, beg, beg + n, la, lb, c3, blk);
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
   }
   return IMAGO_OK;
 }
@@ -445,7 +445,7 @@ int launch_prim3c_ham_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
       k_prim3c_ham_rt<<<(n + 127) / 128, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm,
                                                        coef + (size_t)h * nterm, la, lb,
                                                        H + h * w.blk_total);
-      IMAGO_CUDA(cudaGetLastError());
+      IMAGO_LAUNCHED();
     }
   }
   return IMAGO_OK;
@@ -495,7 +495,7 @@ int launch_prim_kov(const DevSys &s, const DevWork &w, const int *cls_beg,
       default:
         k_prim_kov<<<grid, 128, 0, st>>>(s, w, beg, beg + n, c / 4, c % 4, dk, blk);
     }
-    IMAGO_CUDA(cudaGetLastError());
+    IMAGO_LAUNCHED();
   }
   return IMAGO_OK;
 }
@@ -532,7 +532,7 @@ int launch_prim3c_queue(const DevSys &s, const DevWork &w, const int *cls_beg,
   const long long need = (off + 127) / 128;
   const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(ctas, need));
   k_prim3c_queue<<<grid, 128, 0, st>>>(s, w, qc, terms_dev, blk, counter);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -560,7 +560,7 @@ int launch_prim3c(const DevSys &s, const DevWork &w, const int *cls_beg,
       else                                                                          \
         k_prim3c<a, b, false><<<grid, 128, 0, st>>>(s, w, beg, n, terms_dev, nterm, \
                                                     blk);                           \
-      IMAGO_CUDA(cudaGetLastError());                                               \
+      IMAGO_LAUNCHED();                                                             \
     }                                                                               \
   }
   IMAGO_FOR_SPD_CLASSES(IMAGO_P3)
@@ -589,7 +589,7 @@ int launch_prim3c_rt(const DevSys &s, const DevWork &w, const int *cls_beg,
     k_prim3c_rt<true><<<grid, 128, 0, st>>>(s, w, rc, terms_dev, nterm, blk, add);
   else
     k_prim3c_rt<false><<<grid, 128, 0, st>>>(s, w, rc, terms_dev, nterm, blk, false);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 

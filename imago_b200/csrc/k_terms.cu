@@ -195,7 +195,7 @@ int launch_list_count(const DevSys &s, const DevWork &w, float margin, int2 *uof
   if (w.nunits == 0) return IMAGO_OK;
   const int grid = std::min((w.nunits + kListWarps - 1) / kListWarps, 148 * 8);
   k_list_count<<<grid, 32 * kListWarps, 0, st>>>(s, w, margin, uoff, rad, cursor);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -204,7 +204,7 @@ int launch_list_fill(const DevSys &s, const DevWork &w, float margin, const floa
   if (w.nunits == 0) return IMAGO_OK;
   const int grid = std::min((w.nunits + kFillWarps - 1) / kFillWarps, 148 * 12);
   k_list_fill<<<grid, 32 * kFillWarps, 0, st>>>(s, w, margin, rad, list);
-  IMAGO_CUDA(cudaGetLastError());
+  IMAGO_LAUNCHED();
   return IMAGO_OK;
 }
 
@@ -413,7 +413,7 @@ int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
       if (cc.ncls) {
         k_prim3c_terms_all<<<cc.cta[cc.ncls], kTermThreads, 0, st>>>(s, w, cc, terms_dev + from,
                                                                     tg, b);
-        IMAGO_CUDA(cudaGetLastError());
+        IMAGO_LAUNCHED();
       }
       from = next;
       continue;
@@ -424,7 +424,7 @@ int launch_prim3c_terms(const DevSys &s, const DevWork &w, const int *cls_beg,
     if (n > 0) {                                                                          \
       const unsigned grid = (unsigned)(((long long)n * tg.n + kTermThreads - 1) / kTermThreads); \
       k_prim3c_terms<a, c><<<grid, kTermThreads, 0, st>>>(s, w, beg, n, terms_dev + from, tg, b); \
-      IMAGO_CUDA(cudaGetLastError());                                                     \
+      IMAGO_LAUNCHED();                                                                   \
     }                                                                                     \
   }
     IMAGO_PT(2, 2) IMAGO_PT(1, 2) IMAGO_PT(2, 1) IMAGO_PT(1, 1) IMAGO_PT(0, 2) IMAGO_PT(2, 0)
