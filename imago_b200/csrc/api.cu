@@ -219,10 +219,9 @@ struct imago_ctx {
   DBuf<int> d_type_nalpha, d_type_alpha_off, d_type_nstates, d_type_nvale,
       d_type_state_off, d_type_basis_off, d_type_screen, d_alpha_cls,
       d_state_lm, d_site_type, d_site_cum_vale, d_site_cum_core,
-      d_ptype_alpha_off, d_ptype_nalpha, d_ptype_first_site, d_ptype_mult,
-      d_ptype_screen, d_sp_by_cls;
+      d_ptype_alpha_off, d_ptype_screen, d_sp_by_cls;
   DBuf<double> d_alpha, d_basis, d_site_pos, d_ptype_z, d_ptype_nucalpha,
-      d_palpha, d_cell, d_csize, d_kxyz;
+      d_palpha, d_cell, d_kxyz;
   DBuf<double2> d_phase;
   DBuf<int2> d_kout;
   DBuf<DPair> d_pairs;
@@ -301,12 +300,11 @@ struct imago_ctx {
                     &d_type_nvale, &d_type_state_off, &d_type_basis_off,
                     &d_type_screen, &d_alpha_cls, &d_state_lm, &d_site_type,
                     &d_site_cum_vale, &d_site_cum_core, &d_ptype_alpha_off,
-                    &d_ptype_nalpha, &d_ptype_first_site, &d_ptype_mult,
                     &d_ptype_screen, &d_sp_by_cls})
       b->release(st);
     for (auto *b : {&d_alpha, &d_basis, &d_site_pos, &d_ptype_z,
                     &d_ptype_nucalpha, &d_palpha, &d_cell,
-                    &d_csize, &d_kxyz, &out_stage, &ham_blk, &ham_w, &ham_out, &vec_out})
+                    &d_kxyz, &out_stage, &ham_blk, &ham_w, &ham_out, &vec_out})
       b->release(st);
     for (auto &sc : scr) {
       sc.blk.release(st);
@@ -1153,13 +1151,10 @@ int upload(imago_ctx *c) {
     lm.insert(lm.end(), t.lm.begin(), t.lm.end());
     basis.insert(basis.end(), t.basis.begin(), t.basis.end());
   }
-  std::vector<int> paoff, pn, pfirst, pmult;
+  std::vector<int> paoff;
   std::vector<double> pz, pnuc, palpha;
   for (const HPType &p : c->ptypes) {
     paoff.push_back((int)palpha.size());
-    pn.push_back((int)p.alphas.size());
-    pfirst.push_back(p.first_site < 0 ? 0 : p.first_site);
-    pmult.push_back(p.mult);
     pz.push_back(p.z);
     pnuc.push_back(p.nucalpha);
     palpha.insert(palpha.end(), p.alphas.begin(), p.alphas.end());
@@ -1182,9 +1177,8 @@ int upload(imago_ctx *c) {
   UP(d_alpha, alpha) UP(d_basis, basis) UP(d_site_pos, c->site_pos)
   UP(d_site_type, c->site_type) UP(d_site_cum_vale, c->cum_vale)
   UP(d_site_cum_core, c->cum_core) UP(d_ptype_z, pz) UP(d_ptype_nucalpha, pnuc)
-  UP(d_palpha, palpha) UP(d_ptype_alpha_off, paoff) UP(d_ptype_nalpha, pn)
-  UP(d_ptype_first_site, pfirst) UP(d_ptype_mult, pmult)
-  UP(d_ptype_screen, c->ptype_screen) UP(d_cell, c->cells) UP(d_csize, c->csize)
+  UP(d_palpha, palpha) UP(d_ptype_alpha_off, paoff)
+  UP(d_ptype_screen, c->ptype_screen) UP(d_cell, c->cells)
   UP(d_kxyz, c->kxyz) UP(d_pairs, c->pairs) UP(d_units, c->units)
   UP(d_sps, c->sps) UP(d_sp_by_cls, c->sp_by_cls) UP(d_terms, c->ep_terms)
   UP(d_btile, c->btile) UP(d_btile_w, c->btile_w) UP(d_kout, c->kout)
@@ -1206,11 +1200,10 @@ int upload(imago_ctx *c) {
   if ((rc = c->d_phase.alloc((size_t)c->ncell * c->nk, st))) return rc;
 
   DevSys &s = c->sys;
-  s.nt = c->nt; s.ns = c->ns; s.npt = c->npt; s.nps = c->nps;
+  s.nt = c->nt; s.ns = c->ns; s.npt = c->npt;
   s.nk = c->nka; s.nkt = c->nk; s.kout = c->d_kout.p;
   s.ncell = c->ncell; s.vale_dim = c->vale_dim; s.core_dim = c->core_dim;
   s.T = c->T;
-  std::memcpy(s.rv, c->rv, sizeof s.rv);
   std::memcpy(s.inv, c->inv, sizeof s.inv);
   s.a3_min = tab.a3_min;
   s.bounded = tab.bounded;
@@ -1241,9 +1234,8 @@ int upload(imago_ctx *c) {
   s.site_cum_vale = c->d_site_cum_vale.p; s.site_cum_core = c->d_site_cum_core.p;
   s.ptype_z = c->d_ptype_z.p; s.ptype_nucalpha = c->d_ptype_nucalpha.p;
   s.palpha = c->d_palpha.p; s.ptype_alpha_off = c->d_ptype_alpha_off.p;
-  s.ptype_nalpha = c->d_ptype_nalpha.p; s.ptype_first_site = c->d_ptype_first_site.p;
-  s.ptype_mult = c->d_ptype_mult.p; s.ptype_screen = c->d_ptype_screen.p;
-  s.cell = c->d_cell.p; s.csize = c->d_csize.p; s.kxyz = c->d_kxyz.p;
+  s.ptype_screen = c->d_ptype_screen.p;
+  s.cell = c->d_cell.p; s.kxyz = c->d_kxyz.p;
   s.phase = c->d_phase.p;
   s.flag = c->d_flag.p;
   DevWork &w = c->work;

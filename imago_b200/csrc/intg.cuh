@@ -10,7 +10,7 @@ namespace imago {
 
 // Everything the kernels read about the system, as device pointers.
 struct DevSys {
-  int nt, ns, npt, nps, ncell;
+  int nt, ns, npt, ncell;
   // k-points the stages compute (nk) and the caller's (nkt): M real gives
   // H(-k) = conj H(k), so of two k-points that are each other's negative up
   // to a reciprocal lattice vector only one is summed and orthogonalised.
@@ -21,7 +21,6 @@ struct DevSys {
   const int2 *kout;
   int vale_dim, core_dim;
   double T;            // logBasisFnThresh = -ln(basisFnConvg)
-  double rv[9];        // realVectors [abc*3 + xyz]
   double inv[9];       // invRealVectors [abc*3 + xyz]
   // every k-point is Gamma: all phases are exactly 1, every matrix is real,
   // and the orthogonalisation runs on the real parts only
@@ -41,8 +40,7 @@ struct DevSys {
   const int *site_type, *site_cum_vale, *site_cum_core;
   // potential types and sites
   const double *ptype_z, *ptype_nucalpha, *palpha;
-  const int *ptype_alpha_off, *ptype_nalpha, *ptype_first_site, *ptype_mult,
-      *ptype_screen;
+  const int *ptype_alpha_off, *ptype_screen;
   // 1 where the type's exponents and its screening exponents ascend, so
   // that the screening radius falls from term to term
   const int *ptype_ascends;
@@ -60,7 +58,6 @@ struct DevSys {
   const unsigned char *listed;
   // lattice cells sorted by |R|^2, k-points, phase table
   const double *cell;     // [n*3]
-  const double *csize;    // [n]
   const double *kxyz;     // [nkt*3], computed k-points first
   const double2 *phase;   // [cell * nkt + k]  exp(i k.R)
   // device status word: a kernel whose bounded wait ran out records
@@ -187,9 +184,6 @@ int launch_ortho_full(const DevSys &s, const double2 *vv, const double2 *cv,
 int launch_prim2c_vec(const DevSys &s, const DevWork &w, const int *cls_beg,
                       bool dipole, const double center[3], double *blk,
                       cudaStream_t st);
-// The classes of one three-centre build in work-queue order: class code
-// la * 4 + lb, first entry of its shell-pair list, count, and the first
-// queue item of each class (off[ncls] is the total).
 // EP terms that one thread evaluates in turn: group g is the count[g]
 // terms first[g], first[g] + stride, ... of a launch's term list, all of
 // one potential type.
@@ -200,6 +194,9 @@ struct TermGroups {
   unsigned short count[kMaxTermGroups];
 };
 
+// The classes of one three-centre build in work-queue order: class code
+// la * 4 + lb, first entry of its shell-pair list, count, and the first
+// queue item of each class (off[ncls] is the total).
 struct Prim3cQueue {
   int ncls;
   int cls[16], beg[16], n[16];
