@@ -63,14 +63,14 @@ __global__ void k_secular(int V, long long np, int nk, int pot_dim,
   }
 }
 
-// Hashes of each k-point's H and S, and of their conjugates, by which the
-// host finds the k-points whose problem may be another's conjugate (k and -k
-// of an integral build: the same values with the imaginary parts negated);
-// k_conj_check then compares the matrices themselves.  Sums of mixed bit
-// patterns modulo 2^64 over the upper triangle, so the order of the additions
-// does not matter; H and S apart.  HBM-bound: one pass over what k_secular
-// wrote (Si8, 512 k: 0.18 GB).  mix64 and the constant below are the
-// finaliser and the increment of SplitMix64 (Steele, Lea and Flood 2014).
+// Hashes of each k-point's H and of its conjugate, by which the host finds
+// the k-points whose problem may be another's conjugate (k and -k of an
+// integral build: the same values with the imaginary parts negated);
+// k_conj_check then compares the matrices themselves, S among them.  Sums of
+// mixed bit patterns modulo 2^64 over the upper triangle, so the order of the
+// additions does not matter.  HBM-bound: one pass over the H that k_secular
+// wrote (Si8, 512 k: 0.09 GB).  mix64 and the constant below are the finaliser
+// and the increment of SplitMix64 (Steele, Lea and Flood 2014).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
   x ^= x >> 30;
   x *= 0xbf58476d1ce4e5b9ull;
@@ -80,28 +80,28 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
 }
 
 __global__ void __launch_bounds__(256)
-    k_conj_hash(int V, const double2 *h, const double2 *s, unsigned long long *out) {
+    k_conj_hash(int V, const double2 *h, unsigned long long *out) {
   const int k = blockIdx.x;
   const long long base = (long long)k * V * V;
-  unsigned long long sum[4] = {0, 0, 0, 0};  // H, conj H, S, conj S
+  unsigned long long own = 0, conj = 0;
   for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < V * V; e += gridDim.y * blockDim.x) {
     const int col = e / V, row = e - col * V;
     if (row > col) continue;
     const unsigned long long at = 0x9e3779b97f4a7c15ull * (unsigned)(e + 1);
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const double2 x = (m ? s : h)[base + e];
-      // + 0.0: -0 and +0 are one value
-      const unsigned long long re = mix64((unsigned long long)__double_as_longlong(x.x + 0.0) + at);
-      sum[2 * m] += mix64(re + (unsigned long long)__double_as_longlong(x.y + 0.0));
-      sum[2 * m + 1] += mix64(re + (unsigned long long)__double_as_longlong(0.0 - x.y));
-    }
+    const double2 x = h[base + e];
+    // + 0.0: -0 and +0 are one value
+    const unsigned long long re = mix64((unsigned long long)__double_as_longlong(x.x + 0.0) + at);
+    own += mix64(re + (unsigned long long)__double_as_longlong(x.y + 0.0));
+    conj += mix64(re + (unsigned long long)__double_as_longlong(0.0 - x.y));
   }
 #pragma unroll
-  for (int m = 0; m < 4; ++m) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out + 4 * k + m, sum[m]);
+  for (int o = 16; o > 0; o >>= 1) {
+    own += __shfl_xor_sync(0xffffffffu, own, o);
+    conj += __shfl_xor_sync(0xffffffffu, conj, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(out + 2 * k, own);
+    atomicAdd(out + 2 * k + 1, conj);
   }
 }
 
@@ -653,7 +653,7 @@ extern "C" int imago_secular_pairs(int n, int num_kpoints, const double *h_full,
   if (num_kpoints == 0) return IMAGO_OK;
   cudaStream_t st = (cudaStream_t)stream;
   // the hashes; then, in the same memory, the candidates and their verdicts
-  const size_t nk = (size_t)num_kpoints, bytes = sizeof(unsigned long long) * 4 * nk;
+  const size_t nk = (size_t)num_kpoints, bytes = sizeof(unsigned long long) * 2 * nk;
   void *d = nullptr;
   if (imago::pool_alloc(&d, bytes, st) != cudaSuccess) {
     cudaGetLastError();
@@ -661,33 +661,27 @@ extern "C" int imago_secular_pairs(int n, int num_kpoints, const double *h_full,
   }
   const double2 *h = reinterpret_cast<const double2 *>(h_full);
   const double2 *s = reinterpret_cast<const double2 *>(s_full);
-  std::vector<unsigned long long> hash(4 * nk);
+  std::vector<unsigned long long> hash(2 * nk);
   int rc = IMAGO_OK;
   const unsigned per = (unsigned)std::max(1, std::min(64, 148 * 8 / num_kpoints));
   if (cudaMemsetAsync(d, 0, bytes, st) != cudaSuccess) rc = IMAGO_ERR_CUDA;
   if (!rc) {
     imago::k_conj_hash<<<dim3(num_kpoints, per), 256, 0, st>>>(
-        n, h, s, static_cast<unsigned long long *>(d));
+        n, h, static_cast<unsigned long long *>(d));
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpyAsync(hash.data(), d, bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       rc = IMAGO_ERR_CUDA;
   }
   if (!rc) {
-    // a k-point's candidate is the first earlier one with its conjugate's
-    // hashes
+    // a k-point's candidate is the first with its conjugate's hash
     bool any = false;
-    std::unordered_multimap<unsigned long long, int> seen;
+    std::unordered_map<unsigned long long, int> seen;
     for (int k = 0; k < num_kpoints; ++k) {
-      const unsigned long long *x = &hash[4 * (size_t)k];
-      int first = -1;
-      const auto range = seen.equal_range(x[1]);
-      for (auto it = range.first; it != range.second; ++it)
-        if (hash[4 * (size_t)it->second + 2] == x[3] && (first < 0 || it->second < first))
-          first = it->second;
-      pair[k] = first < 0 ? k : first;
-      any |= first >= 0;
-      if (first < 0) seen.emplace(x[0], k);
+      const auto it = seen.find(hash[2 * (size_t)k + 1]);
+      pair[k] = it == seen.end() ? k : it->second;
+      if (pair[k] == k) seen.emplace(hash[2 * (size_t)k], k);
+      any |= pair[k] != k;
     }
     if (any) {
       int *cand = static_cast<int *>(d), *bad = cand + nk;

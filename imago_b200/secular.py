@@ -241,8 +241,8 @@ class _Conjugates:
     """The k-points whose H and S are an earlier k-point's conjugates, as k
     and -k of an integral build are (imago_secular_pairs, which compares the
     matrices themselves): their eigenvalues are the same and their vectors the
-    conjugates, so only `first` are solved.  Finding them takes 0.24 ms (n =
-    104, 512 k; 0.19 by their hashes alone), and below one matrix per SM a
+    conjugates, so only `first` are solved.  Finding them takes 0.23 ms (n =
+    104, 512 k; 0.19 without comparing the matrices), and below one matrix per SM a
     smaller batch is no faster, so it is tried for n > REDUCE_MAX_N or from
     PAIR_MIN rows in all.  One B200, eigensystems in ms with every k-point
     solved / with pairs: n = 104, 512 k 9.7 / 5.4, 216 k 4.70 / 3.09,

@@ -420,9 +420,9 @@ IMAGO_API int imago_hermitian_solver(int *mode);
 /* K-points whose secular problem is another's conjugate, H(k') = conj H(k)
  * and S(k') = conj S(k) value for value (k and -k of an integral build):
  * pair[k] (host, num_kpoints ints) is such a k-point before k, or k itself.
- * Candidates by hashes of h_full and s_full (device, [num_kpoints][n][n]
- * (re, im), upper triangle by columns as imago_secular_matrices writes them),
- * each then compared with its k-point element by element.  Waits for
+ * Candidates by hashes of h_full, each then compared with its k-point element
+ * by element of h_full and s_full (device, [num_kpoints][n][n] (re, im), upper
+ * triangle by columns as imago_secular_matrices writes them).  Waits for
  * `stream`. */
 IMAGO_API int imago_secular_pairs(int n, int num_kpoints, const double *h_full,
                                   const double *s_full, int *pair, void *stream);
