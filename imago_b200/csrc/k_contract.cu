@@ -22,7 +22,7 @@ namespace imago {
 // (unit, group) every group paid for the staging and waited for its own first
 // chunk, 15 us a CTA.  T = 4 or 8, picked by measurement; 1 for builds of one
 // matrix.  One B200, before / now: Si8 one matrix 0.18 / 0.09 ms, EP 0.53 /
-// 0.42, 162-atom quartz 1.02 / 0.72 and 8.78 / 8.51, Si16 momentum 0.29 / 0.21.
+// 0.38, 162-atom quartz 1.02 / 0.72 and 8.78 / 6.76, Si16 momentum 0.29 / 0.21.
 constexpr int kContractThreads = 128;
 constexpr int kElemsPerThread = 3;  // n_i n_j <= 384 per pass
 constexpr int kSpList = 512;        // shell pairs listed at a time
