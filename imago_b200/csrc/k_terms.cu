@@ -116,6 +116,10 @@ __global__ void __launch_bounds__(32 * kListWarps)
 // across the warp, whose latency bound the form with both (64-atom graphite
 // 0.93 ms, short scoreboard; staging 6.43 -> 6.10 ms, 162-atom quartz 14.6 ->
 // 13.8), and the order of a list is always the same: by step, lane, chunk.
+// Lists of up to a warp's lanes, as where every site has its own type, are
+// ranked by that order directly: clearing and adding up 64 x 32 counters for
+// each took much of the staging (216 diamond atoms with their own types: 59.9 ->
+// 42.2 ms, 162 quartz atoms 23.0 -> 18.0).
 constexpr int kFillWarps = 4, kFillRow = 33;
 
 __global__ void __launch_bounds__(32 * kFillWarps)
@@ -141,6 +145,30 @@ __global__ void __launch_bounds__(32 * kFillWarps)
                    ? min(kListBins - 1, (int)(fmaxf(0.f, sqrtf(d2) - margin) * inv))
                    : -1;
       };
+      ImageRef *out = list + range.x;
+      // the step's lower edge, rounded to stay below the distance
+      auto ref = [&](int i, int b) { return ImageRef{i, b * step * (1.f - 1e-5f)}; };
+      const int len = range.y - range.x;
+      if (len <= 32) {
+        int n = 0;  // bin: the images found, their places in the list's order
+        near_chunks(w, pt, m, lim, lane, [&](int ib) {
+          const int b = place(ib + lane);
+          const unsigned mask = __ballot_sync(0xffffffffu, b >= 0);
+          if (b >= 0) {
+            const int at = n + __popc(mask & ((1u << lane) - 1u));
+            bin[at] = ib + lane;
+            bin[32 + at] = (b << 10) + (lane << 5) + at;
+          }
+          n += __popc(mask);
+        });
+        __syncwarp();
+        const int key = lane < len ? bin[32 + lane] : 0;
+        int rank = 0;
+        for (int l = 0; l < len; ++l) rank += __shfl_sync(0xffffffffu, key, l) < key;
+        if (lane < len) out[rank] = ref(bin[lane], key >> 10);
+        __syncwarp();
+        continue;
+      }
       for (int i = lane; i < kListBins * kFillRow; i += 32) bin[i] = 0;
       __syncwarp();
       near_chunks(w, pt, m, lim, lane, [&](int ib) {
@@ -175,14 +203,9 @@ __global__ void __launch_bounds__(32 * kFillWarps)
       bin[lane * kFillRow + 32] = end[0] - sum[0];
       bin[(lane + 32) * kFillRow + 32] = half + end[1] - sum[1];
       __syncwarp();
-      ImageRef *out = list + range.x;
       near_chunks(w, pt, m, lim, lane, [&](int ib) {
         const int b = place(ib + lane);
-        if (b >= 0) {
-          // the step's lower edge, rounded to stay below the distance
-          out[bin[b * kFillRow + 32] + bin[b * kFillRow + lane]++] =
-              ImageRef{ib + lane, b * step * (1.f - 1e-5f)};
-        }
+        if (b >= 0) out[bin[b * kFillRow + 32] + bin[b * kFillRow + lane]++] = ref(ib + lane, b);
       });
       __syncwarp();
     }
