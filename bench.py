@@ -360,7 +360,7 @@ def prim3c_roofline(g, bufs, stream, flush, torch, peak, steps=3):
     """FP64 roofline of the three-centre primitive stage: the screened
     (shell pair, site, image) triples of the NP build and every EP term per
     class (imago_intg_count_triples) times the per-class flops above, over
-    the k_prim3c time of NP + EP builds run alone (kinds serialised, L2
+    the primitive kernels' time of NP + EP builds run alone (kinds serialised, L2
     flushed before each), against the measured FP64 peak."""
     from imago_b200 import intg
     cnp = g.count_triples(intg.IMAGO_NP)
@@ -384,7 +384,7 @@ def prim3c_roofline(g, bufs, stream, flush, torch, peak, steps=3):
     ms /= steps
     achieved = flops / (ms / 1e3) / 1e12
     return {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-            "frac": achieved / peak if peak else None, "kernel": "k_prim3c (NP + EP)",
+            "frac": achieved / peak if peak else None, "kernel": "k_prim3c_terms and k_prim3c_nuc (EP + NP)",
             "kernel_ms": ms, "algorithmic_flops": flops,
             "triples_np": int(cnp.sum()), "triples_ep": int(cep.sum()),
             "flops_source": "reference recursion flops per class x screened triples"}
@@ -715,11 +715,10 @@ def silica_headline(args, local, stream, torch):
 
 def schedules(g, bufs, stream, flush, torch, steps=3):
     """The three-centre stage's schedules on the context's build: per-class
-    launches, the persistent work-queue launch and per-class launches with
-    two EP terms per thread (device seconds of
-    whole builds replayed from graphs, and the primitive stage's ms with the
-    kinds serialised), the measured choice the context made, and back to
-    the measured choice."""
+    launches, the persistent work-queue launch and several EP terms of a type
+    per thread (device seconds of whole builds replayed from graphs, and the
+    primitive stage's ms with the kinds serialised), the measured choice the
+    context made, and back to the measured choice."""
     out = {"chosen": g.schedule()}
     for mode in ("per_class", "queue", "pairs"):
         g.set_schedule(mode)
